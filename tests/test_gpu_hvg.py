@@ -165,3 +165,33 @@ def test_hvg_called_as_single_cell_calls_it(cuda, golden):
         for a, name in ((mean, "mean"), (var, "var"), (nz, "nnz"), (b, "bsum"),
                         (q, "bsq")):
             assert np.array_equal(a, z[f"{key}_{name}"]), (form, name)
+
+
+def _skewed_csc(lengths, n, dtype, seed):
+    """A CSC matrix whose gene j stores lengths[j] counts (<= n cells)."""
+    rng = np.random.default_rng(seed)
+    ix = [np.sort(rng.choice(n, m, replace=False)) for m in lengths]
+    ip = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    d = rng.integers(1, 40, int(ip[-1]))
+    d[rng.random(d.size) < 0.01] = 60000
+    return d.astype(dtype), np.concatenate(ix).astype(np.int32), ip
+
+
+@pytest.mark.parametrize("lengths", [
+    [1], [0, 0, 4096, 0, 4096, 0], [4095, 1, 4097, 0, 8192, 3], [0] * 70 + [9000] + [1] * 70,
+    [31, 32, 33, 255, 256, 257] * 20, [20000, 0, 19999]])
+def test_hvg_csc_entries_split_across_genes(cuda, lengths):
+    """Genes that start, end and straddle the chunks of entries the CSC kernel
+    splits the matrix into, empty genes between them, with and without a
+    mask: every statistic bit-identical to the oracle's."""
+    n, g = 20000, len(lengths)
+    d, ix, ip = _skewed_csc(lengths, n, np.uint16, sum(lengths))
+    rng = np.random.default_rng(3)
+    clip = (rng.random(g) * 30 + 1).astype(np.float32)
+    for mask in (np.zeros(0, np.int8), (rng.random(n) < 0.7).astype(np.int8)):
+        nc = int(mask.sum()) if mask.size else n
+        got = _run("csc", d, ix, ip, None, mask, nc, g, clip, False)
+        want = (*oh.gene_mean_and_variance_csc(d, ix, ip, mask, nc, g),
+                *oh.clipped_sum_csc(d, ix, ip, mask, clip))
+        for a, w, name in zip(got, want, ("mean", "var", "nnz", "bsum", "bsq")):
+            assert np.array_equal(a, w), name
