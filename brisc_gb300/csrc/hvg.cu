@@ -23,6 +23,7 @@
 // that is not a valid range, sets an error word and the entry is skipped
 // (the reference does not check; here the call returns BGPU_ERR_INVALID).
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -32,9 +33,18 @@ namespace {
 enum : int { kMeanVar = 0, kClipped = 1 };
 
 constexpr int kHvgThreads = 512;
-// Genes whose three 64-bit accumulators fit one CTA's shared memory (96 KB,
-// two CTAs per SM); larger gene counts accumulate in global memory.
-constexpr uint32_t kHvgSmemGenes = 4096;
+// CSR: threads of a CTA, the values that take its shared 32-bit accumulators
+// (larger ones add to the 64-bit totals in global memory), the shared bytes a
+// gene needs (three words), and the loads a lane keeps in flight.
+constexpr int kCsrThreads = 1024;
+constexpr uint32_t kCsrSmall = 15;
+constexpr uint32_t kCsrGeneBytes = 12;
+constexpr int kCsrUnroll = 8;
+constexpr int kCsrRows = 4;        // listed rows a warp reads at once
+constexpr uint32_t kCsrMaxSlices = 8;
+// Most contributions a CTA may add to one gene: each adds at most 15^2 to a
+// 32-bit sum of squares.
+constexpr uint64_t kCsrMaxPerGene = 0xFFFFFFFFull / (kCsrSmall * kCsrSmall);
 
 // `<unsigned long long> x` of the reference, per stored value type. Signed
 // integers wrap modulo 2^64; floating values are truncated toward zero
@@ -55,14 +65,24 @@ __device__ __forceinline__ unsigned long long as_u64(double x) {
   return __double2ull_rz(x);
 }
 
-// acc = [sum | sumsq | count] x g. kMeanVar: count = stored entries.
-// kClipped: values above clip[gene] only count (hvg.pyx:298-303); the
+// The count as 32 bits when it is below 65536 (every real count); false for
+// anything else, which goes through as_u64.
+template <typename V>
+__device__ __forceinline__ bool small_count(V x, uint32_t& w) {
+  w = (uint32_t)x;
+  if constexpr (std::is_floating_point<V>::value)
+    return x >= V(0) && x < V(65536);
+  else
+    return (unsigned long long)(long long)x < 65536ull;
+}
+
+// acc = [sum | sumsq | count] x g, 64-bit. kMeanVar: count = stored entries.
+// kClipped: values above the clip value only count (hvg.pyx:298-303); the
 // comparison converts the integer to float, as C's `value > clip_val[gene]`.
 template <int MODE>
-__device__ __forceinline__ void accumulate(unsigned long long* acc, uint32_t g,
-                                           uint32_t gene, unsigned long long v,
-                                           const float* __restrict__ clip) {
-  if (MODE == kClipped && __ull2float_rn(v) > clip[gene]) {
+__device__ __forceinline__ void add_total(unsigned long long* acc, uint32_t g, uint32_t gene,
+                                          unsigned long long v, float clip) {
+  if (MODE == kClipped && __ull2float_rn(v) > clip) {
     atomicAdd(acc + 2ull * g + gene, 1ull);
     return;
   }
@@ -71,59 +91,181 @@ __device__ __forceinline__ void accumulate(unsigned long long* acc, uint32_t g,
   if (MODE == kMeanVar) atomicAdd(acc + 2ull * g + gene, 1ull);
 }
 
-// CSR input. cells == nullptr: every stored entry in [e0, e1) (flat,
-// grid-stride). cells != nullptr: warp per listed cell, lanes over its row.
-// use_smem: per-CTA accumulators in shared memory, added to `acc` at the end.
+// The totals that a CSR CTA's three words of a gene stand for.
+struct WordTotals {
+  unsigned long long s, s2, c;
+};
+template <int MODE>
+__device__ __forceinline__ WordTotals word_totals(uint32_t w0, uint32_t w1, uint32_t w2) {
+  if (MODE == kMeanVar) return {w0 + w1, w0 + w1 + 2u * w2, w0};  // modulo 2^32
+  return {w0, w1, w2};
+}
+
+// CSR input: one entry, a count of gene `gene`, whose shared words are
+// sw[0..2][j] when the CTA owns the gene. Three 32-bit integer additions at
+// most: kMeanVar keeps the entries, sum (v - 1) and sum v (v - 1) / 2 (all
+// modulo 2^32; a count of 1, most of them, adds to the first word only),
+// kClipped the sums, the sums of squares and the number of clipped entries.
+template <typename V, int MODE>
+__device__ __forceinline__ void csr_entry(uint32_t* sw, uint32_t gs, uint32_t j, V x, float clip,
+                                          unsigned long long* acc, uint32_t g, uint32_t gene) {
+  uint32_t w;
+  const bool small = small_count(x, w);
+  if (small && w <= kCsrSmall) {
+    if (MODE == kClipped) {
+      if ((float)w > clip) {
+        atomicAdd(sw + 2 * gs + j, 1u);
+      } else {
+        atomicAdd(sw + j, w);
+        atomicAdd(sw + gs + j, w * w);
+      }
+    } else {
+      atomicAdd(sw + j, 1u);
+      if (w != 1u) {
+        atomicAdd(sw + gs + j, w - 1u);
+        atomicAdd(sw + 2 * gs + j, w * (w - 1u) / 2u);
+      }
+    }
+    return;
+  }
+  add_total<MODE>(acc, g, gene, small ? (unsigned long long)w : as_u64(x), clip);
+}
+
+// CSR input. A CTA owns the genes [slice * gs, ...) of one of `slices` equal
+// runs of genes and one of the launch's chunks of the entries (cells ==
+// nullptr: a contiguous share of [range[0], range[1])) or of the listed cells
+// (a warp per cell, lanes over its row). It sums them in shared 32-bit words,
+// whose additions the hardware does in shared memory; a 64-bit addition there
+// is a compare-and-swap loop, and one in global memory costs a trip to L2 per
+// entry: 40k x 20,000, 38M float32 entries, 0.98 ms with 64-bit additions in
+// global memory, 0.12 ms. The words go to part[chunk][3][g] and
+// k_hvg_finish adds the chunks. Slices of one chunk are neighbouring CTAs,
+// so that all but the first find the entries in L2.
+// No word overflows: at most kCsrMaxPerGene entries of a gene are added before
+// the words are taken out. The launch bounds a chunk of entries; listed rows
+// go in epochs of `epoch` rows, after each of which but the last the words are
+// added to the 64-bit totals, and a row longer than g, which repeats genes,
+// goes straight to those.
+// gs == 0: no shared words, every entry goes to the 64-bit totals (more genes
+// than kCsrMaxSlices CTAs hold, where re-reading the entries costs more).
 template <typename V, typename I, int MODE>
-__global__ void __launch_bounds__(kHvgThreads)
+__global__ void __launch_bounds__(kCsrThreads)
 k_hvg_csr(const V* __restrict__ data, const I* __restrict__ indices,
           const I* __restrict__ indptr, uint64_t nnz, uint64_t num_rows,
-          uint64_t e0, uint64_t e1, const int64_t* __restrict__ cells,
-          uint64_t num_listed, uint32_t g, const float* __restrict__ clip,
-          unsigned long long* __restrict__ acc, int use_smem,
-          int* __restrict__ err) {
-  extern __shared__ unsigned long long sacc[];
-  if (use_smem) {
-    for (uint32_t i = threadIdx.x; i < 3 * g; i += blockDim.x) sacc[i] = 0ull;
-    __syncthreads();
-  }
-  unsigned long long* a = use_smem ? sacc : acc;
-  auto entry = [&](uint64_t i) {
-    const long long gene = (long long)indices[i];
+          const int64_t* __restrict__ range, const int64_t* __restrict__ cells,
+          uint64_t num_listed, uint64_t epoch, uint32_t g, uint32_t gs, uint32_t slices,
+          const float* __restrict__ clip, unsigned long long* __restrict__ acc,
+          uint32_t* __restrict__ part, int* __restrict__ err) {
+  extern __shared__ uint32_t sw[];  // [3][gs]
+  const uint32_t chunk = blockIdx.x / slices, slice = blockIdx.x % slices;
+  const uint32_t nchunks = gridDim.x / slices;
+  const uint32_t g0 = slice * gs, gn = gs ? min(g, g0 + gs) - g0 : g;
+  for (uint32_t i = threadIdx.x; i < 3 * gs; i += kCsrThreads) sw[i] = 0u;
+  __syncthreads();
+  auto entry = [&](I gi, V x) {
+    const long long gene = (long long)gi;
     if (gene < 0 || gene >= (long long)g) {
       *err = 1;
       return;
     }
-    accumulate<MODE>(a, g, (uint32_t)gene, as_u64(data[i]), clip);
+    const uint32_t j = (uint32_t)gene - g0;
+    if (j >= gn) return;
+    const float cv = MODE == kClipped ? clip[gene] : 0.f;
+    if (gs)
+      csr_entry<V, MODE>(sw, gs, j, x, cv, acc, g, (uint32_t)gene);
+    else
+      add_total<MODE>(acc, g, (uint32_t)gene, as_u64(x), cv);
   };
   if (cells == nullptr) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = e0 + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < e1;
-         i += stride)
-      entry(i);
+    const uint64_t r0 = range ? (uint64_t)range[0] : 0ull;
+    const uint64_t len = (range ? (uint64_t)range[1] : nnz) - r0;
+    const uint64_t per = (len + nchunks - 1) / nchunks;
+    const uint64_t e0 = r0 + min_u64(len, per * chunk), e1 = r0 + min_u64(len, per * (chunk + 1));
+    for (uint64_t i0 = e0 + threadIdx.x; i0 < e1; i0 += (uint64_t)kCsrThreads * kCsrUnroll) {
+      I gi[kCsrUnroll];
+      V x[kCsrUnroll];
+#pragma unroll
+      for (int u = 0; u < kCsrUnroll; ++u) {
+        const uint64_t i = i0 + (uint64_t)u * kCsrThreads;
+        gi[u] = i < e1 ? indices[i] : I(0);
+        x[u] = i < e1 ? data[i] : V(0);
+      }
+#pragma unroll
+      for (int u = 0; u < kCsrUnroll; ++u)
+        if (i0 + (uint64_t)u * kCsrThreads < e1) entry(gi[u], x[u]);
+    }
   } else {
     const int lane = threadIdx.x & 31;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t j = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-         j < num_listed; j += nwarps) {
-      const long long cell = cells[j];
-      if (cell < 0 || (uint64_t)cell >= num_rows) {
-        if (lane == 0) *err = 1;
-        continue;
+    const uint64_t per = (num_listed + nchunks - 1) / nchunks;
+    const uint64_t j0 = min_u64(num_listed, per * chunk), j1 = min_u64(num_listed, per * (chunk + 1));
+    for (uint64_t s0 = j0; s0 < j1; s0 += epoch) {
+      const uint64_t s1 = min_u64(j1, s0 + epoch);
+      // kCsrRows cells per round of a warp: a lane reads each cell's range,
+      // then the warp walks the rows
+      for (uint64_t r0 = s0 + (threadIdx.x >> 5) * kCsrRows; r0 < s1;
+           r0 += (kCsrThreads / 32) * kCsrRows) {
+        long long b = 0, e = 0;
+        if (lane < kCsrRows && r0 + lane < s1) {
+          const long long cell = cells[r0 + lane];
+          if (cell < 0 || (uint64_t)cell >= num_rows) {
+            *err = 1;
+          } else {
+            b = (long long)indptr[cell];
+            e = (long long)indptr[cell + 1];
+            if (b < 0 || e < b || (uint64_t)e > nnz) {
+              *err = 1;
+              b = e = 0;
+            }
+          }
+        }
+        for (int r = 0; r < kCsrRows; ++r) {
+          const uint64_t rb = (uint64_t)__shfl_sync(0xffffffffu, b, r);
+          const uint64_t re = (uint64_t)__shfl_sync(0xffffffffu, e, r);
+          if (re - rb > min_u64(g, kCsrMaxPerGene)) {  // repeats genes
+            for (uint64_t i = rb + lane; i < re; i += 32) {
+              const long long gene = (long long)indices[i];
+              if (gene < 0 || gene >= (long long)g)
+                *err = 1;
+              else if ((uint32_t)gene - g0 < gn)
+                add_total<MODE>(acc, g, (uint32_t)gene, as_u64(data[i]),
+                                MODE == kClipped ? clip[gene] : 0.f);
+            }
+            continue;
+          }
+          for (uint64_t i0 = rb + lane; i0 < re; i0 += 32 * kCsrRows) {
+            I gi[kCsrRows];
+            V x[kCsrRows];
+#pragma unroll
+            for (int u = 0; u < kCsrRows; ++u) {
+              gi[u] = i0 + 32 * u < re ? indices[i0 + 32 * u] : I(0);
+              x[u] = i0 + 32 * u < re ? data[i0 + 32 * u] : V(0);
+            }
+#pragma unroll
+            for (int u = 0; u < kCsrRows; ++u)
+              if (i0 + 32 * u < re) entry(gi[u], x[u]);
+          }
+        }
       }
-      const long long b = (long long)indptr[cell], e = (long long)indptr[cell + 1];
-      if (b < 0 || e < b || (uint64_t)e > nnz) {
-        if (lane == 0) *err = 1;
-        continue;
+      if (s1 < j1 && gs) {
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < gn; i += kCsrThreads) {
+          const uint32_t w0 = sw[i], w1 = sw[gs + i], w2 = sw[2 * gs + i];
+          sw[i] = sw[gs + i] = sw[2 * gs + i] = 0u;
+          if ((w0 | w1 | w2) == 0u) continue;
+          const WordTotals t = word_totals<MODE>(w0, w1, w2);
+          atomicAdd(acc + g0 + i, t.s);
+          atomicAdd(acc + (uint64_t)g + g0 + i, t.s2);
+          atomicAdd(acc + 2ull * g + g0 + i, t.c);
+        }
+        __syncthreads();
       }
-      for (uint64_t i = (uint64_t)b + lane; i < (uint64_t)e; i += 32) entry(i);
     }
   }
-  if (use_smem) {
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < 3 * g; i += blockDim.x)
-      if (sacc[i]) atomicAdd(acc + i, sacc[i]);
-  }
+  if (!gs) return;
+  __syncthreads();
+  for (uint32_t w = 0; w < 3; ++w)
+    for (uint32_t i = threadIdx.x; i < gn; i += kCsrThreads)
+      part[((uint64_t)chunk * 3 + w) * g + g0 + i] = sw[w * gs + i];
 }
 
 __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
@@ -141,7 +283,7 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 // hold most of the entries (the means of genes span orders of magnitude):
 // 400k x 2000, 36M uint16 entries with a mask, 9.3 ms, the longest gene's
 // serial loads; split by entries, kCscUnroll independent loads in flight per
-// lane, 0.26 ms.
+// lane, 0.12 ms.
 // The kernel first checks the ranges it reads: a gene whose range is not
 // within [0, nnz] or decreases sets err, and the call fails.
 constexpr uint32_t kCscChunk = 4096;
@@ -166,6 +308,7 @@ k_hvg_csc(const V* __restrict__ data, const I* __restrict__ indices,
   if (*err) return;  // k_hvg_check_ranges: the ranges are not increasing
   const int lane = threadIdx.x & 31;
   const uint64_t first = (uint64_t)indptr[0], last = (uint64_t)indptr[g];
+  bool bad = false;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t c0 = first + kCscChunk *
                                  ((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5);
@@ -188,39 +331,44 @@ k_hvg_csc(const V* __restrict__ data, const I* __restrict__ indices,
       for (uint64_t i0 = b + lane; i0 < e; i0 += 32 * kCscUnroll) {
         V x[kCscUnroll];
         bool use[kCscUnroll];
+        I cell[kCscUnroll];
+#pragma unroll
+        for (int u = 0; u < kCscUnroll; ++u) {  // every load before the first use
+          use[u] = i0 + 32 * u < e;
+          x[u] = use[u] ? data[i0 + 32 * u] : V(0);
+          cell[u] = mask && use[u] ? indices[i0 + 32 * u] : I(0);
+        }
         if (mask) {
-          I cell[kCscUnroll];
+          int8_t keep[kCscUnroll];
 #pragma unroll
           for (int u = 0; u < kCscUnroll; ++u) {
-            use[u] = i0 + 32 * u < e;
-            cell[u] = use[u] ? indices[i0 + 32 * u] : I(0);
+            const bool in = cell[u] >= 0 && (uint64_t)cell[u] < mask_len;
+            bad = bad || (use[u] && !in);
+            keep[u] = in ? mask[cell[u]] : (int8_t)0;
           }
 #pragma unroll
-          for (int u = 0; u < kCscUnroll; ++u) {
-            x[u] = use[u] ? data[i0 + 32 * u] : V(0);
-            if (use[u] && (cell[u] < 0 || (uint64_t)cell[u] >= mask_len)) {
-              *err = 1;
-              use[u] = false;
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < kCscUnroll; ++u) use[u] = use[u] && mask[cell[u]];
-        } else {
-#pragma unroll
-          for (int u = 0; u < kCscUnroll; ++u) {
-            use[u] = i0 + 32 * u < e;
-            x[u] = use[u] ? data[i0 + 32 * u] : V(0);
-          }
+          for (int u = 0; u < kCscUnroll; ++u) use[u] = use[u] && keep[u] != 0;
         }
 #pragma unroll
         for (int u = 0; u < kCscUnroll; ++u) {
-          const unsigned long long v = as_u64(x[u]);
-          const bool over = MODE == kClipped && __ull2float_rn(v) > cv;
-          if (use[u] && !over) {
-            s += v;
-            s2 += v * v;
+          if (!use[u]) continue;
+          uint32_t w;
+          bool over;
+          if (small_count(x[u], w)) {
+            over = MODE == kClipped && (float)w > cv;
+            if (!over) {
+              s += w;
+              s2 += (unsigned long long)w * w;
+            }
+          } else {
+            const unsigned long long v = as_u64(x[u]);
+            over = MODE == kClipped && __ull2float_rn(v) > cv;
+            if (!over) {
+              s += v;
+              s2 += v * v;
+            }
           }
-          c += use[u] && (MODE == kMeanVar || over) ? 1u : 0u;
+          c += MODE == kMeanVar || over ? 1u : 0u;
         }
       }
       s = warp_sum_u64(s);
@@ -234,37 +382,75 @@ k_hvg_csc(const V* __restrict__ data, const I* __restrict__ indices,
       b = e;
     }
   }
+  if (bad) *err = 1;
 }
 
-// hvg.pyx:66-70 / :246-250, every rounding explicit.
-__global__ void k_hvg_mean_var(const unsigned long long* __restrict__ acc, uint32_t g,
-                               uint64_t num_cells, float inv_num_cells,
-                               float inv_num_pairs, float* __restrict__ mean,
-                               float* __restrict__ var,
-                               uint32_t* __restrict__ nonzero_count) {
-  const uint32_t gene = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gene >= g) return;
-  const unsigned long long s = acc[gene], s2 = acc[(uint64_t)g + gene];
-  mean[gene] = __fmul_rn(__ull2float_rn(s), inv_num_cells);
-  const double sd = __ull2double_rn(s);
-  const double d = __dsub_rn(__dmul_rn(__ull2double_rn(num_cells), __ull2double_rn(s2)),
-                             __dmul_rn(sd, sd));
-  var[gene] = __double2float_rn(__dmul_rn((double)inv_num_pairs, d));
-  nonzero_count[gene] = (uint32_t)acc[2ull * g + gene];
+// Totals of the genes: acc (the 64-bit additions) plus, for CSR, the 32-bit
+// words of the nchunks chunks, then the statistics. A block takes 32 genes, 8
+// threads per gene over the chunks. Nothing is written when err is set.
+//   mean and variance: hvg.pyx:66-70 / :246-250, every rounding explicit;
+//   clipped sums: hvg.pyx:320-325 / :393-399, which the reference's -Ofast
+//   build computes as fused multiply-adds, clip * clip rounded first.
+template <int MODE>
+__global__ void __launch_bounds__(256)
+k_hvg_finish(const unsigned long long* __restrict__ acc, const uint32_t* __restrict__ part,
+             uint32_t nchunks, uint32_t g, uint64_t num_cells, float inv_num_cells,
+             float inv_num_pairs, const float* __restrict__ clip, float* __restrict__ out_a,
+             float* __restrict__ out_b, uint32_t* __restrict__ nonzero_count,
+             const int* __restrict__ err) {
+  __shared__ unsigned long long sh[3][8][33];
+  if (*err) return;
+  const uint32_t lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  const uint32_t gene = blockIdx.x * 32 + lane;
+  unsigned long long s = 0, s2 = 0, c = 0;
+  if (gene < g) {
+#pragma unroll 4
+    for (uint32_t r = row; r < nchunks; r += 8) {
+      const uint32_t* p = part + (uint64_t)r * 3 * g + gene;
+      const uint32_t w0 = p[0], w1 = p[g], w2 = p[2ull * g];
+      const WordTotals t = word_totals<MODE>(w0, w1, w2);
+      s += t.s;
+      s2 += t.s2;
+      c += t.c;
+    }
+  }
+  sh[0][row][lane] = s;
+  sh[1][row][lane] = s2;
+  sh[2][row][lane] = c;
+  __syncthreads();
+  if (row != 0 || gene >= g) return;
+  for (int r = 1; r < 8; ++r) {
+    s += sh[0][r][lane];
+    s2 += sh[1][r][lane];
+    c += sh[2][r][lane];
+  }
+  s += acc[gene];
+  s2 += acc[(uint64_t)g + gene];
+  c += acc[2ull * g + gene];
+  if (MODE == kMeanVar) {
+    out_a[gene] = __fmul_rn(__ull2float_rn(s), inv_num_cells);
+    const double sd = __ull2double_rn(s);
+    const double d = __dsub_rn(__dmul_rn(__ull2double_rn(num_cells), __ull2double_rn(s2)),
+                               __dmul_rn(sd, sd));
+    out_b[gene] = __double2float_rn(__dmul_rn((double)inv_num_pairs, d));
+    nonzero_count[gene] = (uint32_t)c;
+  } else {
+    const float out = __ull2float_rn(c), cv = clip[gene];
+    out_a[gene] = __fmaf_rn(out, cv, __ull2float_rn(s));
+    out_b[gene] = __fmaf_rn(out, __fmul_rn(cv, cv), __ull2float_rn(s2));
+  }
 }
 
-// hvg.pyx:320-325 / :393-399: the reference's -Ofast build computes these as
-// fused multiply-adds, with clip * clip rounded first.
-__global__ void k_hvg_clipped(const unsigned long long* __restrict__ acc, uint32_t g,
-                              const float* __restrict__ clip,
-                              float* __restrict__ batch_counts_sum,
-                              float* __restrict__ squared_batch_counts_sum) {
-  const uint32_t gene = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gene >= g) return;
-  const float out = __ull2float_rn(acc[2ull * g + gene]), c = clip[gene];
-  batch_counts_sum[gene] = __fmaf_rn(out, c, __ull2float_rn(acc[gene]));
-  squared_batch_counts_sum[gene] =
-      __fmaf_rn(out, __fmul_rn(c, c), __ull2float_rn(acc[(uint64_t)g + gene]));
+// The entries a CSR call without a cell list sums: rows [0, rows) of indptr.
+// A range outside [0, nnz] sets err to 2.
+template <typename I>
+__global__ void k_hvg_range(const I* __restrict__ indptr, uint64_t rows, uint64_t nnz,
+                            int64_t* __restrict__ range, int* __restrict__ err) {
+  const int64_t b = (int64_t)indptr[0], e = (int64_t)indptr[rows];
+  const bool ok = b >= 0 && e >= b && (uint64_t)e <= nnz;
+  range[0] = ok ? b : 0;
+  range[1] = ok ? e : 0;
+  if (!ok) *err = 2;
 }
 
 }  // namespace
@@ -321,28 +507,49 @@ struct HvgArgs {
   uint64_t num_listed;
   const int8_t* mask;
   uint64_t mask_len;
-  uint64_t e0, e1;  // CSR flat range
-  uint32_t g;       // genes accumulated
+  const int64_t* range;  // CSR without a cell list: the entries (nullptr: all)
+  uint32_t g;            // genes accumulated
   const float* clip;
   unsigned long long* acc;
+  Scratch* part;       // CSR: the chunks' words
+  uint32_t num_parts;  // chunks
   int* err;
 };
 
 template <typename V, typename I, int MODE>
-int launch_hvg_typed(const bgpu_hvg_input& in, const HvgArgs& a, cudaStream_t s) {
+int launch_hvg_typed(const bgpu_hvg_input& in, HvgArgs& a, cudaStream_t s) {
   const V* data = static_cast<const V*>(a.data);
   const I* idx = static_cast<const I*>(a.indices);
   const I* ptr = static_cast<const I*>(a.indptr);
   if (in.is_csr) {
-    const bool smem = a.g <= kHvgSmemGenes;
-    const size_t sm = smem ? 3ull * a.g * sizeof(unsigned long long) : 0;
-    if (sm > 48 * 1024) BGPU_CUDA((allow_max_smem(k_hvg_csr<V, I, MODE>)));
-    const uint64_t work = a.cells ? a.num_listed * 32 : a.e1 - a.e0;
-    const uint64_t want = std::max<uint64_t>(1, (work + kHvgThreads - 1) / kHvgThreads);
-    const unsigned grid = (unsigned)std::min<uint64_t>(want, (uint64_t)num_sms() * 2);
-    k_hvg_csr<V, I, MODE><<<grid, kHvgThreads, sm, s>>>(
-        data, idx, ptr, in.nnz, in.num_major, a.e0, a.e1, a.cells, a.num_listed,
-        a.g, a.clip, a.acc, smem ? 1 : 0, a.err);
+    // Genes per CTA: the fewest equal runs that fit the shared memory. Two
+    // CTAs per SM where their words fit it twice, else one; chunks for one
+    // wave, fewer when there is too little to read.
+    const uint32_t fit = (uint32_t)((device_smem_optin() - 256) / kCsrGeneBytes);
+    uint32_t slices = (uint32_t)ceil_div(a.g, fit);
+    uint32_t gs = (uint32_t)ceil_div(a.g, slices);
+    if (slices > kCsrMaxSlices) {
+      slices = 1;
+      gs = 0;
+    }
+    const size_t sm = (size_t)gs * kCsrGeneBytes;
+    const uint32_t per_sm = sm <= 112 * 1024 ? 2 : 1;
+    uint64_t chunks = std::max<uint64_t>(1, (uint64_t)num_sms() * per_sm / slices);
+    const uint64_t epoch = std::max<uint64_t>(1, kCsrMaxPerGene / a.g);
+    if (a.cells)
+      chunks = std::min(chunks, ceil_div(a.num_listed, kCsrRows * (kCsrThreads / 32)));
+    else
+      chunks = std::max(std::min(chunks, ceil_div(in.nnz, kCsrThreads * kCsrUnroll)),
+                        ceil_div(in.nnz, kCsrMaxPerGene));
+    chunks = std::max<uint64_t>(chunks, 1);
+    if (gs) {
+      BGPU_TRY(a.part->alloc(chunks * 3 * a.g * 4, s));
+      a.num_parts = (uint32_t)chunks;
+    }
+    BGPU_CUDA((allow_max_smem(k_hvg_csr<V, I, MODE>)));
+    k_hvg_csr<V, I, MODE><<<(unsigned)(chunks * slices), kCsrThreads, sm, s>>>(
+        data, idx, ptr, in.nnz, in.num_major, a.range, a.cells, a.num_listed, epoch, a.g, gs,
+        slices, a.clip, a.acc, (uint32_t*)a.part->p, a.err);
   } else {
     k_hvg_check_ranges<I><<<(a.g + kHvgThreads - 1) / kHvgThreads, kHvgThreads, 0, s>>>(
         ptr, in.nnz, a.g, a.err);
@@ -356,7 +563,7 @@ int launch_hvg_typed(const bgpu_hvg_input& in, const HvgArgs& a, cudaStream_t s)
 }
 
 template <typename I, int MODE>
-int launch_hvg_index(const bgpu_hvg_input& in, const HvgArgs& a, cudaStream_t s) {
+int launch_hvg_index(const bgpu_hvg_input& in, HvgArgs& a, cudaStream_t s) {
   switch (in.value_type) {
     case BGPU_VALUE_U16: return launch_hvg_typed<uint16_t, I, MODE>(in, a, s);
     case BGPU_VALUE_U32: return launch_hvg_typed<uint32_t, I, MODE>(in, a, s);
@@ -370,20 +577,20 @@ int launch_hvg_index(const bgpu_hvg_input& in, const HvgArgs& a, cudaStream_t s)
   return BGPU_ERR_INVALID;
 }
 
-int64_t read_index(const void* p, int index_type, uint64_t i) {
-  return index_type == BGPU_INDEX_I64 ? static_cast<const int64_t*>(p)[i]
-                                      : static_cast<const int32_t*>(p)[i];
-}
+// Device buffers of one call.
+struct HvgWork {
+  Scratch data, idx, ptr, cells, mask, err, acc, part, range;
+};
 
-// Stages the inputs, accumulates the integer sums into acc (3 x g) and checks
-// the kernels' error word. num_cells: as the reference's argument. For CSR
+// Stages the inputs and launches the accumulation of the integer sums into
+// a.acc (3 x g) and, for CSR, a.part. num_cells: as the reference's argument. For CSR
 // without a cell list, mean/variance sums every stored entry
 // (hvg.pyx:43-52) and the clipped sums every entry of rows [0, num_cells)
 // (hvg.pyx:292-303); with a list, mean/variance takes its first num_cells
 // cells (hvg.pyx:56-63) and the clipped sums all of them (hvg.pyx:305-314).
 template <int MODE>
 int hvg_accumulate(const bgpu_hvg_input* in, uint64_t num_cells, uint32_t g,
-                   const float* clip_dev, Scratch& acc, cudaStream_t s) {
+                   const float* clip_dev, HvgWork& w, HvgArgs& a, cudaStream_t s) {
   const size_t vsz = hvg_value_size(in->value_type);
   BGPU_REQUIRE(vsz != 0, BGPU_ERR_INVALID, "unknown value_type");
   BGPU_REQUIRE(in->index_type == BGPU_INDEX_I32 || in->index_type == BGPU_INDEX_I64,
@@ -401,7 +608,6 @@ int hvg_accumulate(const bgpu_hvg_input* in, uint64_t num_cells, uint32_t g,
     BGPU_REQUIRE(g <= in->num_major, BGPU_ERR_INVALID,
                  "indptr has fewer genes than num_genes");
 
-  HvgArgs a{};
   a.g = g;
   a.clip = clip_dev;
   uint64_t listed = 0;
@@ -409,69 +615,58 @@ int hvg_accumulate(const bgpu_hvg_input* in, uint64_t num_cells, uint32_t g,
     listed = MODE == kMeanVar ? num_cells : in->num_cell_indices;
     BGPU_REQUIRE(listed <= in->num_cell_indices, BGPU_ERR_INVALID,
                  "cell_indices holds fewer than num_cells cells");
-  } else if (in->is_csr) {
-    if (MODE == kMeanVar) {
-      a.e0 = 0;
-      a.e1 = in->nnz;
-    } else {
-      BGPU_REQUIRE(num_cells <= in->num_major, BGPU_ERR_INVALID,
-                   "num_cells exceeds the rows of indptr");
-      int64_t b = 0, e = 0;
-      if (dev) {
-        int64_t two[2] = {0, 0};
-        const char* base = static_cast<const char*>(in->indptr);
-        BGPU_CUDA(cudaMemcpyAsync(&two[0], base, isz, cudaMemcpyDeviceToHost, s));
-        BGPU_CUDA(cudaMemcpyAsync(&two[1], base + num_cells * isz, isz,
-                                  cudaMemcpyDeviceToHost, s));
-        BGPU_CUDA(cudaStreamSynchronize(s));
-        if (isz == 4) {  // the low words hold the int32 values (little endian)
-          b = (int32_t)(uint32_t)two[0];
-          e = (int32_t)(uint32_t)two[1];
-        } else {
-          b = two[0];
-          e = two[1];
-        }
-      } else {
-        b = read_index(in->indptr, in->index_type, 0);
-        e = read_index(in->indptr, in->index_type, num_cells);
-      }
-      BGPU_REQUIRE(b >= 0 && e >= b && (uint64_t)e <= in->nnz, BGPU_ERR_INVALID,
-                   "indptr is not a valid range");
-      a.e0 = (uint64_t)b;
-      a.e1 = (uint64_t)e;
-    }
+  } else if (in->is_csr && MODE == kClipped) {
+    BGPU_REQUIRE(num_cells <= in->num_major, BGPU_ERR_INVALID,
+                 "num_cells exceeds the rows of indptr");
   }
 
-  Scratch d_data, d_idx, d_ptr, d_cells, d_mask, d_err;
-  BGPU_TRY(stage(in->data, in->nnz * vsz, dev, d_data, &a.data, s));
-  BGPU_TRY(stage(in->indices, in->nnz * isz, dev, d_idx, &a.indices, s));
-  BGPU_TRY(stage(in->indptr, (in->num_major + 1) * isz, dev, d_ptr, &a.indptr, s));
+  BGPU_TRY(stage(in->data, in->nnz * vsz, dev, w.data, &a.data, s));
+  BGPU_TRY(stage(in->indices, in->nnz * isz, dev, w.idx, &a.indices, s));
+  BGPU_TRY(stage(in->indptr, (in->num_major + 1) * isz, dev, w.ptr, &a.indptr, s));
   const void* cells = nullptr;
   if (in->is_csr && in->cell_indices)
-    BGPU_TRY(stage(in->cell_indices, listed * sizeof(int64_t), dev, d_cells, &cells, s));
+    BGPU_TRY(stage(in->cell_indices, listed * sizeof(int64_t), dev, w.cells, &cells, s));
   a.cells = static_cast<const int64_t*>(cells);
   a.num_listed = listed;
   const void* mask = nullptr;
   if (!in->is_csr && in->cell_mask)
-    BGPU_TRY(stage(in->cell_mask, in->cell_mask_len, dev, d_mask, &mask, s));
+    BGPU_TRY(stage(in->cell_mask, in->cell_mask_len, dev, w.mask, &mask, s));
   a.mask = static_cast<const int8_t*>(mask);
   a.mask_len = in->cell_mask_len;
 
-  BGPU_TRY(acc.alloc(3ull * std::max<uint32_t>(g, 1) * sizeof(unsigned long long), s));
-  BGPU_TRY(d_err.alloc(sizeof(int), s));
-  a.acc = static_cast<unsigned long long*>(acc.p);
-  a.err = static_cast<int*>(d_err.p);
-  BGPU_CUDA(cudaMemsetAsync(acc.p, 0, 3ull * std::max<uint32_t>(g, 1) * 8, s));
-  BGPU_CUDA(cudaMemsetAsync(d_err.p, 0, sizeof(int), s));
-  if (g > 0 && (in->is_csr ? (a.cells ? listed > 0 : a.e1 > a.e0) : true)) {
+  BGPU_TRY(w.acc.alloc(3ull * std::max<uint32_t>(g, 1) * sizeof(unsigned long long), s));
+  BGPU_TRY(w.err.alloc(sizeof(int), s));
+  a.acc = static_cast<unsigned long long*>(w.acc.p);
+  a.err = static_cast<int*>(w.err.p);
+  a.part = &w.part;
+  BGPU_CUDA(cudaMemsetAsync(w.acc.p, 0, 3ull * std::max<uint32_t>(g, 1) * 8, s));
+  BGPU_CUDA(cudaMemsetAsync(w.err.p, 0, sizeof(int), s));
+  if (in->is_csr && !a.cells && MODE == kClipped) {
+    BGPU_TRY(w.range.alloc(2 * sizeof(int64_t), s));
+    a.range = static_cast<const int64_t*>(w.range.p);
+    if (in->index_type == BGPU_INDEX_I64)
+      k_hvg_range<int64_t><<<1, 1, 0, s>>>(static_cast<const int64_t*>(a.indptr), num_cells,
+                                           in->nnz, static_cast<int64_t*>(w.range.p), a.err);
+    else
+      k_hvg_range<int32_t><<<1, 1, 0, s>>>(static_cast<const int32_t*>(a.indptr), num_cells,
+                                           in->nnz, static_cast<int64_t*>(w.range.p), a.err);
+    BGPU_CHECK_LAUNCH();
+  }
+  if (g > 0 && (in->is_csr ? (a.cells ? listed > 0 : in->nnz > 0) : true)) {
     if (in->index_type == BGPU_INDEX_I64)
       BGPU_TRY((launch_hvg_index<int64_t, MODE>(*in, a, s)));
     else
       BGPU_TRY((launch_hvg_index<int32_t, MODE>(*in, a, s)));
   }
+  return BGPU_OK;
+}
+
+// Waits for the stream and reports what the kernels found wrong.
+int hvg_check(const HvgArgs& a, cudaStream_t s) {
   int herr = 0;
-  BGPU_CUDA(cudaMemcpyAsync(&herr, d_err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  BGPU_CUDA(cudaMemcpyAsync(&herr, a.err, sizeof(int), cudaMemcpyDeviceToHost, s));
   BGPU_CUDA(cudaStreamSynchronize(s));
+  BGPU_REQUIRE(herr != 2, BGPU_ERR_INVALID, "indptr is not a valid range");
   BGPU_REQUIRE(herr == 0, BGPU_ERR_INVALID,
                "a gene or cell index, or an indptr range, is out of bounds");
   return BGPU_OK;
@@ -489,8 +684,9 @@ extern "C" int bgpu_gene_mean_var(const bgpu_hvg_input* in, uint64_t num_cells,
                "bad gene mean/variance arguments");
   cudaStream_t s = (cudaStream_t)stream;
   const uint32_t g = in->num_genes;
-  Scratch acc;
-  BGPU_TRY(hvg_accumulate<kMeanVar>(in, num_cells, g, nullptr, acc, s));
+  HvgWork w;
+  HvgArgs a{};
+  BGPU_TRY(hvg_accumulate<kMeanVar>(in, num_cells, g, nullptr, w, a, s));
   // float inv_num_cells = 1.0 / num_cells; inv_num_pairs_of_cells =
   // 1.0 / (num_cells * (num_cells - 1)), an integer product (hvg.pyx:24-25)
   const float inv_n = (float)(1.0 / (double)num_cells);
@@ -509,17 +705,18 @@ extern "C" int bgpu_gene_mean_var(const bgpu_hvg_input* in, uint64_t num_cells,
     dn = static_cast<uint32_t*>(o_nz.p);
   }
   if (g > 0) {
-    k_hvg_mean_var<<<(g + 255) / 256, 256, 0, s>>>(
-        static_cast<const unsigned long long*>(acc.p), g, num_cells, inv_n, inv_p, dm,
-        dv, dn);
+    k_hvg_finish<kMeanVar><<<(unsigned)ceil_div(g, 32), 256, 0, s>>>(
+        a.acc, (const uint32_t*)w.part.p, a.num_parts, g, num_cells, inv_n, inv_p, nullptr, dm,
+        dv, dn, a.err);
     BGPU_CHECK_LAUNCH();
   }
+  BGPU_TRY(hvg_check(a, s));
   if (!dev && g > 0) {
     BGPU_CUDA(cudaMemcpyAsync(mean, dm, g * 4ull, cudaMemcpyDeviceToHost, s));
     BGPU_CUDA(cudaMemcpyAsync(var, dv, g * 4ull, cudaMemcpyDeviceToHost, s));
     BGPU_CUDA(cudaMemcpyAsync(nonzero_count, dn, g * 4ull, cudaMemcpyDeviceToHost, s));
+    BGPU_CUDA(cudaStreamSynchronize(s));
   }
-  BGPU_CUDA(cudaStreamSynchronize(s));
   return BGPU_OK;
 }
 
@@ -538,9 +735,9 @@ extern "C" int bgpu_clipped_sum(const bgpu_hvg_input* in, uint64_t num_cells,
   Scratch d_clip, o_b, o_s;
   const void* clip = nullptr;
   BGPU_TRY(stage(clip_val, g * 4ull, dev, d_clip, &clip, s));
-  Scratch acc;
-  BGPU_TRY(hvg_accumulate<kClipped>(in, num_cells, g, static_cast<const float*>(clip),
-                                    acc, s));
+  HvgWork w;
+  HvgArgs a{};
+  BGPU_TRY(hvg_accumulate<kClipped>(in, num_cells, g, static_cast<const float*>(clip), w, a, s));
   float* db = batch_counts_sum;
   float* ds = squared_batch_counts_sum;
   if (!dev) {
@@ -550,16 +747,17 @@ extern "C" int bgpu_clipped_sum(const bgpu_hvg_input* in, uint64_t num_cells,
     ds = static_cast<float*>(o_s.p);
   }
   if (g > 0) {
-    k_hvg_clipped<<<(g + 255) / 256, 256, 0, s>>>(
-        static_cast<const unsigned long long*>(acc.p), g, static_cast<const float*>(clip),
-        db, ds);
+    k_hvg_finish<kClipped><<<(unsigned)ceil_div(g, 32), 256, 0, s>>>(
+        a.acc, (const uint32_t*)w.part.p, a.num_parts, g, 0, 0.f, 0.f,
+        static_cast<const float*>(clip), db, ds, nullptr, a.err);
     BGPU_CHECK_LAUNCH();
   }
+  BGPU_TRY(hvg_check(a, s));
   if (!dev && g > 0) {
     BGPU_CUDA(cudaMemcpyAsync(batch_counts_sum, db, g * 4ull, cudaMemcpyDeviceToHost, s));
     BGPU_CUDA(cudaMemcpyAsync(squared_batch_counts_sum, ds, g * 4ull,
                               cudaMemcpyDeviceToHost, s));
+    BGPU_CUDA(cudaStreamSynchronize(s));
   }
-  BGPU_CUDA(cudaStreamSynchronize(s));
   return BGPU_OK;
 }

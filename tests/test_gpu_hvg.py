@@ -195,3 +195,32 @@ def test_hvg_csc_entries_split_across_genes(cuda, lengths):
                 *oh.clipped_sum_csc(d, ix, ip, mask, clip))
         for a, w, name in zip(got, want, ("mean", "var", "nnz", "bsum", "bsq")):
             assert np.array_equal(a, w), name
+
+
+@pytest.mark.parametrize("n,g", [(1, 1), (700, 31), (5000, 4097), (300, 18910), (300, 37900),
+                                 (64, 160000)])
+def test_hvg_csr_gene_slices(cuda, n, g):
+    """Gene counts around what one, two and more CTAs hold in shared memory and
+    past what they hold at all, with zeros and counts on both sides of the
+    32-bit accumulators' limit, whole and by cell list (repeated cells, and a
+    row that repeats genes): bit-identical to the oracle's."""
+    rng = np.random.default_rng(g)
+    lens = rng.integers(0, min(g, 400) + 1, n)
+    lens[0] = min(g, 400)
+    ip = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    ix = np.concatenate([rng.choice(g, m, replace=False) for m in lens]).astype(np.int64)
+    d = rng.choice([0, 1, 1, 1, 2, 3, 14, 15, 16, 17, 300, 65535, 65536], ix.size).astype(np.float32)
+    if n > 1:  # the last row holds one gene more often than there are genes
+        extra = min(g, 500) + 7
+        ip[-1] += extra
+        ix = np.concatenate([ix, np.full(extra, g - 1)])
+        d = np.concatenate([d, np.ones(extra, np.float32)])
+    clip = rng.choice(np.float32([0.5, 2, 14.5, 15, 299]), g)
+    cells = np.concatenate([np.arange(n), np.arange(n)[::-2], [n - 1, n - 1]]).astype(np.int64)
+    for c in (np.zeros(0, np.int64), cells):
+        nc = len(c) if len(c) else n
+        got = _run("csr", d, ix, ip, c, None, nc, g, clip, False)
+        want = (*oh.gene_mean_and_variance_csr(d, ix, ip, c, nc, g),
+                *oh.clipped_sum_csr(d, ix, ip, nc, g, c, clip))
+        for a, w, name in zip(got, want, ("mean", "var", "nnz", "bsum", "bsq")):
+            assert np.array_equal(a, w, equal_nan=True), name
