@@ -162,3 +162,75 @@ def test_neighbors_pipeline_matches_reference(cuda, golden, name):
     norms = np.einsum("ij,ij->i", X, X).astype(np.float32)
     same, worst = oknn.compare(X, ident, norms, nbr, ref)
     assert same >= 0.99 and worst <= 1.0, (same, worst)
+
+
+def _chain(X, C):
+    """x.c for every pair as the FP32 fused-multiply-add chain over the
+    dimensions in order (each step's product and sum rounded once: the sum
+    is formed in extended precision)."""
+    acc = np.zeros((len(X), len(C)), np.float32)
+    for j in range(X.shape[1]):
+        p = np.multiply.outer(X[:, j].astype(np.longdouble), C[:, j].astype(np.longdouble))
+        acc = (p + acc).astype(np.float32)
+    return acc
+
+
+def _fma(a, b, c):
+    return (np.longdouble(a) * b + c).astype(np.float32)
+
+
+def _lists(dist, order, size):
+    """Each row's list after offering the columns of `order[row]` in order, a
+    column replacing the first worst entry when strictly closer."""
+    n = len(dist)
+    out_d = np.full((n, size), np.finfo(np.float32).max, np.float32)
+    out_i = np.full((n, size), 0xFFFFFFFF, np.uint32)
+    for i in range(n):
+        for c in order[i]:
+            w = int(np.argmax(out_d[i]))
+            if dist[i, c] < out_d[i, w]:
+                out_d[i, w], out_i[i, w] = dist[i, c], c
+        o = np.lexsort((out_i[i], out_d[i]))
+        out_d[i], out_i[i] = out_d[i, o], out_i[i, o]
+    return out_i, out_d
+
+
+@pytest.mark.parametrize("n,d,nc,k,cs", [
+    (33, 1, 3, 4, 2), (129, 13, 5, 32, 5), (300, 50, 9, 33, 4), (257, 61, 40, 20, 12),
+    (200, 62, 7, 65, 7), (260, 128, 33, 128, 33), (700, 8, 620, 5, 256), (90, 4, 1, 10, 1)])
+def test_knn_self_bit_exact_with_ties(cuda, n, d, nc, k, cs):
+    """The tensor cores only select candidates: neighbours, distances and
+    nearest clusters are bit for bit those of the exhaustive FP32 loop, also
+    where rows repeat (equal distances, the reference's tie rule), clusters are
+    empty or start inside an 8-row group, more than 512 clusters are searched
+    by one CTA's cells, and one cell is far larger than the rest."""
+    rng = np.random.default_rng(n * d)
+    X = rng.standard_normal((n, d)).astype(np.float32) * np.float32(3)
+    X[rng.integers(0, n, n // 3)] = X[rng.integers(0, n, n // 3)]
+    X[n // 2] *= 50
+    C = rng.standard_normal((nc, d)).astype(np.float32) * np.float32(3)
+    if nc > 2:
+        C[-1] = C[0]
+    lab = np.sort(rng.integers(0, max(1, nc - 1), n))
+    counts = np.bincount(lab, minlength=nc).astype(np.uint32)
+    norms = np.einsum("ij,ij->i", X, X).astype(np.float32)
+    so = rng.permutation(n).astype(np.uint32)
+    c = dict(X=X, sorted_order=so, centroids=C, num_cells_per_cluster=counts,
+             cell_norms=norms, num_neighbors=k, num_clusters_searched=cs)
+    o = _run(c)
+    cn = C[:, 0] * C[:, 0]
+    for j in range(1, d):
+        cn = _fma(C[:, j], C[:, j], cn)
+    pd = _fma(np.float32(-2), _chain(X, C), cn[None, :])
+    near, cdist = _lists(pd, [range(nc)] * n, cs)
+    np.testing.assert_array_equal(o["nearest_clusters"], near)
+    np.testing.assert_array_equal(o["centroid_distances"], cdist)
+    start = np.concatenate([[0], np.cumsum(counts)]).astype(int)
+    dist = norms[:, None] + _fma(np.float32(-2), _chain(X, X), norms[None, :])
+    order = [[r for u in np.sort(near[i]) for r in range(start[u], start[u + 1]) if r != i]
+             for i in range(n)]
+    want_i, want_d = _lists(dist, order, k)
+    have = want_i != 0xFFFFFFFF
+    np.testing.assert_array_equal(o["distances"], want_d)
+    np.testing.assert_array_equal(o["neighbors"] != 0xFFFFFFFF, have)
+    np.testing.assert_array_equal(o["neighbors"][have], so[want_i[have]])
