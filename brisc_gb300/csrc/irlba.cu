@@ -1128,10 +1128,18 @@ extern "C" void bgpu_solve_opts_default(bgpu_solve_opts* o) {
 static void choose_shapes(Matrix& m) {
   const double avg = m.n ? (double)m.nnz / (double)m.n : 0.0;
   int G = 4;
-  while (G < 32 && G * 8 < avg) G *= 2;  // about two 4-entry loads per lane
+  // two to four 4-entry loads per lane, all in flight: with fewer, a warp
+  // waits on its row alone (50k x 2000 floats, 150 entries per row: 24.8 us
+  // with 32 lanes per row, 21.2 us with 16)
+  while (G < 32 && G * 16 < avg) G *= 2;
   m.spmv_group = G;
   m.spmv_blocks = num_sms() * 8;
+  // genes per CTA of the panel products: fewer where the panels alone do not
+  // give every SM eight CTAs
   m.rmat_colgroup = m.g <= 512 ? 64 : 256;
+  while (m.rmat_colgroup > 64 &&
+         m.num_panels * ceil_div(m.g, m.rmat_colgroup) < (uint64_t)num_sms() * 8)
+    m.rmat_colgroup /= 2;
   // X.v kernel: the segmented stream keeps every lane busy on short rows;
   // 8 lanes per row amortise their per-row work better on long ones.
   m.spmv_seg = m.csr_heads && avg < 64.0;

@@ -41,6 +41,7 @@
 #include <vector>
 
 #include "matrix.cuh"
+#include "moments.cuh"
 
 namespace bgpu {
 
@@ -137,7 +138,9 @@ k_xv_sell_multi(const __grid_constant__ TaskList<XvTask> L) {
 
 // ---------------------------------------------------------------------------
 // X^T.u (kMom = false) and the per-gene moments (kMom = true: u = 1, value
-// and squared value summed in FP64).
+// and squared value summed as float pairs per segment, then in FP64; the
+// moments of 28.5M entries at 300k x 2000: 303 us with FP64 sums per entry,
+// 77 us).
 template <bool kMom>
 struct XtAcc;
 template <>
@@ -146,13 +149,7 @@ struct XtAcc<false> {
   __device__ __forceinline__ void add(float v) { s += v; }
 };
 template <>
-struct XtAcc<true> {
-  double s = 0.0, q = 0.0;
-  __device__ __forceinline__ void add(float v) {
-    s += (double)v;
-    q += (double)v * (double)v;
-  }
-};
+struct XtAcc<true> : PairMoments {};
 
 __host__ __device__ inline uint32_t xt_esc_floats(uint32_t esc_max) {
   return (esc_max + 3u) & ~3u;
@@ -250,8 +247,22 @@ __device__ __forceinline__ void xt_sell_body(const XtView& X, const float* __res
       }
       if (gene != kNoGene) {  // one segment per gene and panel: no collisions
         if constexpr (kMom) {
-          gm[gene].x += acc.s;
-          gm[gene].y += acc.q;
+          double s = acc.sum(), q = acc.squares();
+          if (!acc.good()) {  // out of the pairs' range: the segment again, in FP64
+            s = q = 0.0;
+            for (uint32_t k = 0; k < U; ++k) {
+              const uint2 a = ld_stream_u2(src + (uint64_t)k * 32);
+              const uint32_t off[4] = {a.x & 0xffffu, a.x >> 16, a.y & 0xffffu, a.y >> 16};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const double v = (double)smem_at(smem, off[i]);
+                s += v;
+                q += v * v;
+              }
+            }
+          }
+          gm[gene].x += s;
+          gm[gene].y += q;
         } else {
           gs[gene] += acc.s;
         }

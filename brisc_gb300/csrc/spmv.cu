@@ -8,8 +8,8 @@
 //  X^T.u   (brisc/pca.pyx:478-511 rmatvec_csc_parallel_raw): one CTA per
 //          (row panel, gene group). The panel's u and size factors are staged
 //          in shared memory, so the per-entry gathers hit shared memory instead
-//          of L2; one warp reduces one gene's segment (a warp-segmented
-//          reduction, no atomics) into a per-panel partial (gene-major
+//          of L2; a group of lanes reduces one gene's segment (a fixed shuffle
+//          tree, no atomics) into a per-panel partial (gene-major
 //          layout); a second pass adds the partials of all panels in panel
 //          order. These register-vector kernels serve layouts outside the
 //          streaming kernels' limits (stream.cu).
@@ -18,6 +18,7 @@
 #include <algorithm>
 
 #include "matrix.cuh"
+#include "moments.cuh"
 
 namespace bgpu {
 
@@ -80,7 +81,20 @@ k_spmv(CsrView X, const float* __restrict__ v, const float* __restrict__ sd,
   }
 }
 
-template <int MODE>
+// Lanes per (panel, gene) segment: G lanes take 4 G entries per step, 32 / G
+// segments per warp. A whole warp per segment leaves most lanes without an
+// entry where segments are short (1024 rows x 8 %: 80 entries) and pays its
+// shuffles per segment: 50k x 2000 float values, 7.8M entries: X^T.u 47 us,
+// moments 212 us with 32 lanes and one load at a time, 39 us and 50 us with 8 lanes and
+// kSegLoads loads in flight.
+constexpr int kSegLoads = 3;
+template <int G>
+struct Segments {
+  const uint32_t lane = threadIdx.x & (G - 1);
+  const uint32_t first = threadIdx.x / G, step = 256 / G;
+};
+
+template <int MODE, int G>
 __global__ void __launch_bounds__(256)
 k_rmat_partials(CscView X, const float* __restrict__ u,
                 const float* __restrict__ u_scale, float* __restrict__ u_out,
@@ -105,51 +119,71 @@ k_rmat_partials(CscView X, const float* __restrict__ u,
     }
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int nw = blockDim.x >> 5;
+  const Segments<G> seg;
   const int64_t pbase = X.rowptr[r0];
   const int32_t* cp = X.colptr + (uint64_t)p * (X.g + 1);
   const uint32_t c0 = blockIdx.y * colgroup;
   const uint32_t c1 = min(X.g, c0 + colgroup);
-  for (uint32_t c = c0 + wid; c < c1; c += nw) {
-    const int64_t e0 = pbase + cp[c], e1 = pbase + cp[c + 1];
+  // every lane of a warp takes the same number of turns (group_sum shuffles);
+  // the next segment's bounds load while this one is summed
+  uint32_t c = c0 + seg.first;
+  int64_t n0 = c < c1 ? cp[c] : 0, n1 = c < c1 ? cp[c + 1] : 0;
+  for (uint32_t cb = c0; cb < c1; cb += seg.step, c += seg.step) {
+    const int64_t e0 = pbase + n0, e1 = pbase + n1;
+    const uint32_t cn = c + seg.step;
+    n0 = cn < c1 ? cp[cn] : 0;
+    n1 = cn < c1 ? cp[cn + 1] : 0;
     float acc = 0.f;
-    if constexpr (MODE == kCounts) {
-#pragma unroll 4
-      for (int64_t b = (e0 & ~3LL) + 4 * lane; b < e1; b += 128) {
-        const uint4 q = ld_stream_u4(X.packed + b);
-        const uint32_t qq[4] = {q.x, q.y, q.z, q.w};
+    for (int64_t b = (e0 & ~3LL) + 4 * seg.lane; b < e1; b += 4 * G * kSegLoads) {
+      if constexpr (MODE == kCounts) {
+        uint4 q[kSegLoads];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int64_t e = b + k;
-          if (e >= e0 && e < e1) {
-            const uint32_t lr = (qq[k] >> 16) & (P - 1);  // bit 31 may flag a segment head
-            acc += norm_count(qq[k] & 0xffffu, fs[lr]) * us[lr];
+        for (int i = 0; i < kSegLoads; ++i)
+          q[i] = b + 4 * G * i < e1 ? ld_stream_u4(X.packed + b + 4 * G * i)
+                                    : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int i = 0; i < kSegLoads; ++i) {
+          const uint32_t qq[4] = {q[i].x, q[i].y, q[i].z, q[i].w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int64_t e = b + 4 * G * i + k;
+            if (e >= e0 && e < e1) {
+              const uint32_t lr = (qq[k] >> 16) & (P - 1);  // bit 31 may flag a segment head
+              acc += norm_count(qq[k] & 0xffffu, fs[lr]) * us[lr];
+            }
+          }
+        }
+      } else {
+        uint4 qv[kSegLoads];
+        uint2 qr[kSegLoads];
+#pragma unroll
+        for (int i = 0; i < kSegLoads; ++i) {
+          const bool in = b + 4 * G * i < e1;
+          qv[i] = in ? ld_stream_u4(X.val + b + 4 * G * i) : make_uint4(0u, 0u, 0u, 0u);
+          qr[i] = in ? ld_stream_u2(X.row + b + 4 * G * i) : make_uint2(0u, 0u);
+        }
+#pragma unroll
+        for (int i = 0; i < kSegLoads; ++i) {
+          const float vv[4] = {__uint_as_float(qv[i].x), __uint_as_float(qv[i].y),
+                               __uint_as_float(qv[i].z), __uint_as_float(qv[i].w)};
+          const uint32_t rr[4] = {qr[i].x & 0xffffu, qr[i].x >> 16, qr[i].y & 0xffffu,
+                                  qr[i].y >> 16};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int64_t e = b + 4 * G * i + k;
+            if (e >= e0 && e < e1) acc += vv[k] * us[rr[k]];
           }
         }
       }
-    } else {
-#pragma unroll 4
-      for (int64_t b = (e0 & ~3LL) + 4 * lane; b < e1; b += 128) {
-        const uint4 qv = ld_stream_u4(X.val + b);
-        const uint2 qr = ld_stream_u2(X.row + b);
-        const float vv[4] = {__uint_as_float(qv.x), __uint_as_float(qv.y),
-                             __uint_as_float(qv.z), __uint_as_float(qv.w)};
-        const uint32_t rr[4] = {qr.x & 0xffffu, qr.x >> 16, qr.y & 0xffffu,
-                                qr.y >> 16};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int64_t e = b + k;
-          if (e >= e0 && e < e1) acc += vv[k] * us[rr[k]];
-        }
-      }
     }
-    acc = warp_sum(acc);
-    if (lane == 0) partials[(uint64_t)c * X.num_panels + p] = acc;
+    acc = group_sum<G>(acc);
+    if (seg.lane == 0 && c < c1) partials[(uint64_t)c * X.num_panels + p] = acc;
   }
 }
 
-template <int MODE>
+// Per (panel, gene): sum and sum of squares of the values, as float pairs per
+// lane (moments.cuh), the lanes added in FP64.
+template <int MODE, int G>
 __global__ void __launch_bounds__(256)
 k_gene_moments(CscView X, double2* __restrict__ partials, uint32_t colgroup) {
   extern __shared__ float sm[];
@@ -166,17 +200,23 @@ k_gene_moments(CscView X, double2* __restrict__ partials, uint32_t colgroup) {
     }
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int nw = blockDim.x >> 5;
+  const Segments<G> seg;
   const int64_t pbase = X.rowptr[r0];
   const int32_t* cp = X.colptr + (uint64_t)p * (X.g + 1);
   const uint32_t c0 = blockIdx.y * colgroup;
   const uint32_t c1 = min(X.g, c0 + colgroup);
-  for (uint32_t c = c0 + wid; c < c1; c += nw) {
-    const int64_t e0 = pbase + cp[c], e1 = pbase + cp[c + 1];
-    double s1 = 0.0, s2 = 0.0;
-    for (int64_t b = (e0 & ~3LL) + 4 * lane; b < e1; b += 128) {
-      float vals[4];
+  uint32_t c = c0 + seg.first;
+  int64_t n0 = c < c1 ? cp[c] : 0, n1 = c < c1 ? cp[c + 1] : 0;
+  for (uint32_t cb = c0; cb < c1; cb += seg.step, c += seg.step) {
+    const int64_t e0 = pbase + n0, e1 = pbase + n1;
+    const uint32_t cn = c + seg.step;
+    n0 = cn < c1 ? cp[cn] : 0;
+    n1 = cn < c1 ? cp[cn + 1] : 0;
+    auto values = [&](int64_t b, float (&vals)[4]) {
+      if (b >= e1) {
+        vals[0] = vals[1] = vals[2] = vals[3] = 0.f;
+        return;
+      }
       if constexpr (MODE == kCounts) {
         const uint4 q = ld_stream_u4(X.packed + b);
         const uint32_t qq[4] = {q.x, q.y, q.z, q.w};
@@ -199,28 +239,65 @@ k_gene_moments(CscView X, double2* __restrict__ partials, uint32_t colgroup) {
           vals[k] = (e >= e0 && e < e1) ? vv[k] : 0.f;
         }
       }
+    };
+    PairMoments m;
+    for (int64_t b = (e0 & ~3LL) + 4 * seg.lane; b < e1; b += 4 * G * kSegLoads) {
+      float vals[kSegLoads][4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        s1 += (double)vals[k];
-        s2 += (double)vals[k] * (double)vals[k];
+      for (int i = 0; i < kSegLoads; ++i) values(b + 4 * G * i, vals[i]);
+#pragma unroll
+      for (int i = 0; i < kSegLoads; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) m.add(vals[i][k]);
+    }
+    double s1 = m.sum(), s2 = m.squares();
+    if (!m.good()) {  // out of the pairs' range (or no entry): again, in FP64
+      s1 = s2 = 0.0;
+      for (int64_t b = (e0 & ~3LL) + 4 * seg.lane; b < e1; b += 4 * G) {
+        float vals[4];
+        values(b, vals);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          s1 += (double)vals[k];
+          s2 += (double)vals[k] * (double)vals[k];
+        }
       }
     }
-    s1 = warp_sum(s1);
-    s2 = warp_sum(s2);
-    if (lane == 0) partials[(uint64_t)p * X.g + c] = make_double2(s1, s2);
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+    }
+    if (seg.lane == 0 && c < c1) partials[(uint64_t)p * X.g + c] = make_double2(s1, s2);
   }
 }
 
-__global__ void k_gene_sd(const double2* __restrict__ partials,
-                          uint32_t num_panels, uint32_t g, uint64_t n,
-                          float* __restrict__ sd) {
-  uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= g) return;
+// The standard deviations from the panels' (or CTAs') moments: a block takes
+// 32 genes (lane = gene, so the loads are runs of the gene-major row), its
+// warps take every 32nd panel and are added in warp order. A thread per gene
+// instead is a serial chain of loads: 114 us for 608 panels x 2000 genes, 17 us.
+constexpr int kSdWarps = 32;
+__global__ void __launch_bounds__(32 * kSdWarps)
+k_gene_sd(const double2* __restrict__ partials, uint32_t num_panels, uint32_t g, uint64_t n,
+          float* __restrict__ sd) {
+  __shared__ double2 sh[kSdWarps][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint32_t c = blockIdx.x * 32 + lane;
   double s1 = 0.0, s2 = 0.0;
-  for (uint32_t p = 0; p < num_panels; ++p) {
-    double2 t = partials[(uint64_t)p * g + c];
-    s1 += t.x;
-    s2 += t.y;
+  if (c < g) {
+#pragma unroll 4
+    for (uint32_t p = wid; p < num_panels; p += kSdWarps) {
+      const double2 t = partials[(uint64_t)p * g + c];
+      s1 += t.x;
+      s2 += t.y;
+    }
+  }
+  sh[wid][lane] = make_double2(s1, s2);
+  __syncthreads();
+  if (wid != 0 || c >= g) return;
+  for (int w = 1; w < kSdWarps; ++w) {
+    s1 += sh[w][lane].x;
+    s2 += sh[w][lane].y;
   }
   const double dn = (double)n;
   // pca.pyx:83-86: sqrt((n * sum_sq - sum^2) / (n (n - 1))), clipped at 1e-8
@@ -288,52 +365,64 @@ int launch_matvec(const Matrix& m, const float* v, const float* sd, float* y,
   return BGPU_OK;
 }
 
+// Segments of more than 128 entries on average keep a whole warp's lanes at
+// work; below that 8 lanes per segment (see Segments).
+static bool wide_segments(const Matrix& m) {
+  return (double)m.nnz > 128.0 * (double)m.num_panels * (double)m.g;
+}
+
+template <int MODE, int G>
+static int launch_partials_typed(const Matrix& m, const float* u, const float* u_scale_dev,
+                                 float* u_out, float* partials, cudaStream_t s) {
+  const uint32_t cg = m.rmat_colgroup;
+  const dim3 grid(m.num_panels, (unsigned)ceil_div(m.g, cg));
+  const size_t smem = (size_t)m.P * 2 * sizeof(float);
+  if (smem > 48 * 1024) BGPU_CUDA((allow_max_smem(k_rmat_partials<MODE, G>)));
+  k_rmat_partials<MODE, G><<<grid, 256, smem, s>>>(csc_view(m), u, u_scale_dev, u_out, partials,
+                                                   cg);
+  BGPU_CHECK_LAUNCH();
+  return BGPU_OK;
+}
+
+template <int MODE, int G>
+static int launch_moments_typed(const Matrix& m, double* partials, cudaStream_t s) {
+  const uint32_t cg = m.rmat_colgroup;
+  const dim3 grid(m.num_panels, (unsigned)ceil_div(m.g, cg));
+  const size_t smem = (size_t)m.P * 2 * sizeof(float);
+  if (smem > 48 * 1024) BGPU_CUDA((allow_max_smem(k_gene_moments<MODE, G>)));
+  k_gene_moments<MODE, G><<<grid, 256, smem, s>>>(csc_view(m), (double2*)partials, cg);
+  BGPU_CHECK_LAUNCH();
+  return BGPU_OK;
+}
+
 int launch_rmatvec_partials(const Matrix& m, const float* u,
                             const float* u_scale_dev, float* u_out,
                             float* partials, cudaStream_t s) {
-  const CscView X = csc_view(m);
-  const uint32_t cg = m.rmat_colgroup;
-  dim3 grid(m.num_panels, (unsigned)ceil_div(m.g, cg));
-  const size_t smem = (size_t)m.P * 2 * sizeof(float);
-  if (m.mode == kCounts) {
-    if (smem > 48 * 1024)
-      BGPU_CUDA(allow_max_smem(k_rmat_partials<kCounts>));
-    k_rmat_partials<kCounts><<<grid, 256, smem, s>>>(X, u, u_scale_dev, u_out,
-                                                     partials, cg);
-  } else {
-    if (smem > 48 * 1024)
-      BGPU_CUDA(allow_max_smem(k_rmat_partials<kFloat>));
-    k_rmat_partials<kFloat><<<grid, 256, smem, s>>>(X, u, u_scale_dev, u_out,
-                                                    partials, cg);
-  }
-  BGPU_CHECK_LAUNCH();
-  return BGPU_OK;
+  const bool wide = wide_segments(m);
+  if (m.mode == kCounts)
+    return wide ? launch_partials_typed<kCounts, 32>(m, u, u_scale_dev, u_out, partials, s)
+                : launch_partials_typed<kCounts, 8>(m, u, u_scale_dev, u_out, partials, s);
+  return wide ? launch_partials_typed<kFloat, 32>(m, u, u_scale_dev, u_out, partials, s)
+              : launch_partials_typed<kFloat, 8>(m, u, u_scale_dev, u_out, partials, s);
 }
 
 int launch_gene_stddev(const Matrix& m, double* partials, float* sd,
                        cudaStream_t s) {
   if (m.sell) {  // per-CTA moments over the sliced-ELL panels, CTA order
     BGPU_TRY(launch_xt_moments(m, partials, s));
-    k_gene_sd<<<(unsigned)ceil_div(m.g, 256), 256, 0, s>>>(
+    k_gene_sd<<<(unsigned)ceil_div(m.g, 32), 32 * kSdWarps, 0, s>>>(
         (const double2*)partials, m.num_panels, m.g, m.n, sd);
     BGPU_CHECK_LAUNCH();
     return BGPU_OK;
   }
-  const CscView X = csc_view(m);
-  const uint32_t cg = m.rmat_colgroup;
-  dim3 grid(m.num_panels, (unsigned)ceil_div(m.g, cg));
-  const size_t smem = (size_t)m.P * 2 * sizeof(float);
-  if (m.mode == kCounts) {
-    if (smem > 48 * 1024)
-      BGPU_CUDA(allow_max_smem(k_gene_moments<kCounts>));
-    k_gene_moments<kCounts><<<grid, 256, smem, s>>>(X, (double2*)partials, cg);
-  } else {
-    if (smem > 48 * 1024)
-      BGPU_CUDA(allow_max_smem(k_gene_moments<kFloat>));
-    k_gene_moments<kFloat><<<grid, 256, smem, s>>>(X, (double2*)partials, cg);
-  }
-  BGPU_CHECK_LAUNCH();
-  k_gene_sd<<<(unsigned)ceil_div(m.g, 256), 256, 0, s>>>(
+  const bool wide = wide_segments(m);
+  if (m.mode == kCounts)
+    BGPU_TRY((wide ? launch_moments_typed<kCounts, 32>(m, partials, s)
+                   : launch_moments_typed<kCounts, 8>(m, partials, s)));
+  else
+    BGPU_TRY((wide ? launch_moments_typed<kFloat, 32>(m, partials, s)
+                   : launch_moments_typed<kFloat, 8>(m, partials, s)));
+  k_gene_sd<<<(unsigned)ceil_div(m.g, 32), 32 * kSdWarps, 0, s>>>(
       (const double2*)partials, m.num_panels, m.g, m.n, sd);
   BGPU_CHECK_LAUNCH();
   return BGPU_OK;

@@ -310,3 +310,30 @@ def test_row_order_does_not_change_products(cuda):
         out.append(y.cpu().numpy())
         M.close()
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-15, 1e-22, 1e16, 0.0])
+@pytest.mark.parametrize("n,g,density", [(1, 3, 0.9), (1023, 40, 0.3), (1025, 70, 0.02),
+                                         (5000, 300, 0.2)])
+def test_gene_stddev_of_any_scale(cuda, n, g, density, scale):
+    """The clipped standard deviation of float values whose squares are
+    ordinary, too small or too large for FP32 pairs, or all zero, against
+    FP64: within one float rounding of it and of the cancellation in n s2 -
+    s1^2, which FP64 sums of the same values leave (1e-6 relative where the
+    spread is the values' own)."""
+    import torch
+    rng = np.random.default_rng(n + g)
+    X = sp.random(n, g, density, "csr", dtype=np.float32, random_state=rng,
+                  data_rvs=lambda k: rng.lognormal(0, 1, k) * rng.choice([-1, 1], k))
+    X.data = (X.data.astype(np.float64) * scale).astype(np.float32)
+    M = DeviceMatrix(X.indptr.astype(np.int64), X.indices.astype(np.int64), X.data, n, g)
+    sd = torch.empty(g, dtype=torch.float32, device=cuda)
+    M.gene_stddev(sd)
+    M.close()
+    D = X.toarray().astype(np.float64)
+    s1, s2 = D.sum(0), (D * D).sum(0)
+    with np.errstate(all="ignore"):
+        want = np.sqrt(np.maximum((n * s2 - s1 * s1) / (n * (n - 1.0)), 0)) if n > 1 \
+            else np.zeros(g)
+    want = np.maximum(np.nan_to_num(want), 1e-8)
+    np.testing.assert_allclose(sd.cpu().numpy(), want.astype(np.float32), rtol=1e-6)
