@@ -802,7 +802,7 @@ int harmony_run(const float* PCs, float* Z, float* Y, float* R, const uint32_t* 
   std::vector<void*> allocs;
   auto dalloc = [&](auto** p, size_t bytes) -> int {
     void* q = nullptr;
-    BGPU_CUDA(cudaMallocAsync(&q, std::max<size_t>(bytes, 16), s));
+    BGPU_CUDA(scratch_alloc(&q, std::max<size_t>(bytes, 16), s));
     allocs.push_back(q);
     *p = (std::remove_reference_t<decltype(**p)>*)q;
     return BGPU_OK;

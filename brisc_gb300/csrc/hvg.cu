@@ -465,7 +465,7 @@ struct Scratch {  // stream-ordered device buffer, freed on the same stream
   ~Scratch() { if (p) cudaFreeAsync(p, s); }
   int alloc(size_t bytes, cudaStream_t stream) {
     s = stream;
-    cudaError_t e = cudaMallocAsync(&p, std::max<size_t>(bytes, 16), stream);
+    cudaError_t e = scratch_alloc(&p, std::max<size_t>(bytes, 16), stream);
     if (e != cudaSuccess) {
       p = nullptr;
       set_error(std::string("cudaMalloc(") + std::to_string(bytes) +

@@ -69,6 +69,46 @@ int device_smem_optin() {
   return cache[dev];
 }
 
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
+  static std::mutex mu;
+  static std::vector<cudaMemPool_t> pools;  // per device, for the process
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  cudaMemPool_t pool = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    if ((int)pools.size() <= dev) pools.resize(dev + 1, nullptr);
+    if (!pools[dev]) {
+      cudaMemPoolProps props{};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      cudaMemPool_t made = nullptr;
+      e = cudaMemPoolCreate(&made, &props);
+      if (e != cudaSuccess) return e;
+      uint64_t kept = kScratchKept;
+      int off = 0;
+      e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &kept);
+      if (e == cudaSuccess)
+        e = cudaMemPoolSetAttribute(made, cudaMemPoolReuseAllowInternalDependencies, &off);
+      if (e != cudaSuccess) {
+        cudaMemPoolDestroy(made);
+        return e;
+      }
+      pools[dev] = made;
+    }
+    pool = pools[dev];
+  }
+  e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+  if (e != cudaErrorMemoryAllocation) return e;
+  // what the pool keeps may be what is missing: give it back and try again
+  (void)cudaGetLastError();
+  cudaStreamSynchronize(s);
+  cudaMemPoolTrimTo(pool, 0);
+  return cudaMallocFromPoolAsync(p, bytes, pool, s);
+}
+
 // ---------------------------------------------------------------------------
 // PCG32 + Box-Muller start vector, restating brisc/cyutils.pyx:1153-1232 and
 // brisc/pca.pyx:801-806 operation for operation (float arithmetic as there).
@@ -123,7 +163,7 @@ struct Buf {
 int balloc(Buf& b, size_t bytes, bool zero, cudaStream_t s) {
   if (bytes == 0) bytes = 16;
   b.s = s;
-  cudaError_t e = cudaMallocAsync(&b.p, bytes, s);
+  cudaError_t e = scratch_alloc(&b.p, bytes, s);
   if (e != cudaSuccess) {
     b.p = nullptr;
     set_error(std::string("cudaMalloc(") + std::to_string(bytes) +

@@ -157,7 +157,7 @@ extern "C" int bgpu_knn_self(const float* X, const uint32_t* sorted_order,
   const size_t nb = round_up((size_t)nc * 4, 256), ob = round_up(((size_t)nc + 1) * 8, 256);
   unsigned char* mem = nullptr;
   const size_t rb = round_up((n + 1) * 4, 256);
-  BGPU_CUDA(cudaMallocAsync((void**)&mem, xb + cb + nb + ob + rb + 256, s));
+  BGPU_CUDA(scratch_alloc((void**)&mem, xb + cb + nb + ob + rb + 256, s));
   float* cn = (float*)(mem + xb + cb);
   uint64_t* coff = (uint64_t*)(mem + xb + cb + nb);
   uint32_t* replay = (uint32_t*)(mem + xb + cb + nb + ob);
@@ -364,13 +364,13 @@ extern "C" int bgpu_kmeans(const float* X, uint32_t* cluster_labels, float* cent
   const size_t cb = round_up(knn_operand_bytes(nc, d), 256);
   unsigned char* mem = nullptr;  // operands of the cells and the centroids, error word
   float *cn = nullptr, *sums = nullptr, *norms = cell_norms, *own_norms = nullptr;
-  BGPU_CUDA(cudaMallocAsync((void**)&didx, (size_t)nc * 4, s));
-  BGPU_CUDA(cudaMallocAsync((void**)&cn, (size_t)nc * 4, s));
-  BGPU_CUDA(cudaMallocAsync((void**)&sums, sums_bytes, s));
-  BGPU_CUDA(cudaMallocAsync((void**)&mem, xb + cb + 256, s));
+  BGPU_CUDA(scratch_alloc((void**)&didx, (size_t)nc * 4, s));
+  BGPU_CUDA(scratch_alloc((void**)&cn, (size_t)nc * 4, s));
+  BGPU_CUDA(scratch_alloc((void**)&sums, sums_bytes, s));
+  BGPU_CUDA(scratch_alloc((void**)&mem, xb + cb + 256, s));
   int* err = (int*)(mem + xb + cb);
   if (!norms) {
-    BGPU_CUDA(cudaMallocAsync((void**)&own_norms, n * 4, s));
+    BGPU_CUDA(scratch_alloc((void**)&own_norms, n * 4, s));
     norms = own_norms;
   }
   auto cleanup = [&]() {
@@ -415,7 +415,7 @@ extern "C" int bgpu_kmeans(const float* X, uint32_t* cluster_labels, float* cent
         if (hcount[c] == 0) empty.push_back(c);
       if (!empty.empty()) {  // relocate_empty_clusters (kmeans.pyx:747-820)
         float* dist = nullptr;
-        BGPU_CUDA(cudaMallocAsync((void**)&dist, n * 4, s));
+        BGPU_CUDA(scratch_alloc((void**)&dist, n * 4, s));
         k_km_assigned<<<(unsigned)ceil_div(n, 256), 256, 0, s>>>(X, cluster_labels, Cc,
                                                                   n, d, dist);
         std::vector<float> hd(n), hx, hcn(per);

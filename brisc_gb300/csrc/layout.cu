@@ -31,7 +31,7 @@ struct DevBuf {
   int alloc(size_t bytes, cudaStream_t stream) {
     if (bytes == 0) bytes = 16;
     s = stream;
-    cudaError_t e = cudaMallocAsync(&p, bytes, stream);
+    cudaError_t e = scratch_alloc(&p, bytes, stream);
     if (e != cudaSuccess) {
       p = nullptr;
       set_error(std::string("cudaMalloc(") + std::to_string(bytes) +

@@ -548,9 +548,9 @@ extern "C" int bgpu_small_svd(const float* B, uint32_t m, float* Ub, float* Sb,
   const size_t cnt = (size_t)m * (m + 1);
   double* Bd = nullptr;
   void* gwork = nullptr;
-  BGPU_CUDA(cudaMallocAsync((void**)&Bd, cnt * 8, s));
+  BGPU_CUDA(scratch_alloc((void**)&Bd, cnt * 8, s));
   if (jacobi_smem_bytes(m, true) > 220 * 1024)
-    BGPU_CUDA(cudaMallocAsync(&gwork, jacobi_global_bytes(m, true), s));
+    BGPU_CUDA(scratch_alloc(&gwork, jacobi_global_bytes(m, true), s));
   int rc = launch_float_to_double(B, cnt, Bd, s);
   if (rc == BGPU_OK)
     rc = launch_jacobi_svd(nullptr, Bd, m, Ub, Sb, Vbt, nullptr, nullptr, gwork,
