@@ -729,26 +729,29 @@ __global__ void k_check_indptr(const I* __restrict__ indptr, uint64_t n,
     atomicOr(err, kErrIndptr);
 }
 
-template <typename I>
-int check_indptr(const void* indptr, uint64_t n, cudaStream_t s) {
-  DevBuf e;
-  BGPU_TRY(e.alloc(sizeof(int), s));
-  BGPU_CUDA(cudaMemsetAsync(e.p, 0, sizeof(int), s));
-  k_check_indptr<I><<<grid_for(n + 1, 256), 256, 0, s>>>((const I*)indptr, n,
-                                                         (int*)e.p);
+// Launches the check; the kernels behind it do nothing where it set *err, and
+// the call reads *err once, at its end (indptr_status).
+int check_indptr(const void* indptr, int index_type, uint64_t n, DevBuf& err, cudaStream_t s) {
+  BGPU_TRY(err.alloc(sizeof(int), s));
+  BGPU_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), s));
+  if (index_type == BGPU_INDEX_I64)
+    k_check_indptr<int64_t><<<grid_for(n + 1, 256), 256, 0, s>>>((const int64_t*)indptr, n,
+                                                                 (int*)err.p);
+  else
+    k_check_indptr<int32_t><<<grid_for(n + 1, 256), 256, 0, s>>>((const int32_t*)indptr, n,
+                                                                 (int*)err.p);
   BGPU_CHECK_LAUNCH();
-  int herr = 0;
-  BGPU_CUDA(cudaMemcpyAsync(&herr, e.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-  BGPU_CUDA(cudaStreamSynchronize(s));
-  BGPU_REQUIRE(herr == 0, BGPU_ERR_INVALID,
-               "indptr must start at 0 and be non-decreasing");
   return BGPU_OK;
 }
 
-int check_indptr_any(const void* indptr, int index_type, uint64_t n,
-                     cudaStream_t s) {
-  return index_type == BGPU_INDEX_I64 ? check_indptr<int64_t>(indptr, n, s)
-                                      : check_indptr<int32_t>(indptr, n, s);
+int indptr_status(const DevBuf& err, cudaStream_t s) {
+  int herr = 0;
+  BGPU_CUDA(cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  BGPU_CUDA(cudaStreamSynchronize(s));
+  BGPU_REQUIRE((herr & kErrIndptr) == 0, BGPU_ERR_INVALID,
+               "indptr must start at 0 and be non-decreasing");
+  BGPU_REQUIRE(herr == 0, BGPU_ERR_INVALID, "a column index is outside [0, n_col)");
+  return BGPU_OK;
 }
 
 template <typename V>
@@ -757,24 +760,75 @@ __device__ __forceinline__ unsigned long long as_u64(V x) {
   return (unsigned long long)x;
 }
 
+template <typename V>
+__device__ __forceinline__ bool below_64k(V x) {
+  if constexpr (std::is_signed<V>::value) return x >= V(0) && x < V(65535);
+  else return x < V(65535);
+}
+
+// Row sums: a warp takes kSumRows rows at a time, the first kRowLoads loads of
+// each in flight together. Entries
+// below 65535 (any real counts) sum in 32 bits with one
+// hardware reduction; the 64-bit shuffles serve the rest. 200k x 2000 floats,
+// 19M entries: 86 us with a row at a time and 64-bit conversions and shuffles
+// throughout, 45 us.
+constexpr int kRowLoads = 4;
+constexpr int kSumRows = 4;
 template <typename I, typename V>
 __global__ void k_row_sums(const I* __restrict__ indptr, const V* __restrict__ values,
                            uint64_t n, const uint8_t* __restrict__ qc,
                            unsigned long long* __restrict__ row_sums,
-                           unsigned long long* __restrict__ totals /*[2]*/) {
+                           unsigned long long* __restrict__ totals /*[2]*/,
+                           const int* __restrict__ err) {
+  if (*err) return;
   const int lane = threadIdx.x & 31;
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
   unsigned long long tot = 0, nqc = 0;
-  for (uint64_t r = warp; r < n; r += nwarps) {
-    int64_t e0 = (int64_t)indptr[r], e1 = (int64_t)indptr[r + 1];
-    unsigned long long s = 0;
-    for (int64_t e = e0 + lane; e < e1; e += 32) s += as_u64(values[e]);
+  auto add = [&](V x, uint32_t& s32, unsigned long long& s) {
+    if (below_64k(x)) {
+      s32 += (uint32_t)x;
+      if (s32 >= (1u << 26)) {  // 32 lanes' sums stay within 32 bits
+        s += s32;
+        s32 = 0;
+      }
+    } else {
+      s += as_u64(x);
+    }
+  };
+  for (uint64_t r0 = warp * kSumRows; r0 < n; r0 += nwarps * kSumRows) {
+    int64_t bound = 0;
+    if (lane <= kSumRows) bound = (int64_t)indptr[min_u64(r0 + lane, n)];
+    V x[kSumRows][kRowLoads];  // the first 32 kRowLoads entries of every row
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) {
-      row_sums[r] = s;
-      if (!qc || qc[r]) { tot += s; nqc += 1; }
+    for (int k = 0; k < kSumRows; ++k) {
+      const int64_t e0 = __shfl_sync(0xffffffffu, bound, k) + lane;
+      const int64_t e1 = __shfl_sync(0xffffffffu, bound, k + 1);
+#pragma unroll
+      for (int i = 0; i < kRowLoads; ++i)
+        x[k][i] = e0 + 32 * i < e1 ? values[e0 + 32 * i] : V(0);
+    }
+#pragma unroll
+    for (int k = 0; k < kSumRows; ++k) {
+      const int64_t e0 = __shfl_sync(0xffffffffu, bound, k);
+      const int64_t e1 = __shfl_sync(0xffffffffu, bound, k + 1);
+      const uint64_t r = r0 + k;
+      if (r >= n) break;
+      unsigned long long s = 0;
+      uint32_t s32 = 0;
+#pragma unroll
+      for (int i = 0; i < kRowLoads; ++i) add(x[k][i], s32, s);
+      for (int64_t e = e0 + 32 * kRowLoads + lane; e < e1; e += 32) add(values[e], s32, s);
+      unsigned long long sum = __reduce_add_sync(0xffffffffu, s32);
+      if (__any_sync(0xffffffffu, s != 0ull)) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        sum += s;
+      }
+      if (lane == 0) {
+        row_sums[r] = sum;
+        if (!qc || qc[r]) { tot += sum; nqc += 1; }
+      }
     }
   }
   if (lane == 0 && (tot || nqc)) {
@@ -785,9 +839,9 @@ __global__ void k_row_sums(const I* __restrict__ indptr, const V* __restrict__ v
 
 __global__ void k_isf(const unsigned long long* __restrict__ row_sums, uint64_t n,
                       int method, const unsigned long long* __restrict__ totals,
-                      float* __restrict__ isf) {
+                      float* __restrict__ isf, const int* __restrict__ err) {
   uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n || *err) return;
   float nf;
   if (method == 0) {
     nf = 10000.f;  // normalize.pyx:55
@@ -802,7 +856,8 @@ __global__ void k_isf(const unsigned long long* __restrict__ row_sums, uint64_t 
 template <typename I, typename V>
 __global__ void k_new_row_sums(const I* __restrict__ indptr, const V* __restrict__ values,
                                uint64_t n, const float* __restrict__ isf,
-                               float* __restrict__ nrs) {
+                               float* __restrict__ nrs, const int* __restrict__ err) {
+  if (*err) return;
   const int lane = threadIdx.x & 31;
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
@@ -838,8 +893,9 @@ __global__ void k_block_float_sum(const float* __restrict__ x, uint64_t n,
 __global__ void k_post(const float* __restrict__ partial, uint32_t nblocks,
                        const unsigned long long* __restrict__ totals,
                        const float* __restrict__ nrs, uint64_t n,
-                       float* __restrict__ post) {
+                       float* __restrict__ post, const int* __restrict__ err) {
   __shared__ float nf2;
+  if (*err) return;
   if (threadIdx.x == 0) {
     float t = 0.f;
     for (uint32_t b = 0; b < nblocks; ++b) t += partial[b];
@@ -854,7 +910,9 @@ __global__ void k_post(const float* __restrict__ partial, uint32_t nblocks,
 template <typename I, typename V>
 __global__ void k_normalize(const I* __restrict__ indptr, const V* __restrict__ values,
                             uint64_t n, const float* __restrict__ isf,
-                            const float* __restrict__ post, float* __restrict__ out) {
+                            const float* __restrict__ post, float* __restrict__ out,
+                            const int* __restrict__ err) {
+  if (*err) return;
   const int lane = threadIdx.x & 31;
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
@@ -862,9 +920,17 @@ __global__ void k_normalize(const I* __restrict__ indptr, const V* __restrict__ 
     int64_t e0 = (int64_t)indptr[r], e1 = (int64_t)indptr[r + 1];
     const float f = isf[r];
     const float q = post ? post[r] : 1.f;
-    for (int64_t e = e0 + lane; e < e1; e += 32) {
-      float v = log1pf((float)values[e] * f);
-      out[e] = post ? v * q : v;
+    for (int64_t e = e0 + lane; e < e1; e += 32 * kRowLoads) {
+      float x[kRowLoads];
+#pragma unroll
+      for (int i = 0; i < kRowLoads; ++i)
+        x[i] = e + 32 * i < e1 ? (float)values[e + 32 * i] : 0.f;
+#pragma unroll
+      for (int i = 0; i < kRowLoads; ++i) {
+        if (e + 32 * i >= e1) break;
+        const float v = log1pf(x[i] * f);
+        out[e + 32 * i] = post ? v * q : v;
+      }
     }
   }
 }
@@ -872,7 +938,8 @@ __global__ void k_normalize(const I* __restrict__ indptr, const V* __restrict__ 
 template <typename I, typename V>
 int size_factors_typed(const void* indptr, const void* values, uint64_t n,
                        int method, const uint8_t* qc, float* isf, float* post,
-                       uint64_t* row_sums_out, cudaStream_t s) {
+                       uint64_t* row_sums_out, const DevBuf& err, cudaStream_t s) {
+  const int* bad = (const int*)err.p;
   DevBuf t_rs, t_tot, t_nrs, t_part;
   unsigned long long* rs = (unsigned long long*)row_sums_out;
   if (!rs) {
@@ -885,65 +952,65 @@ int size_factors_typed(const void* indptr, const void* values, uint64_t n,
   int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(n, 8),
                                                             (uint64_t)num_sms() * 16));
   k_row_sums<I, V><<<blocks, 256, 0, s>>>((const I*)indptr, (const V*)values, n,
-                                          qc, rs, tot);
+                                          qc, rs, tot, bad);
   BGPU_CHECK_LAUNCH();
-  k_isf<<<grid_for(n, 256), 256, 0, s>>>(rs, n, method, tot, isf);
+  k_isf<<<grid_for(n, 256), 256, 0, s>>>(rs, n, method, tot, isf, bad);
   BGPU_CHECK_LAUNCH();
   if (method == 2) {
     BGPU_TRY(t_nrs.alloc(n * 4, s));
     float* nrs = (float*)t_nrs.p;
     k_new_row_sums<I, V><<<blocks, 256, 0, s>>>((const I*)indptr,
-                                                (const V*)values, n, isf, nrs);
+                                                (const V*)values, n, isf, nrs, bad);
     BGPU_CHECK_LAUNCH();
     uint32_t nb = (uint32_t)ceil_div(n, 1024);
     BGPU_TRY(t_part.alloc(nb * 4, s));
     k_block_float_sum<<<nb, 1024, 0, s>>>(nrs, n, qc, (float*)t_part.p);
     BGPU_CHECK_LAUNCH();
     k_post<<<grid_for(n, 256, 4096), 256, 0, s>>>((const float*)t_part.p, nb,
-                                                  tot, nrs, n, post);
+                                                  tot, nrs, n, post, bad);
     BGPU_CHECK_LAUNCH();
   }
-  BGPU_CUDA(cudaStreamSynchronize(s));
-  return BGPU_OK;
+  return indptr_status(err, s);
 }
 
 template <typename I>
 int size_factors_by_value(const void* indptr, int vt, const void* values,
                           uint64_t n, int method, const uint8_t* qc, float* isf,
-                          float* post, uint64_t* rs, cudaStream_t s) {
+                          float* post, uint64_t* rs, const DevBuf& err, cudaStream_t s) {
   switch (vt) {
     case BGPU_VALUE_U16:
-      return size_factors_typed<I, uint16_t>(indptr, values, n, method, qc, isf, post, rs, s);
+      return size_factors_typed<I, uint16_t>(indptr, values, n, method, qc, isf, post, rs, err, s);
     case BGPU_VALUE_U32:
-      return size_factors_typed<I, uint32_t>(indptr, values, n, method, qc, isf, post, rs, s);
+      return size_factors_typed<I, uint32_t>(indptr, values, n, method, qc, isf, post, rs, err, s);
     case BGPU_VALUE_I32:
-      return size_factors_typed<I, int32_t>(indptr, values, n, method, qc, isf, post, rs, s);
+      return size_factors_typed<I, int32_t>(indptr, values, n, method, qc, isf, post, rs, err, s);
     default:
-      return size_factors_typed<I, float>(indptr, values, n, method, qc, isf, post, rs, s);
+      return size_factors_typed<I, float>(indptr, values, n, method, qc, isf, post, rs, err, s);
   }
 }
 
 template <typename I>
 int normalize_by_value(const void* indptr, int vt, const void* values,
                        uint64_t n, const float* isf, const float* post,
-                       float* out, cudaStream_t s) {
+                       float* out, const DevBuf& err, cudaStream_t s) {
+  const int* bad = (const int*)err.p;
   int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(n, 8),
                                                             (uint64_t)num_sms() * 16));
   switch (vt) {
     case BGPU_VALUE_U16:
-      k_normalize<I, uint16_t><<<blocks, 256, 0, s>>>((const I*)indptr, (const uint16_t*)values, n, isf, post, out);
+      k_normalize<I, uint16_t><<<blocks, 256, 0, s>>>((const I*)indptr, (const uint16_t*)values, n, isf, post, out, bad);
       break;
     case BGPU_VALUE_U32:
-      k_normalize<I, uint32_t><<<blocks, 256, 0, s>>>((const I*)indptr, (const uint32_t*)values, n, isf, post, out);
+      k_normalize<I, uint32_t><<<blocks, 256, 0, s>>>((const I*)indptr, (const uint32_t*)values, n, isf, post, out, bad);
       break;
     case BGPU_VALUE_I32:
-      k_normalize<I, int32_t><<<blocks, 256, 0, s>>>((const I*)indptr, (const int32_t*)values, n, isf, post, out);
+      k_normalize<I, int32_t><<<blocks, 256, 0, s>>>((const I*)indptr, (const int32_t*)values, n, isf, post, out, bad);
       break;
     default:
-      k_normalize<I, float><<<blocks, 256, 0, s>>>((const I*)indptr, (const float*)values, n, isf, post, out);
+      k_normalize<I, float><<<blocks, 256, 0, s>>>((const I*)indptr, (const float*)values, n, isf, post, out, bad);
   }
   BGPU_CHECK_LAUNCH();
-  return BGPU_OK;
+  return indptr_status(err, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -952,6 +1019,7 @@ template <typename I>
 __global__ void k_global_hist(const I* __restrict__ Ap, const I* __restrict__ Aj,
                               uint64_t n, uint32_t g, uint32_t num_sub,
                               long long* __restrict__ cnt, int* err) {
+  if (*err & kErrIndptr) return;
   const int lane = threadIdx.x & 31;
   const uint64_t s = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   if (s >= num_sub) return;
@@ -969,7 +1037,8 @@ __global__ void k_global_scatter(const I* __restrict__ Ap, const I* __restrict__
                                  const uint32_t* __restrict__ Ax, uint64_t n,
                                  uint32_t g, uint32_t num_sub,
                                  long long* __restrict__ cnt, I* __restrict__ Bi,
-                                 uint32_t* __restrict__ Bx) {
+                                 uint32_t* __restrict__ Bx, const int* __restrict__ err) {
+  if (*err) return;
   const int lane = threadIdx.x & 31;
   const uint64_t s = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   if (s >= num_sub) return;
@@ -989,41 +1058,206 @@ __global__ void k_global_scatter(const I* __restrict__ Ap, const I* __restrict__
 
 template <typename I>
 __global__ void k_store_bp(const long long* __restrict__ cp, I* __restrict__ Bp,
-                           uint32_t g) {
+                           uint32_t g, const int* __restrict__ err) {
   uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c <= g) Bp[c] = (I)cp[c];
+  if (c <= g && !*err) Bp[c] = (I)cp[c];
+}
+
+// The transpose for up to kTrGenes columns. A CTA takes a run of rows
+// (a sub-block), its eight warps consecutive parts of it:
+//  k_tr_hist     the sub-block's entries per column, in shared memory;
+//  k_tr_offsets  per column, the entries of the sub-blocks before each
+//                (in place) and the column's total;
+//  k_panel_scan  the columns' first positions (one row of totals);
+//  k_tr_scatter  every entry to its place. Each warp counts its own part per
+//                column in shared memory, the warps' starts follow, and the
+//                warp walks its entries in storage order, 32 at a time;
+//                entries of one column among the 32 are ranked by lane, so
+//                rows ascend within each column.
+// Sub-blocks are short so that the CTAs at work fill short stretches of each
+// column at the same time: the 4-byte stores of a 32-byte sector then meet in
+// L2. With one wave of long sub-blocks (439 rows) the scatter took 773 us, with
+// 128 rows 551, with 64 rows 330 (200k x 2000, 19M entries). One warp per 256
+// rows with global counters, and one CTA to scan them, took 2.05 ms in all, this
+// 0.40 ms. More columns than fit take that path.
+constexpr uint32_t kTrGenes = 6144;
+constexpr uint64_t kTrRows = 64;
+constexpr int kTrThreads = 256;
+constexpr int kTrWarps = kTrThreads / 32;
+constexpr int kTrLoads = 4;
+
+template <typename I>
+__global__ void __launch_bounds__(kTrThreads)
+k_tr_hist(const I* __restrict__ Ap, const I* __restrict__ Aj, uint64_t n, uint32_t g,
+          uint64_t rows_per, uint32_t* __restrict__ cnt, int* __restrict__ err) {
+  extern __shared__ uint32_t h[];
+  if (*err & kErrIndptr) return;
+  for (uint32_t c = threadIdx.x; c < g; c += kTrThreads) h[c] = 0u;
+  __syncthreads();
+  const uint64_t r0 = blockIdx.x * rows_per, r1 = min_u64(n, r0 + rows_per);
+  const int64_t e0 = (int64_t)Ap[r0], e1 = (int64_t)Ap[r1];
+  bool bad = false;
+  for (int64_t e = e0 + threadIdx.x; e < e1; e += kTrThreads * kTrLoads) {
+    I c[kTrLoads];
+#pragma unroll
+    for (int i = 0; i < kTrLoads; ++i)
+      c[i] = e + kTrThreads * i < e1 ? Aj[e + kTrThreads * i] : I(-1);
+#pragma unroll
+    for (int i = 0; i < kTrLoads; ++i) {
+      if (e + kTrThreads * i >= e1) break;
+      if (c[i] < 0 || (int64_t)c[i] >= (int64_t)g) bad = true;
+      else atomicAdd(&h[c[i]], 1u);
+    }
+  }
+  if (bad) atomicOr(err, kErrIndex);
+  __syncthreads();
+  for (uint32_t c = threadIdx.x; c < g; c += kTrThreads)
+    cnt[(uint64_t)blockIdx.x * g + c] = h[c];
+}
+
+// A block takes 32 columns (lane = column), its 32 warps runs of sub-blocks.
+__global__ void __launch_bounds__(1024)
+k_tr_offsets(uint32_t* __restrict__ cnt, uint32_t num_sub, uint32_t g,
+             long long* __restrict__ totals, const int* __restrict__ err) {
+  __shared__ uint32_t part[32][33];
+  if (*err) return;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint32_t c = blockIdx.x * 32 + lane;
+  const uint32_t per = (num_sub + 31) / 32;
+  const uint32_t s0 = min(num_sub, wid * per), s1 = min(num_sub, s0 + per);
+  uint32_t t = 0;
+  if (c < g) {
+#pragma unroll 8
+    for (uint32_t s = s0; s < s1; ++s) t += cnt[(uint64_t)s * g + c];
+  }
+  part[wid][lane] = t;
+  __syncthreads();
+  uint32_t run = 0;
+  long long total = 0;
+  for (int w = 0; w < 32; ++w) {
+    if (w < wid) run += part[w][lane];
+    total += part[w][lane];
+  }
+  if (c >= g) return;
+  if (wid == 0) totals[c] = total;
+#pragma unroll 8
+  for (uint32_t s = s0; s < s1; ++s) {
+    const uint32_t v = cnt[(uint64_t)s * g + c];
+    cnt[(uint64_t)s * g + c] = run;
+    run += v;
+  }
+}
+
+template <typename I>
+__global__ void __launch_bounds__(kTrThreads)
+k_tr_scatter(const I* __restrict__ Ap, const I* __restrict__ Aj,
+             const uint32_t* __restrict__ Ax, uint64_t n, uint32_t g, uint64_t rows_per,
+             const uint32_t* __restrict__ cnt, const long long* __restrict__ start,
+             I* __restrict__ Bi, uint32_t* __restrict__ Bx, const int* __restrict__ err) {
+  extern __shared__ uint32_t wc[];  // [warp][column]
+  if (*err) return;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (uint32_t c = threadIdx.x; c < kTrWarps * g; c += kTrThreads) wc[c] = 0u;
+  __syncthreads();
+  const uint64_t r0 = blockIdx.x * rows_per, r1 = min_u64(n, r0 + rows_per);
+  const uint64_t per = (r1 - r0 + kTrWarps - 1) / kTrWarps;
+  const uint64_t ra = min_u64(r1, r0 + wid * per), rb = min_u64(r1, ra + per);
+  const int64_t e0 = (int64_t)Ap[ra], e1 = (int64_t)Ap[rb];
+  uint32_t* my = wc + (uint64_t)wid * g;
+#pragma unroll 4
+  for (int64_t e = e0 + lane; e < e1; e += 32) atomicAdd(&my[Aj[e]], 1u);
+  __syncthreads();
+  for (uint32_t c = threadIdx.x; c < g; c += kTrThreads) {
+    uint32_t run = cnt[(uint64_t)blockIdx.x * g + c];
+#pragma unroll
+    for (int w = 0; w < kTrWarps; ++w) {
+      const uint32_t t = wc[(uint64_t)w * g + c];
+      wc[(uint64_t)w * g + c] = run;
+      run += t;
+    }
+  }
+  __syncthreads();
+  uint64_t r = ra;  // the row of this lane's entry
+  int64_t rend = ra < rb ? (int64_t)Ap[ra + 1] : e1;
+  for (int64_t eb = e0; eb < e1; eb += 32 * kTrLoads) {
+    uint32_t c[kTrLoads], x[kTrLoads];
+#pragma unroll
+    for (int i = 0; i < kTrLoads; ++i) {
+      const int64_t e = eb + 32 * i + lane;
+      c[i] = e < e1 ? (uint32_t)Aj[e] : 0xFFFFFFFFu;
+      x[i] = e < e1 ? Ax[e] : 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < kTrLoads; ++i) {
+      const int64_t e = eb + 32 * i + lane;
+      if (eb + 32 * i >= e1) break;
+      while (e < e1 && e >= rend) rend = (int64_t)Ap[++r + 1];
+      const uint32_t peers = __match_any_sync(0xffffffffu, c[i]);
+      const int leader = __ffs(peers) - 1;
+      uint32_t slot = 0;
+      if (lane == leader && c[i] != 0xFFFFFFFFu) {
+        slot = my[c[i]];
+        my[c[i]] = slot + __popc(peers);
+      }
+      slot = __shfl_sync(0xffffffffu, slot, leader) + __popc(peers & ((1u << lane) - 1u));
+      if (c[i] != 0xFFFFFFFFu) {
+        const int64_t dst = start[c[i]] + slot;
+        Bi[dst] = (I)r;
+        Bx[dst] = x[i];
+      }
+      __syncwarp();
+    }
+  }
 }
 
 template <typename I>
 int csr_tocsc_typed(uint64_t n, uint32_t g, const void* Ap, const void* Aj,
-                    const void* Ax, void* Bp, void* Bi, void* Bx, cudaStream_t s) {
-  const uint32_t num_sub = (uint32_t)ceil_div(n, kSubRows);
-  DevBuf t_cnt, t_cp, t_err;
-  BGPU_TRY(t_cnt.alloc((size_t)num_sub * g * 8, s));
+                    const void* Ax, void* Bp, void* Bi, void* Bx, const DevBuf& err,
+                    cudaStream_t s) {
+  int* bad = (int*)err.p;
+  DevBuf t_cnt, t_cp;
   BGPU_TRY(t_cp.alloc((size_t)(g + 1) * 8, s));
-  BGPU_TRY(t_err.alloc(4, s));
-  long long* cnt = (long long*)t_cnt.p;
-  BGPU_CUDA(cudaMemsetAsync(cnt, 0, (size_t)num_sub * g * 8, s));
-  BGPU_CUDA(cudaMemsetAsync(t_err.p, 0, 4, s));
-  const int wblocks = (int)ceil_div(num_sub, 8);
-  k_global_hist<I><<<wblocks, 256, 0, s>>>((const I*)Ap, (const I*)Aj, n, g,
-                                           num_sub, cnt, (int*)t_err.p);
+  long long* cp = (long long*)t_cp.p;
+  if (g <= kTrGenes) {
+    const size_t smem = (size_t)kTrWarps * g * 4;
+    const uint64_t rows_per = kTrRows;
+    const uint32_t num_sub = (uint32_t)ceil_div(n, rows_per);
+    DevBuf t_tot;
+    BGPU_TRY(t_cnt.alloc((size_t)num_sub * g * 4, s));
+    BGPU_TRY(t_tot.alloc((size_t)g * 8, s));
+    uint32_t* cnt = (uint32_t*)t_cnt.p;
+    BGPU_CUDA((allow_max_smem(k_tr_scatter<I>)));
+    k_tr_hist<I><<<num_sub, kTrThreads, g * 4, s>>>((const I*)Ap, (const I*)Aj, n, g, rows_per,
+                                                    cnt, bad);
+    BGPU_CHECK_LAUNCH();
+    k_tr_offsets<<<(unsigned)ceil_div(g, 32), 1024, 0, s>>>(cnt, num_sub, g,
+                                                           (long long*)t_tot.p, bad);
+    BGPU_CHECK_LAUNCH();
+    k_panel_scan<long long><<<1, 1024, 0, s>>>((long long*)t_tot.p, cp, g, 1, 1);
+    BGPU_CHECK_LAUNCH();
+    k_tr_scatter<I><<<num_sub, kTrThreads, smem, s>>>((const I*)Ap, (const I*)Aj,
+                                                      (const uint32_t*)Ax, n, g, rows_per, cnt,
+                                                      cp, (I*)Bi, (uint32_t*)Bx, bad);
+    BGPU_CHECK_LAUNCH();
+  } else {
+    const uint32_t num_sub = (uint32_t)ceil_div(n, kSubRows);
+    BGPU_TRY(t_cnt.alloc((size_t)num_sub * g * 8, s));
+    long long* cnt = (long long*)t_cnt.p;
+    BGPU_CUDA(cudaMemsetAsync(cnt, 0, (size_t)num_sub * g * 8, s));
+    const int wblocks = (int)ceil_div(num_sub, 8);
+    k_global_hist<I><<<wblocks, 256, 0, s>>>((const I*)Ap, (const I*)Aj, n, g, num_sub, cnt,
+                                             bad);
+    BGPU_CHECK_LAUNCH();
+    k_panel_scan<long long><<<1, 1024, 0, s>>>(cnt, cp, g, num_sub, num_sub);
+    BGPU_CHECK_LAUNCH();
+    k_global_scatter<I><<<wblocks, 256, 0, s>>>((const I*)Ap, (const I*)Aj,
+                                                (const uint32_t*)Ax, n, g, num_sub, cnt,
+                                                (I*)Bi, (uint32_t*)Bx, bad);
+    BGPU_CHECK_LAUNCH();
+  }
+  k_store_bp<I><<<grid_for(g + 1, 256), 256, 0, s>>>(cp, (I*)Bp, g, bad);
   BGPU_CHECK_LAUNCH();
-  k_panel_scan<long long><<<1, 1024, 0, s>>>(cnt, (long long*)t_cp.p, g, num_sub,
-                                             num_sub);
-  BGPU_CHECK_LAUNCH();
-  k_global_scatter<I><<<wblocks, 256, 0, s>>>((const I*)Ap, (const I*)Aj,
-                                              (const uint32_t*)Ax, n, g, num_sub,
-                                              cnt, (I*)Bi, (uint32_t*)Bx);
-  BGPU_CHECK_LAUNCH();
-  k_store_bp<I><<<grid_for(g + 1, 256), 256, 0, s>>>((const long long*)t_cp.p,
-                                                     (I*)Bp, g);
-  BGPU_CHECK_LAUNCH();
-  int herr = 0;
-  BGPU_CUDA(cudaMemcpyAsync(&herr, t_err.p, 4, cudaMemcpyDeviceToHost, s));
-  BGPU_CUDA(cudaStreamSynchronize(s));
-  BGPU_REQUIRE(herr == 0, BGPU_ERR_INVALID, "a column index is outside [0, n_col)");
-  return BGPU_OK;
+  return indptr_status(err, s);
 }
 
 }  // namespace
@@ -1043,12 +1277,13 @@ extern "C" int bgpu_size_factors(const void* indptr, int index_type,
   BGPU_REQUIRE(method != 2 || post, BGPU_ERR_INVALID, "method 2 needs `post`");
   BGPU_REQUIRE(num_cells >= 1, BGPU_ERR_INVALID, "num_cells must be positive");
   cudaStream_t s = (cudaStream_t)stream;
-  BGPU_TRY(check_indptr_any(indptr, index_type, num_cells, s));
+  DevBuf err;
+  BGPU_TRY(check_indptr(indptr, index_type, num_cells, err, s));
   if (index_type == BGPU_INDEX_I64)
     return size_factors_by_value<int64_t>(indptr, value_type, values, num_cells,
-                                          method, qc_mask, isf, post, row_sums, s);
+                                          method, qc_mask, isf, post, row_sums, err, s);
   return size_factors_by_value<int32_t>(indptr, value_type, values, num_cells,
-                                        method, qc_mask, isf, post, row_sums, s);
+                                        method, qc_mask, isf, post, row_sums, err, s);
 }
 
 extern "C" int bgpu_normalize_csr(const void* indptr, int index_type,
@@ -1059,12 +1294,13 @@ extern "C" int bgpu_normalize_csr(const void* indptr, int index_type,
   BGPU_REQUIRE(indptr && values && isf && normalized, BGPU_ERR_INVALID,
                "indptr, values, isf and normalized must not be NULL");
   cudaStream_t s = (cudaStream_t)stream;
-  BGPU_TRY(check_indptr_any(indptr, index_type, num_cells, s));
+  DevBuf err;
+  BGPU_TRY(check_indptr(indptr, index_type, num_cells, err, s));
   if (index_type == BGPU_INDEX_I64)
     return normalize_by_value<int64_t>(indptr, value_type, values, num_cells,
-                                       isf, post, normalized, s);
+                                       isf, post, normalized, err, s);
   return normalize_by_value<int32_t>(indptr, value_type, values, num_cells, isf,
-                                     post, normalized, s);
+                                     post, normalized, err, s);
 }
 
 extern "C" int bgpu_csr_tocsc(uint64_t n_row, uint32_t n_col, const void* Ap,
@@ -1073,8 +1309,9 @@ extern "C" int bgpu_csr_tocsc(uint64_t n_row, uint32_t n_col, const void* Ap,
   BGPU_REQUIRE(Ap && Bp && n_row >= 1 && n_col >= 1, BGPU_ERR_INVALID,
                "bad csr_tocsc arguments");
   cudaStream_t s = (cudaStream_t)stream;
-  BGPU_TRY(check_indptr_any(Ap, index_type, n_row, s));
+  DevBuf err;
+  BGPU_TRY(check_indptr(Ap, index_type, n_row, err, s));
   if (index_type == BGPU_INDEX_I64)
-    return csr_tocsc_typed<int64_t>(n_row, n_col, Ap, Aj, Ax, Bp, Bi, Bx, s);
-  return csr_tocsc_typed<int32_t>(n_row, n_col, Ap, Aj, Ax, Bp, Bi, Bx, s);
+    return csr_tocsc_typed<int64_t>(n_row, n_col, Ap, Aj, Ax, Bp, Bi, Bx, err, s);
+  return csr_tocsc_typed<int32_t>(n_row, n_col, Ap, Aj, Ax, Bp, Bi, Bx, err, s);
 }

@@ -337,3 +337,57 @@ def test_gene_stddev_of_any_scale(cuda, n, g, density, scale):
             else np.zeros(g)
     want = np.maximum(np.nan_to_num(want), 1e-8)
     np.testing.assert_allclose(sd.cpu().numpy(), want.astype(np.float32), rtol=1e-6)
+
+
+@pytest.mark.parametrize("itype", [np.int32, np.int64])
+@pytest.mark.parametrize("n,g", [(1, 1), (63, 31), (64, 33), (65, 6144), (40000, 37), (3000, 6145),
+                                 (20000, 2000)])
+def test_csr_tocsc_rows_ascend(cuda, n, g, itype):
+    """The transpose around its sub-blocks of rows and the columns that fit
+    shared memory, with empty rows and columns, long rows and repeated columns
+    in a row: bit for bit a stable sort of the entries by column."""
+    import torch
+    rng = np.random.default_rng(n + g)
+    lens = rng.integers(0, min(g, 40) + 1, n)
+    lens[rng.integers(0, n, max(1, n // 50))] = rng.integers(0, 3 * min(g, 300) + 1)
+    ip = np.concatenate([[0], np.cumsum(lens)]).astype(itype)
+    ix = rng.integers(0, max(1, g - g // 7), int(ip[-1])).astype(itype)
+    x = rng.integers(0, 2**31, ix.size).astype(np.int32)
+    rows = np.repeat(np.arange(n), lens)
+    order = np.argsort(ix, kind="stable")
+    dip, dix, dx = (torch.from_numpy(a).to(cuda) for a in (ip, ix, x))
+    bp = torch.empty(g + 1, dtype=dip.dtype, device=cuda)
+    bi, bx = torch.empty_like(dix), torch.empty_like(dx)
+    _lib.call("bgpu_csr_tocsc", n, g, dip.data_ptr(), dix.data_ptr(), dx.data_ptr(),
+              _lib.INDEX_I32 if itype == np.int32 else _lib.INDEX_I64, bp.data_ptr(),
+              bi.data_ptr(), bx.data_ptr(), None)
+    assert np.array_equal(bp.cpu().numpy(),
+                          np.concatenate([[0], np.cumsum(np.bincount(ix, minlength=g))]))
+    if g > 6144:  # entries of one row and column may change places there
+        key = lambda c, r, v: sorted(zip(c.tolist(), r.tolist(), v.tolist()))  # noqa: E731
+        c = np.repeat(np.arange(g), np.bincount(ix, minlength=g))
+        assert key(c, bi.cpu().numpy(), bx.cpu().numpy()) == key(ix, rows, x)
+        return
+    assert np.array_equal(bi.cpu().numpy(), rows[order])
+    assert np.array_equal(bx.cpu().numpy(), x[order])
+
+
+@pytest.mark.parametrize("vtype", ["uint16", "int32", "float32"])
+def test_row_sums_of_large_values(cuda, vtype):
+    """Row sums whose entries and totals cross 2^16, 2^26 and 2^32, exactly."""
+    import torch
+    rng = np.random.default_rng(5)
+    top = {"uint16": 65535, "int32": 2**31 - 1, "float32": 2**24}[vtype]
+    lens = np.array([0, 1, 2, 31, 32, 33, 127, 128, 129, 5000, 40000])
+    ip = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    v = np.where(rng.random(ip[-1]) < 0.5, top - rng.integers(0, 3, ip[-1]),
+                 rng.integers(0, 65536, ip[-1])).astype(vtype)
+    dv = torch.from_numpy(v.view(np.int16) if vtype == "uint16" else v).to(cuda)
+    dip = torch.from_numpy(ip).to(cuda)
+    isf = torch.empty(len(lens), dtype=torch.float32, device=cuda)
+    rs = torch.empty(len(lens), dtype=torch.int64, device=cuda)
+    vt = {"uint16": _lib.VALUE_U16, "int32": _lib.VALUE_I32, "float32": _lib.VALUE_F32}[vtype]
+    _lib.call("bgpu_size_factors", dip.data_ptr(), _lib.INDEX_I64, dv.data_ptr(), vt, len(lens),
+              0, None, isf.data_ptr(), None, rs.data_ptr(), None)
+    want = [int(v[a:b].astype(np.int64).sum()) for a, b in zip(ip[:-1], ip[1:])]
+    assert rs.cpu().tolist() == want
