@@ -137,6 +137,37 @@ __device__ __forceinline__ float group_sum(float v) {
   return v;
 }
 
+// Programmatic dependent launch. A kernel launched with launch_pdl may start
+// while the one before it in the stream still runs: what it does before
+// pdl_wait() overlaps that kernel (and hides its own launch). pdl_wait()
+// returns when the kernel before has completed and its writes are visible;
+// pdl_trigger(), called right behind it, lets the next kernel start the same
+// way. So before its pdl_wait() a kernel may read what kernels at least two
+// before it wrote, and must not write anything. Both do nothing in a kernel
+// that was launched without the attribute.
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                              cudaStream_t s, A&&... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
 // Streaming 128-bit load that bypasses L1 (the matrix is read once per pass).
 __device__ __forceinline__ uint4 ld_stream_u4(const void* p) {
   uint4 r;

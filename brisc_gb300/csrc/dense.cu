@@ -46,13 +46,15 @@ __device__ __forceinline__ bool second_pass_skipped(const float* gate) {
 // __launch_bounds__(256, 8): 32 registers, so the 1024-row blocks of a
 // million-cell basis (977) all run in one wave (8 per SM, 2048 threads, each
 // with kDotCols 16-byte loads in flight).
+// Few blocks (small n) leave SMs idle, so [c_lo, c_hi) can be a part of the
+// columns: the launch splits them over blockIdx.y.
 constexpr int kDotCols = 4;
 
 __device__ __forceinline__ void udots_body(const float* __restrict__ U, uint64_t ldu,
                                            uint32_t ncols, const float* __restrict__ y,
                                            float* __restrict__ part, uint32_t pstride,
                                            int with_sum, const float* __restrict__ gate,
-                                           uint64_t b) {
+                                           uint64_t b, uint32_t c_lo, uint32_t c_hi) {
   if (second_pass_skipped(gate)) return;
   extern __shared__ float wsum[];  // 8 x (ncols + 1)
   const uint32_t ld = ncols + 1;
@@ -65,13 +67,13 @@ __device__ __forceinline__ void udots_body(const float* __restrict__ U, uint64_t
     const float s = warp_sum(yv.x + yv.y + yv.z + yv.w);
     if (lane == 0) wsum[wid * ld + ncols] = s;
   }
-  for (uint32_t c0 = 0; c0 < ncols; c0 += kDotCols) {
+  for (uint32_t c0 = c_lo; c0 < c_hi; c0 += kDotCols) {
     float acc[kDotCols];
 #pragma unroll
     for (int k = 0; k < kDotCols; ++k) {
       const uint32_t c = c0 + k;
       acc[k] = 0.f;
-      if (in && c < ncols) {
+      if (in && c < c_hi) {
         const float4 u = __ldcs(reinterpret_cast<const float4*>(U + c * ldu + row0));
         acc[k] = dot4(u, yv);
       }
@@ -81,24 +83,29 @@ __device__ __forceinline__ void udots_body(const float* __restrict__ U, uint64_t
     if (lane == 0) {
 #pragma unroll
       for (int k = 0; k < kDotCols; ++k)
-        if (c0 + k < ncols) wsum[wid * ld + c0 + k] = acc[k];
+        if (c0 + k < c_hi) wsum[wid * ld + c0 + k] = acc[k];
     }
   }
   __syncthreads();
-  const uint32_t nout = ncols + (with_sum ? 1u : 0u);
-  for (uint32_t c = threadIdx.x; c < nout; c += blockDim.x) {
+  const uint32_t nout = c_hi + (with_sum ? 1u : 0u);
+  for (uint32_t c = c_lo + threadIdx.x; c < nout; c += blockDim.x) {
+    const uint32_t col = c < c_hi ? c : ncols;  // the last one is the sum of y
     float t = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) t += wsum[w * ld + c];
-    part[b * pstride + c] = t;
+    for (int w = 0; w < 8; ++w) t += wsum[w * ld + col];
+    part[b * pstride + col] = t;
   }
 }
 
 __global__ void __launch_bounds__(256, 8)
 k_udots(const float* __restrict__ U, uint64_t ldu, uint32_t ncols,
         const float* __restrict__ y, float* __restrict__ part,
-        uint32_t pstride, int with_sum, const float* __restrict__ gate) {
-  udots_body(U, ldu, ncols, y, part, pstride, with_sum, gate, blockIdx.x);
+        uint32_t pstride, int with_sum, const float* __restrict__ gate, uint32_t cols_per) {
+  pdl_wait();
+  pdl_trigger();
+  const uint32_t c_lo = min(ncols, blockIdx.y * cols_per), c_hi = min(ncols, c_lo + cols_per);
+  udots_body(U, ldu, ncols, y, part, pstride, with_sum && blockIdx.y == 0, gate, blockIdx.x,
+             c_lo, c_hi);
 }
 
 __global__ void __launch_bounds__(256, 8)
@@ -106,7 +113,23 @@ k_udots_multi(const __grid_constant__ TaskList<UdotsTask> L) {
   const uint32_t i = task_of(L.first, L.count, blockIdx.x);
   const UdotsTask& t = L.t[i];
   udots_body(t.U, t.ldu, t.ncols, t.y, t.part, t.pstride, t.with_sum, t.gate,
-             blockIdx.x - L.first[i]);
+             blockIdx.x - L.first[i], 0, t.ncols);
+}
+
+// What a finished norm leaves behind (one thread): s = |y_out|^2, sc = |y_in -
+// mean|^2.
+__device__ __forceinline__ void store_norm(double s, double sc, const NormFinish& fin) {
+  double a = sqrt(s);
+  if (a < 1e-8) a = 1e-8;  // clip_val, pca.pyx:1084-1085
+  fin.B[fin.j + (uint64_t)fin.j * fin.m] = a;
+  const float af = (float)a;
+  fin.scal[0] = af;
+  fin.scal[1] = 1.f / af;  // inverse_alpha, pca.pyx:1086
+  if (fin.gate) {
+    fin.gate[0] = (float)s;
+    fin.gate[1] = (float)sc;
+  }
+  *fin.counter = 0u;  // every block has taken its ticket
 }
 
 // alpha = max(sqrt(sum_b part[b * pstride]), 1e-8) in FP64 (clip_val,
@@ -136,17 +159,7 @@ __device__ void finish_norm_block(const float* part, uint64_t nblocks,
       s += dred[0][w];
       sc += dred[1][w];
     }
-    double a = sqrt(s);
-    if (a < 1e-8) a = 1e-8;  // clip_val, pca.pyx:1084-1085
-    fin.B[fin.j + (uint64_t)fin.j * fin.m] = a;
-    const float af = (float)a;
-    fin.scal[0] = af;
-    fin.scal[1] = 1.f / af;  // inverse_alpha, pca.pyx:1086
-    if (fin.gate) {
-      fin.gate[0] = (float)s;
-      fin.gate[1] = (float)sc;
-    }
-    *fin.counter = 0u;  // every block has taken its ticket
+    store_norm(s, sc, fin);
   }
 }
 
@@ -233,8 +246,139 @@ k_uupdate(const float* __restrict__ U, uint64_t ldu, uint32_t ncols,
           float* __restrict__ norm_part, uint32_t pstride, int with_centred,
           const float* __restrict__ gate, unsigned long long* __restrict__ taken,
           NormFinish fin) {
+  pdl_wait();
+  pdl_trigger();
   uupdate_body(U, ldu, ncols, coef, mean_sum, n, y_in, y_out, norm_part, pstride,
                with_centred, gate, taken, fin, blockIdx.x, gridDim.x);
+}
+
+// The updates of an adaptive step for few 1024-row blocks: the same rows, sums
+// and order,
+// spread over four 64-thread CTAs per block, with kSplitLoads columns in
+// flight per thread (a block's CTA alone keeps 4, and at 2.7k rows three CTAs
+// walked 100 columns in 61 us, this in 11, L2 cold). Up to kFoldBlocks blocks each CTA also
+// adds the blocks' dots itself, in k_reduce_cols' order (with at most 32
+// blocks a plain sum over the blocks), which saves that launch. First pass
+// (taken == nullptr): centred, with the gate's sums. Second pass: behind the
+// gate, no mean. wpart: per block its 8 warps' sums of squares, then of
+// centred squares; the last CTA adds them as finish_norm_block does.
+constexpr int kSplit = 4;
+constexpr int kSplitThreads = 256 / kSplit;
+constexpr int kSplitLoads = 16;
+constexpr uint32_t kFoldBlocks = 32;
+
+__global__ void __launch_bounds__(kSplitThreads)
+k_uupdate_split(const float* __restrict__ U, uint64_t ldu, uint32_t ncols,
+                const float* __restrict__ coef, const float* __restrict__ part,
+                uint32_t pstride, uint32_t nblocks, uint64_t n, float* y,
+                float* __restrict__ wpart, const float* __restrict__ gate,
+                unsigned long long* __restrict__ taken, NormFinish fin) {
+  extern __shared__ float cs[];  // ncols coefficients, then the sum of y
+  pdl_wait();
+  pdl_trigger();
+  if (second_pass_skipped(gate)) return;
+  const bool first = taken == nullptr;
+  if (taken && blockIdx.x == 0 && threadIdx.x == 0) {
+    taken[0] += 1ull;
+    taken[1] += ncols;
+  }
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (uint32_t c = threadIdx.x; c < ncols + (first ? 1u : 0u); c += kSplitThreads) {
+    float r;
+    if (part) {
+      r = 0.f;
+#pragma unroll 8
+      for (uint32_t b = 0; b < nblocks; ++b) r += part[(uint64_t)b * pstride + c];
+    } else {
+      r = coef[c];
+    }
+    cs[c] = r;
+  }
+  __syncthreads();
+  const uint64_t b = blockIdx.x / kSplit;
+  const uint32_t quarter = blockIdx.x % kSplit;
+  const uint64_t row0 = b * kRowBlock + (quarter * kSplitThreads + threadIdx.x) * 4ull;
+  float sq = 0.f, sqc = 0.f;
+  if (row0 < ldu) {
+    float4 yv = *reinterpret_cast<const float4*>(y + row0);
+    const float mean = first ? cs[ncols] / (float)n : 0.f;  // pca.pyx:1025-1028
+    const float cx = (row0 + 0 < n) ? yv.x - mean : 0.f;
+    const float cy = (row0 + 1 < n) ? yv.y - mean : 0.f;
+    const float cz = (row0 + 2 < n) ? yv.z - mean : 0.f;
+    const float cw = (row0 + 3 < n) ? yv.w - mean : 0.f;
+    sqc = sumsq4(cx, cy, cz, cw);
+    float4 t = make_float4(mean, mean, mean, mean);
+    for (uint32_t c0 = 0; c0 < ncols; c0 += kSplitLoads) {
+      float4 u[kSplitLoads];
+#pragma unroll
+      for (int k = 0; k < kSplitLoads; ++k)
+        if (c0 + k < ncols)
+          u[k] = *reinterpret_cast<const float4*>(U + (uint64_t)(c0 + k) * ldu + row0);
+#pragma unroll
+      for (int k = 0; k < kSplitLoads; ++k) {
+        if (c0 + k >= ncols) break;
+        const float w = cs[c0 + k];
+        t.x = __fmaf_rn(u[k].x, w, t.x);
+        t.y = __fmaf_rn(u[k].y, w, t.y);
+        t.z = __fmaf_rn(u[k].z, w, t.z);
+        t.w = __fmaf_rn(u[k].w, w, t.w);
+      }
+    }
+    yv.x = (row0 + 0 < n) ? yv.x - t.x : 0.f;
+    yv.y = (row0 + 1 < n) ? yv.y - t.y : 0.f;
+    yv.z = (row0 + 2 < n) ? yv.z - t.z : 0.f;
+    yv.w = (row0 + 3 < n) ? yv.w - t.w : 0.f;
+    *reinterpret_cast<float4*>(y + row0) = yv;
+    sq = sumsq4(yv.x, yv.y, yv.z, yv.w);
+  }
+  sq = warp_sum(sq);
+  sqc = warp_sum(sqc);
+  if (lane == 0) {
+    const uint32_t w = quarter * (kSplitThreads / 32) + wid;
+    wpart[b * 16 + w] = sq;
+    wpart[b * 16 + 8 + w] = sqc;
+  }
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(fin.counter, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  // the 256 threads of finish_norm_block, 64 at a time
+  __shared__ double dred[2][8];
+  for (int v = wid; v < 8; v += kSplitThreads / 32) {
+    double t = 0.0, tc = 0.0;
+    if ((uint32_t)v * 32 >= nblocks) {  // no block: zeros, without the FP64 shuffles
+      if (lane == 0) dred[0][v] = dred[1][v] = 0.0;
+      continue;
+    }
+    for (uint32_t blk = v * 32 + lane; blk < nblocks; blk += 256) {
+      float f = 0.f, fc = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        f += __ldcg(wpart + blk * 16 + w);
+        fc += __ldcg(wpart + blk * 16 + 8 + w);
+      }
+      t += (double)f;
+      tc += (double)fc;
+    }
+    t = warp_sum(t);
+    tc = warp_sum(tc);
+    if (lane == 0) {
+      dred[0][v] = t;
+      dred[1][v] = tc;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0, sc = 0.0;
+    for (int w = 0; w < 8; ++w) {
+      s += dred[0][w];
+      sc += dred[1][w];
+    }
+    store_norm(s, sc, fin);
+  }
 }
 
 __global__ void __launch_bounds__(256, 8)
@@ -341,6 +485,8 @@ __device__ __forceinline__ void reduce_cols_body(const float* __restrict__ part,
 __global__ void __launch_bounds__(1024)
 k_reduce_cols(const float* __restrict__ part, uint64_t nblocks, uint32_t pstride,
               uint32_t ncols, float* __restrict__ out, const float* __restrict__ gate) {
+  pdl_wait();
+  pdl_trigger();
   reduce_cols_body(part, nblocks, pstride, ncols, out, gate, blockIdx.x);
 }
 
@@ -406,11 +552,20 @@ k_vstep(const float* __restrict__ zin, float* __restrict__ V, uint64_t ldv,
 // Gram-Schmidt dots and the norm are all-reduced through distributed shared
 // memory, every CTA summing the 8 partials in rank order (so all CTAs hold
 // the same bits and the result does not depend on timing).
+// It is a chain of short phases (latency, not bytes), so what can leave the
+// chain does: kCached copies the CTA's part of V's columns into shared memory
+// before pdl_wait(), while the kernels before still run, and every phase reads
+// it there; sums in FP64 are made by the warps that have terms, and the
+// square root by one thread (GB300 issues an FP64 instruction of one warp in
+// the time of tens of FP32 ones: 32 warps each computing the same root took
+// longer than the products). 2000 genes x 100 columns: 21 -> 14 us.
 constexpr int kVCluster = 8;
 static_assert(kVCluster == (int)kVStepCtas, "one V-step task is one cluster");
 constexpr int kVThreads = 1024;
 constexpr int kVSplit = 4;  // threads sharing one gene's update sum
+constexpr int kVLoads = 8;  // columns' or genes' loads in flight per thread
 
+template <bool kCached>
 __device__ __forceinline__ void vstep_cluster_body(
     const float* __restrict__ zin, float* __restrict__ V, uint64_t ldv, uint32_t g,
     uint32_t j, uint32_t m, const float* __restrict__ scal, double* __restrict__ B,
@@ -426,17 +581,34 @@ __device__ __forceinline__ void vstep_cluster_body(
   float* pd = zs + ((slice + 3) & ~3u);       // 2 x (m + 1) partials (per pass)
   float* dots = pd + 2 * (m + 1);             // m + 1
   float* upd = dots + ((m + 4) & ~3u);        // kVSplit x slice partial updates
+  float* vs = upd + kVSplit * slice;          // kCached: (j + 1) x slice columns of V
   __shared__ double pn;                       // partial squared norm
   __shared__ double wred[kVThreads / 32];
   __shared__ float wz[kVThreads / 32];
   __shared__ float pz1;                       // partial |z after pass 0|^2
+  __shared__ float s_inv;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const uint32_t q = cluster.block_rank();
-  const uint32_t c0 = q * slice, c1 = min(g, c0 + slice);
+  const uint32_t c0 = min(g, q * slice), c1 = min(g, c0 + slice), cn = c1 - c0;
+  if constexpr (kCached) {
+    for (uint32_t col = wid; col <= j; col += kVThreads / 32)
+      for (uint32_t i = lane; i < cn; i += 32)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                         smem_u32(vs + (size_t)col * slice + i)),
+                     "l"(V + (uint64_t)col * ldv + c0 + i)
+                     : "memory");
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+  }
+  // element i of the CTA's part of V's column col
+  auto column = [&](uint32_t col, uint32_t i) {
+    return kCached ? vs[(size_t)col * slice + i] : V[(uint64_t)col * ldv + c0 + i];
+  };
+  pdl_wait();
+  pdl_trigger();
+  __syncthreads();
   const float alpha = scal[0];
-  const float* vj = V + (uint64_t)j * ldv;
-  for (uint32_t c = c0 + threadIdx.x; c < c1; c += kVThreads)
-    zs[c - c0] = __fmaf_rn(-alpha, vj[c], zin[c]);  // pca.pyx:1104-1105
+  for (uint32_t i = threadIdx.x; i < cn; i += kVThreads)
+    zs[i] = __fmaf_rn(-alpha, column(j, i), zin[c0 + i]);  // pca.pyx:1104-1105
   __syncthreads();
   for (int pass = 0; pass < npass; ++pass) {
     float* pdp = pd + (pass & 1) * (m + 1);
@@ -445,34 +617,49 @@ __device__ __forceinline__ void vstep_cluster_body(
     for (uint32_t col = wid; col < ncol; col += kVThreads / 32) {
       float d = 0.f;
       if (col <= j) {
-        const float* vc = V + (uint64_t)col * ldv;
-        for (uint32_t c = c0 + lane; c < c1; c += 32) d = __fmaf_rn(vc[c], zs[c - c0], d);
+        for (uint32_t i = lane; i < cn; i += 32 * kVLoads) {
+          float v[kVLoads];  // every load before the first use
+#pragma unroll
+          for (int k = 0; k < kVLoads; ++k) v[k] = i + 32 * k < cn ? column(col, i + 32 * k) : 0.f;
+#pragma unroll
+          for (int k = 0; k < kVLoads; ++k)
+            if (i + 32 * k < cn) d = __fmaf_rn(v[k], zs[i + 32 * k], d);
+        }
       } else {
-        for (uint32_t c = c0 + lane; c < c1; c += 32) d = __fmaf_rn(zs[c - c0], zs[c - c0], d);
+        for (uint32_t i = lane; i < cn; i += 32) d = __fmaf_rn(zs[i], zs[i], d);
       }
       d = warp_sum(d);
       if (lane == 0) pdp[col] = d;
     }
     cluster.sync();  // every CTA's partials are visible
     for (uint32_t col = threadIdx.x; col < ncol; col += kVThreads) {
-      float t = 0.f;
-      for (uint32_t r = 0; r < kVCluster; ++r) t += cluster.map_shared_rank(pdp, r)[col];
+      float p[kVCluster], t = 0.f;
+#pragma unroll
+      for (uint32_t r = 0; r < kVCluster; ++r) p[r] = cluster.map_shared_rank(pdp, r)[col];
+#pragma unroll
+      for (uint32_t r = 0; r < kVCluster; ++r) t += p[r];
       dots[col] = t;
     }
     __syncthreads();
     // each gene's sum over columns split in kVSplit fixed strands (col = h,
     // h + kVSplit, ...), added in strand order
     for (uint32_t t = threadIdx.x; t < kVSplit * slice; t += kVThreads) {
-      const uint32_t h = t / slice, c = c0 + t % slice;
+      const uint32_t h = t / slice, i = t % slice;
       float acc = 0.f;
-      if (c < c1)
-        for (uint32_t col = h; col <= j; col += kVSplit)
-          acc = __fmaf_rn(V[c + (uint64_t)col * ldv], dots[col], acc);
+      if (i < cn)
+        for (uint32_t col = h; col <= j; col += kVSplit * kVLoads) {
+          float v[kVLoads];
+#pragma unroll
+          for (int k = 0; k < kVLoads; ++k)
+            v[k] = col + kVSplit * k <= j ? column(col + kVSplit * k, i) : 0.f;
+#pragma unroll
+          for (int k = 0; k < kVLoads; ++k)
+            if (col + kVSplit * k <= j) acc = __fmaf_rn(v[k], dots[col + kVSplit * k], acc);
+        }
       upd[t] = acc;
     }
     __syncthreads();
-    for (uint32_t c = c0 + threadIdx.x; c < c1; c += kVThreads) {
-      const uint32_t i = c - c0;
+    for (uint32_t i = threadIdx.x; i < cn; i += kVThreads) {
       float t = 0.f;
 #pragma unroll
       for (int h = 0; h < kVSplit; ++h) t += upd[h * slice + i];
@@ -481,8 +668,7 @@ __device__ __forceinline__ void vstep_cluster_body(
     __syncthreads();
     if (adaptive && pass == 0) {
       float s1 = 0.f;
-      for (uint32_t c = c0 + threadIdx.x; c < c1; c += kVThreads)
-        s1 = __fmaf_rn(zs[c - c0], zs[c - c0], s1);
+      for (uint32_t i = threadIdx.x; i < cn; i += kVThreads) s1 = __fmaf_rn(zs[i], zs[i], s1);
       s1 = warp_sum(s1);
       if (lane == 0) wz[wid] = s1;
       __syncthreads();
@@ -492,50 +678,64 @@ __device__ __forceinline__ void vstep_cluster_body(
         pz1 = t;
       }
       cluster.sync();
-      float z1 = 0.f;
-      for (uint32_t r = 0; r < kVCluster; ++r) z1 += *cluster.map_shared_rank(&pz1, r);
+      float p[kVCluster], z1 = 0.f;
+#pragma unroll
+      for (uint32_t r = 0; r < kVCluster; ++r) p[r] = *cluster.map_shared_rank(&pz1, r);
+#pragma unroll
+      for (uint32_t r = 0; r < kVCluster; ++r) z1 += p[r];
       if (z1 >= 0.5f * dots[j + 1]) break;  // the same in every CTA
     }
   }
   float* out = (j + 1 < m) ? V + (uint64_t)(j + 1) * ldv : rem;
   if (j + 1 < m) {
     double ss = 0.0;
-    for (uint32_t c = c0 + threadIdx.x; c < c1; c += kVThreads)
-      ss = __fma_rn((double)zs[c - c0], (double)zs[c - c0], ss);
-    ss = warp_sum(ss);
+    if ((uint32_t)wid * 32 < cn) {  // warps without a gene hold zero
+      for (uint32_t i = threadIdx.x; i < cn; i += kVThreads)
+        ss = __fma_rn((double)zs[i], (double)zs[i], ss);
+      ss = warp_sum(ss);
+    }
     if (lane == 0) wred[wid] = ss;
     __syncthreads();
     if (threadIdx.x == 0) {
       double t = 0.0;
-      for (int w = 0; w < kVThreads / 32; ++w) t += wred[w];
+      const int warps = (int)min((cn + 31) / 32, (uint32_t)kVThreads / 32);
+      for (int w = 0; w < warps; ++w) t += wred[w];
       pn = t;
     }
     cluster.sync();
-    double s2 = 0.0;
-    for (uint32_t r = 0; r < kVCluster; ++r) s2 += *cluster.map_shared_rank(&pn, r);
-    double beta = sqrt(s2);
-    if (beta < 1e-8) beta = 1e-8;  // pca.pyx:1165-1166
-    if (q == 0 && threadIdx.x == 0) B[j + (uint64_t)(j + 1) * m] = beta;
-    const float inv = 1.f / (float)beta;
-    for (uint32_t c = c0 + threadIdx.x; c < c1; c += kVThreads) out[c] = zs[c - c0] * inv;
+    if (threadIdx.x == 0) {
+      double p[kVCluster], s2 = 0.0;
+#pragma unroll
+      for (uint32_t r = 0; r < kVCluster; ++r) p[r] = *cluster.map_shared_rank(&pn, r);
+#pragma unroll
+      for (uint32_t r = 0; r < kVCluster; ++r) s2 += p[r];
+      double beta = sqrt(s2);
+      if (beta < 1e-8) beta = 1e-8;  // pca.pyx:1165-1166
+      if (q == 0) B[j + (uint64_t)(j + 1) * m] = beta;
+      s_inv = 1.f / (float)beta;
+    }
+    __syncthreads();
+    const float inv = s_inv;
+    for (uint32_t i = threadIdx.x; i < cn; i += kVThreads) out[c0 + i] = zs[i] * inv;
   } else {
-    for (uint32_t c = c0 + threadIdx.x; c < c1; c += kVThreads) out[c] = zs[c - c0];
+    for (uint32_t i = threadIdx.x; i < cn; i += kVThreads) out[c0 + i] = zs[i];
   }
   cluster.sync();  // no CTA leaves while another may read its shared memory
 }
 
+template <bool kCached>
 __global__ void __cluster_dims__(kVCluster, 1, 1) __launch_bounds__(kVThreads)
 k_vstep_cluster(const float* __restrict__ zin, float* __restrict__ V, uint64_t ldv,
                 uint32_t g, uint32_t j, uint32_t m, const float* __restrict__ scal,
                 double* __restrict__ B, float* __restrict__ rem, int passes) {
-  vstep_cluster_body(zin, V, ldv, g, j, m, scal, B, rem, passes);
+  vstep_cluster_body<kCached>(zin, V, ldv, g, j, m, scal, B, rem, passes);
 }
 
 // one cluster per task: CTAs [8 i, 8 i + 8) of the grid
 __global__ void __cluster_dims__(kVCluster, 1, 1) __launch_bounds__(kVThreads)
 k_vstep_cluster_multi(const __grid_constant__ TaskList<VstepTask> L) {
   const VstepTask& t = L.t[blockIdx.x / kVCluster];
-  vstep_cluster_body(t.z, t.V, t.ldv, t.g, t.j, t.m, t.scal, t.B, t.rem, t.passes);
+  vstep_cluster_body<false>(t.z, t.V, t.ldv, t.g, t.j, t.m, t.scal, t.B, t.rem, t.passes);
 }
 
 // Tall-skinny SIMT GEMM: CTA tile 128 rows x 128 columns, K in steps of 16.
@@ -638,9 +838,17 @@ int launch_udots(const float* U, uint64_t ldu, uint32_t ncols, const float* y,
   const size_t smem = 8ull * (ncols + 1) * sizeof(float);
   BGPU_REQUIRE(smem <= 227 * 1024, BGPU_ERR_UNSUPPORTED, "U dots: too many columns");
   if (smem > 48 * 1024) BGPU_CUDA(allow_max_smem(k_udots));
-  k_udots<<<(unsigned)nblocks, 256, smem, s>>>(U, ldu, ncols, y, part, pstride,
-                                               with_sum ? 1 : 0, gate);
-  BGPU_CHECK_LAUNCH();
+  // four CTAs per SM from the blocks and parts of the columns, at least 8
+  // columns each
+  uint32_t ny = 1;
+  if (ncols > 8 && nblocks < (uint64_t)num_sms() * 4)
+    ny = (uint32_t)std::min<uint64_t>(ceil_div(ncols, 8),
+                                      (uint64_t)num_sms() * 4 / nblocks);
+  ny = std::max(ny, 1u);
+  const uint32_t per = std::max(1u, (uint32_t)ceil_div(ncols, ny));
+  const dim3 grid((unsigned)nblocks, std::max(1u, (uint32_t)ceil_div(ncols, per)));
+  BGPU_CUDA(launch_pdl(k_udots, grid, 256, smem, s, U, ldu, ncols, y, part, pstride,
+                       with_sum ? 1 : 0, gate, per));
   return BGPU_OK;
 }
 
@@ -652,10 +860,26 @@ int launch_uupdate(const float* U, uint64_t ldu, uint32_t ncols,
                    unsigned long long* taken, NormFinish fin) {
   BGPU_REQUIRE(!fin.B || (norm_part && fin.counter && fin.scal), BGPU_ERR_INVALID,
                "U update: norm finish needs partials, a ticket counter and scal");
-  k_uupdate<<<(unsigned)nblocks, 256, std::max<size_t>(ncols, 1) * 4, s>>>(
-      U, ldu, ncols, coef, mean_sum, n, y_in, y_out, norm_part, pstride,
-      with_centred ? 1 : 0, gate, taken, fin);
-  BGPU_CHECK_LAUNCH();
+  BGPU_CUDA(launch_pdl(k_uupdate, (unsigned)nblocks, 256, std::max<size_t>(ncols, 1) * 4, s, U,
+                       ldu, ncols, coef, mean_sum, n, y_in, y_out, norm_part, pstride,
+                       with_centred ? 1 : 0, gate, taken, fin));
+  return BGPU_OK;
+}
+
+bool uupdate_split_pays(uint64_t nblocks) { return nblocks <= (uint64_t)num_sms() * 2; }
+
+int launch_split_update(const float* U, uint64_t ldu, uint32_t ncols, float* part,
+                        uint32_t pstride, uint64_t nblocks, float* coef, uint64_t n, float* y,
+                        float* wpart, const float* gate, unsigned long long* taken,
+                        NormFinish fin, cudaStream_t s, uint32_t* launches) {
+  const bool fold = nblocks <= kFoldBlocks;
+  if (!fold)
+    BGPU_TRY(launch_reduce_cols(part, nblocks, pstride, ncols + (taken ? 0 : 1), coef, s, gate));
+  *launches += fold ? 1 : 2;
+  BGPU_CUDA(launch_pdl(k_uupdate_split, (unsigned)nblocks * kSplit, kSplitThreads,
+                       (ncols + 1) * 4, s, U, ldu, ncols, (const float*)coef,
+                       (const float*)(fold ? part : nullptr), pstride, (uint32_t)nblocks, n, y,
+                       wpart, gate, taken, fin));
   return BGPU_OK;
 }
 
@@ -683,10 +907,8 @@ int launch_reduce_cols(const float* part, uint64_t nblocks, uint32_t pstride,
                        uint32_t ncols, float* out, cudaStream_t s,
                        const float* gate) {
   if (ncols == 0) return BGPU_OK;
-  k_reduce_cols<<<(unsigned)ceil_div(ncols, 32), 1024, 0, s>>>(part, nblocks,
-                                                               pstride, ncols, out,
-                                                               gate);
-  BGPU_CHECK_LAUNCH();
+  BGPU_CUDA(launch_pdl(k_reduce_cols, (unsigned)ceil_div(ncols, 32), 1024, 0, s, part, nblocks,
+                       pstride, ncols, out, gate));
   return BGPU_OK;
 }
 
@@ -705,8 +927,16 @@ int launch_vstep(const float* z, float* V, uint64_t ldv, uint32_t g,
                  float* rem, int passes, cudaStream_t s) {
   const size_t csm = vstep_cluster_smem(g, m);
   if (csm <= 48 * 1024) {
-    k_vstep_cluster<<<kVCluster, kVThreads, csm, s>>>(z, V, ldv, g, j, m, scal, B,
-                                                     rem, passes);
+    const size_t cached = csm + (size_t)(j + 1) * ((g + kVCluster - 1) / kVCluster) * 4;
+    if (cached <= 200 * 1024) {
+      BGPU_CUDA(allow_max_smem(k_vstep_cluster<true>));
+      BGPU_CUDA(launch_pdl(k_vstep_cluster<true>, kVCluster, kVThreads, cached, s, z, V, ldv, g,
+                           j, m, scal, B, rem, passes));
+    } else {
+      BGPU_CUDA(launch_pdl(k_vstep_cluster<false>, kVCluster, kVThreads, csm, s, z, V, ldv, g, j,
+                           m, scal, B, rem, passes));
+    }
+    return BGPU_OK;
   } else {
     k_vstep<<<1, 1024, (size_t)m * sizeof(float), s>>>(  // adaptive: 2 passes
         z, V, ldv, g, j, m, scal, B, rem, passes == 0 ? 2 : passes);

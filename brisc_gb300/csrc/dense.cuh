@@ -46,6 +46,18 @@ int launch_uupdate(const float* U, uint64_t ldu, uint32_t ncols,
                    bool with_centred = false, const float* gate = nullptr,
                    unsigned long long* taken = nullptr, NormFinish fin = {});
 
+// An adaptive step's update in place, its column sums included: part holds the
+// blocks' dots (first pass: and the sum of y), coef receives their totals
+// where a launch of its own adds them. First pass (taken == nullptr): y <- y -
+// (mean + U . coef); second pass: behind gate, y <- y - U . coef, counted in
+// taken. wpart: nblocks x 16 floats. Bit-identical to launch_reduce_cols +
+// launch_uupdate; for up to two blocks per SM (uupdate_split_pays).
+bool uupdate_split_pays(uint64_t nblocks);
+int launch_split_update(const float* U, uint64_t ldu, uint32_t ncols, float* part,
+                        uint32_t pstride, uint64_t nblocks, float* coef, uint64_t n, float* y,
+                        float* wpart, const float* gate, unsigned long long* taken,
+                        NormFinish fin, cudaStream_t s, uint32_t* launches);
+
 // CGS2 middle pass in one read of U: y_out = y_in - (mean + U[:, :ncols] coef)
 // as launch_uupdate, and part[b * pstride + c] = U[rows of b, c] . y_out[rows
 // of b] over 256-row blocks b (uupdate_dots_blocks(n) of them).

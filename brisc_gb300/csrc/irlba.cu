@@ -195,7 +195,7 @@ struct Solver {
   Buf U, Unew, V, Vnew, y0, y1, part, coef, zpart, zvec, rem, sd, Bf, Ub, Sb,
       Vbt, oaw, svdwork, scal, smax, B, st, sdpart, svdinfo, ub_last,
       sb64, ratios, rotd, rotpiv, tailw, mergew,
-      derr, taken, ticket;
+      derr, taken, ticket, wpart;
   uint32_t svd_mode = 0;     // opts.svd_mode
   bool svd64 = false;        // full FP64 Jacobi (svd_mode 1)
   uint32_t merged_svds = 0;  // restarts solved by the secular merge
@@ -306,6 +306,7 @@ struct Solver {
     BGPU_TRY(balloc(svdinfo, 16, true, s));
     BGPU_TRY(balloc(taken, 16, true, s));
     BGPU_TRY(balloc(ticket, 16, true, s));
+    if (uupdate_split_pays(nb)) BGPU_TRY(balloc(wpart, nb * 64, false, s));
     return BGPU_OK;
   }
 
@@ -352,8 +353,12 @@ struct Solver {
       yfin = y1p;
     } else {
       BGPU_TRY(launch_udots(Up, ldu, j, y0p, nb, partp, ps, true, s));
-      BGPU_TRY(launch_reduce_cols(partp, nb, ps, j + 1, coefp, s));
-      launches += 2;
+      launches += 1;
+      const bool split = adaptive && uupdate_split_pays(nb);
+      if (!split) {
+        BGPU_TRY(launch_reduce_cols(partp, nb, ps, j + 1, coefp, s));
+        launches += 1;
+      }
       // algorithmic U-pass bytes (dots + update per pass): 2 n j 4 passes;
       // an adaptive solve adds its second passes from the device count at
       // the end
@@ -373,14 +378,24 @@ struct Solver {
         float* gate = coef2 + m;  // past the second pass's j <= m - 1 dots
         NormFinish fin1 = fin;
         fin1.gate = gate;
-        BGPU_TRY(launch_uupdate(Up, ldu, j, coefp, coefp + j, n, y0p, y0p, nb,
-                                partp, ps, s, true, nullptr, nullptr, fin1));
-        BGPU_TRY(launch_udots(Up, ldu, j, y0p, nb, partp, ps, false, s, gate));
-        BGPU_TRY(launch_reduce_cols(partp, nb, ps, j, coef2, s, gate));
-        BGPU_TRY(launch_uupdate(Up, ldu, j, coef2, nullptr, n, y0p, y0p, nb,
-                                partp, ps, s, false, gate,
-                                taken.as<unsigned long long>(), fin));
-        launches += 4;
+        unsigned long long* tk = taken.as<unsigned long long>();
+        if (split) {
+          uint32_t made = 1;  // the second pass's dots
+          BGPU_TRY(launch_split_update(Up, ldu, j, partp, ps, nb, coefp, n, y0p,
+                                       wpart.as<float>(), nullptr, nullptr, fin1, s, &made));
+          BGPU_TRY(launch_udots(Up, ldu, j, y0p, nb, partp, ps, false, s, gate));
+          BGPU_TRY(launch_split_update(Up, ldu, j, partp, ps, nb, coef2, n, y0p,
+                                       wpart.as<float>(), gate, tk, fin, s, &made));
+          launches += made;
+        } else {
+          BGPU_TRY(launch_uupdate(Up, ldu, j, coefp, coefp + j, n, y0p, y0p, nb,
+                                  partp, ps, s, true, nullptr, nullptr, fin1));
+          BGPU_TRY(launch_udots(Up, ldu, j, y0p, nb, partp, ps, false, s, gate));
+          BGPU_TRY(launch_reduce_cols(partp, nb, ps, j, coef2, s, gate));
+          BGPU_TRY(launch_uupdate(Up, ldu, j, coef2, nullptr, n, y0p, y0p, nb,
+                                  partp, ps, s, false, gate, tk, fin));
+          launches += 4;
+        }
         yfin = y0p;
       } else {
         if (uupdate_dots_smem(j) <= 227 * 1024) {

@@ -59,6 +59,7 @@ constexpr uint32_t kXtMaxEsc = 8192;        // escape slots: offsets < 65536
 constexpr uint32_t kXtMaxUnits = kXtMaxP / 4;
 constexpr uint32_t kTabStride = 17;         // per-lane X.v count table slot
 constexpr uint32_t kNoGene = 0xffffu;
+constexpr int kXvLoads = 8;
 
 enum SellErr : int { kSellErrLong = 1, kSellErrEsc = 2 };
 
@@ -66,6 +67,8 @@ enum SellErr : int { kSellErrLong = 1, kSellErrEsc = 2 };
 // X.v
 // cta, ctas: the CTA's index and the CTAs of the launch (the warps stride
 // the groups; each row's sum is one lane's whatever the grid)
+// T: threads of the CTA
+template <int T>
 __device__ __forceinline__ void xv_sell_body(const XvView& X, const float* __restrict__ v,
                                              const float* __restrict__ sd,
                                              float* __restrict__ y, uint32_t cta,
@@ -73,14 +76,26 @@ __device__ __forceinline__ void xv_sell_body(const XvView& X, const float* __res
   extern __shared__ __align__(16) float sm[];
   float* w = sm;                                   // v / sd, g floats
   float* tabs = sm + ((X.g + 3) & ~3u);            // [warp][lane][kTabStride]
-  for (uint32_t c = threadIdx.x; c < X.g; c += kSellThreads)
-    w[c] = sd ? v[c] / sd[c] : v[c];  // pca.pyx:461-462
+  pdl_wait();
+  pdl_trigger();
+  for (uint32_t c0 = threadIdx.x; c0 < X.g; c0 += T * kXvLoads) {
+    float a[kXvLoads], b[kXvLoads];  // every load before the first division
+#pragma unroll
+    for (int k = 0; k < kXvLoads; ++k) {
+      const uint32_t c = c0 + k * T;
+      a[k] = c < X.g ? v[c] : 0.f;
+      b[k] = sd && c < X.g ? sd[c] : 1.f;
+    }
+#pragma unroll
+    for (int k = 0; k < kXvLoads; ++k)
+      if (c0 + k * T < X.g) w[c0 + k * T] = sd ? a[k] / b[k] : a[k];  // pca.pyx:461-462
+  }
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   float* tb = tabs + (wid * 32 + lane) * kTabStride;
-  const uint32_t nwarps = ctas * kSellWarps;
+  const uint32_t nwarps = ctas * (T / 32);
   const uint2 z2 = make_uint2(0u, 0u);
-  for (uint32_t q = cta * kSellWarps + wid; q < X.groups; q += nwarps) {
+  for (uint32_t q = cta * (T / 32) + wid; q < X.groups; q += nwarps) {
     const uint64_t pos = (uint64_t)q * 32 + lane;
     const float f = X.isf[pos];  // 0 on the padding lanes of the last group
     tb[0] = 0.f;
@@ -126,14 +141,25 @@ __device__ __forceinline__ void xv_sell_body(const XvView& X, const float* __res
 __global__ void __launch_bounds__(kSellThreads, kXvCtasPerSm)
 k_xv_sell(XvView X, const float* __restrict__ v, const float* __restrict__ sd,
           float* __restrict__ y) {
-  xv_sell_body(X, v, sd, y, blockIdx.x, gridDim.x);
+  xv_sell_body<kSellThreads>(X, v, sd, y, blockIdx.x, gridDim.x);
+}
+
+// The same for few groups: CTAs of four warps, so that a few thousand rows
+// reach more than a dozen SMs (2.7k rows: 85 groups on 22 CTAs instead of 11;
+// 23 -> 21 us cold, 16 in the solve). A row's sum is its lane's, whatever the CTA.
+constexpr int kXvSmallThreads = 128;
+__global__ void __launch_bounds__(kXvSmallThreads)
+k_xv_sell_small(XvView X, const float* __restrict__ v, const float* __restrict__ sd,
+                float* __restrict__ y) {
+  xv_sell_body<kXvSmallThreads>(X, v, sd, y, blockIdx.x, gridDim.x);
 }
 
 __global__ void __launch_bounds__(kSellThreads, kXvCtasPerSm)
 k_xv_sell_multi(const __grid_constant__ TaskList<XvTask> L) {
   const uint32_t i = task_of(L.first, L.count, blockIdx.x);
   const XvTask& t = L.t[i];
-  xv_sell_body(t.X, t.v, t.sd, t.y, blockIdx.x - L.first[i], L.first[i + 1] - L.first[i]);
+  xv_sell_body<kSellThreads>(t.X, t.v, t.sd, t.y, blockIdx.x - L.first[i],
+                             L.first[i + 1] - L.first[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -183,6 +209,8 @@ __device__ __forceinline__ void xt_sell_body(const XtView& X, const float* __res
     if constexpr (kMom) gm[c] = make_double2(0.0, 0.0);
     else gs[c] = 0.f;
   }
+  pdl_wait();
+  pdl_trigger();
   const float scale = (!kMom && u_scale) ? *u_scale : 1.f;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const uint32_t P = X.P;
@@ -835,8 +863,8 @@ XtView xt_view(const Matrix& m) {
   return v;
 }
 
-static size_t xv_smem_bytes(uint32_t g) {
-  return (((size_t)g + 3) / 4 * 4 + (size_t)kSellThreads * kTabStride) * 4;
+static size_t xv_smem_bytes(uint32_t g, int threads = kSellThreads) {
+  return (((size_t)g + 3) / 4 * 4 + (size_t)threads * kTabStride) * 4;
 }
 
 uint32_t xv_sell_ctas(const Matrix& m) {
@@ -850,10 +878,15 @@ uint32_t xt_sell_ctas(const Matrix& m) { return m.xt.panels ? m.xt.ctas : 1u; }
 int launch_xv_sell(const Matrix& m, const float* v, const float* sd, float* y,
                    cudaStream_t s) {
   const XvView X = xv_view(m);
+  if (X.groups <= 4u * (uint32_t)num_sms()) {  // 8-warp CTAs would leave half the SMs idle
+    const unsigned ctas = (unsigned)ceil_div(X.groups, kXvSmallThreads / 32);
+    BGPU_CUDA(launch_pdl(k_xv_sell_small, ctas, kXvSmallThreads,
+                         xv_smem_bytes(m.g, kXvSmallThreads), s, X, v, sd, y));
+    return BGPU_OK;
+  }
   const size_t smem = xv_smem_bytes(m.g);
   if (smem > 48 * 1024) BGPU_CUDA(allow_max_smem(k_xv_sell));
-  k_xv_sell<<<xv_sell_ctas(m), kSellThreads, smem, s>>>(X, v, sd, y);
-  BGPU_CHECK_LAUNCH();
+  BGPU_CUDA(launch_pdl(k_xv_sell, xv_sell_ctas(m), kSellThreads, smem, s, X, v, sd, y));
   return BGPU_OK;
 }
 
@@ -886,9 +919,8 @@ int launch_xt_sell(const Matrix& m, const float* u, const float* u_scale, float*
   const XtView X = xt_view(m);
   const size_t smem = xt_smem_bytes(X.P, X.g, X.esc_max, false);
   BGPU_CUDA(allow_max_smem(k_xt_sell<false>));
-  k_xt_sell<false><<<X.panels ? m.xt.ctas : 1, kSellThreads, smem, s>>>(
-      X, u, u_scale, u_out, partT, nullptr);
-  BGPU_CHECK_LAUNCH();
+  BGPU_CUDA(launch_pdl(k_xt_sell<false>, X.panels ? m.xt.ctas : 1, kSellThreads, smem, s, X, u,
+                       u_scale, u_out, partT, (double2*)nullptr));
   return BGPU_OK;
 }
 

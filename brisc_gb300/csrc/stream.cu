@@ -648,6 +648,8 @@ __global__ void __launch_bounds__(256)
 k_reduce_panels_t(const float* __restrict__ partT, uint32_t num_panels,
                   uint32_t g, const float* __restrict__ sd,
                   float* __restrict__ z) {
+  pdl_wait();
+  pdl_trigger();
   reduce_panels_body(partT, num_panels, g, sd, z, blockIdx.x);
 }
 
@@ -779,8 +781,8 @@ uint32_t reduce_panels_ctas(const Matrix& m) { return (uint32_t)ceil_div(m.g, 8)
 
 int launch_reduce_panels_t(const Matrix& m, const float* partT, const float* sd,
                            float* z, cudaStream_t s) {
-  k_reduce_panels_t<<<reduce_panels_ctas(m), 256, 0, s>>>(partT, m.num_panels, m.g, sd, z);
-  BGPU_CHECK_LAUNCH();
+  BGPU_CUDA(launch_pdl(k_reduce_panels_t, reduce_panels_ctas(m), 256, 0, s, partT, m.num_panels,
+                       m.g, sd, z));
   return BGPU_OK;
 }
 

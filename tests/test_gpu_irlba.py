@@ -317,3 +317,28 @@ def test_adaptive_equals_single_pass_when_no_cancellation(cuda, golden, name):
     assert a.info["second_passes"] == 0
     assert np.array_equal(a.PCs, b.PCs)
     assert np.array_equal(a.singular_values, b.singular_values)
+
+
+@pytest.mark.parametrize("n", [40, 1024, 1025, 2700, 32768, 32769, 40000])
+def test_small_and_large_paths_of_the_u_pass_agree(cuda, n):
+    """The first update split over quarter blocks with its column sums folded
+    in, and the second pass as one cluster, against a batch of one solve,
+    which launches the whole-block kernels: the same bits, on matrices around
+    the row counts where the paths change, with steps that need their second
+    pass (a third of the cells repeat others)."""
+    import torch
+    from brisc_gb300.batch import SharedMatrix, pca_subsets
+    c = nb_counts(n, 300, seed=n, density=0.08, workers=1)
+    n = c.num_cells
+    rows = np.arange(n)
+    rows[: n // 3] = rows[n - n // 3:]
+    S = SharedMatrix(c.indptr, c.indices, c.data, n, 300, inv_size_factors=c.isf)
+    k, m = min(8, n), min(30, n)
+    fused = pca_subsets(S, [rows], num_PCs=k, subspace_size=m, max_iterations=6, mode="fused")[0]
+    M = S.subset(rows)
+    single = M.solve(k, m, max_iterations=6)
+    M.close()
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(single.PCs, fused.result.PCs)
+    np.testing.assert_array_equal(single.singular_values, fused.result.singular_values)
+    assert single.info["second_passes"] == fused.result.info["second_passes"]
