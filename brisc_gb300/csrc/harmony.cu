@@ -26,8 +26,9 @@
 // sum here runs in a fixed order, so runs are bit-identical.
 //
 // GPU shape. The block-sequential update is the critical path: one launch
-// of k_h_block per block (one CTA per chunk), each CTA
-//  - sorts its chunk's cells by batch (stable) in shared memory, so per-batch
+// of k_h_block per block (one CTA, or a cluster of CTAs with a part of the
+// cells each, per chunk), each CTA
+//  - sorts its cells by batch (stable) in shared memory, so per-batch
 //    sums over the chunk are runs of one batch: a register per cluster;
 //  - stages tiles of the cells' R rows and Z rows in shared memory; a thread
 //    per cluster sums the old R (old cluster/batch sums), then computes its
@@ -37,7 +38,7 @@
 //    and sums them per cluster and batch; with the objective wanted, also
 //    the cells' k-means error and entropy terms (those of the final R with
 //    the Y of the pass: the objective after the pass);
-//  - writes its chunk's changes of E and O; the last CTA of each group of 16
+//  - writes its chunk's changes of E and O; the last CTA of each group of 32
 //    chunks (an atomic ticket after a fence, no waiting) sums the group's in
 //    chunk order, and the last group adds the group sums to E and O in group
 //    order, so the next block's launch sees them.
@@ -50,9 +51,13 @@
 #include <type_traits>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "pcg.h"
 #include "tma.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace bgpu {
 namespace {
@@ -66,7 +71,8 @@ constexpr uint32_t kHMaxChunk = 1024;
 constexpr uint32_t kHCellsPerWarp = 4;       // cells a warp scores at once
 constexpr size_t kHSmemBudget = 110 * 1024;      // two block CTAs per SM
 constexpr size_t kHSmemBudgetOne = 220 * 1024;   // one block CTA per SM
-constexpr uint32_t kHFoldGroup = 16;  // chunks folded together before the final fold
+constexpr uint32_t kHFoldGroup = 32;  // chunks folded together before the final fold
+constexpr uint32_t kHMaxSplit = 8;    // CTAs (one cluster) that share a chunk
 
 struct BlockArgs {
   const float* Z;
@@ -75,6 +81,8 @@ struct BlockArgs {
   const uint32_t* order;   // cell order (nullptr: natural order)
   uint64_t start, len;     // positions [start, start + len) of the order
   uint32_t d, C, B, chunk, tile;
+  uint32_t split, sub;     // CTAs per chunk, cells of a chunk per CTA
+  uint32_t rvec, zvec;     // floats per asynchronous copy of R's and Z's rows
   float tos;               // 2 / sigma
   float ens;               // exp(-2 / sigma)
   const float* Pr;         // B
@@ -98,6 +106,30 @@ __device__ __forceinline__ void cp_async4(float* dst, const float* src, bool val
                "r"(valid ? 4 : 0)
                : "memory");
 }
+// One row of len floats by a warp, `vec` (1, 2 or 4) floats per copy: both
+// rows aligned to it and len a multiple of it.
+__device__ __forceinline__ void copy_row(float* dst, const float* src, uint32_t len, uint32_t vec,
+                                         int lane) {
+  if (vec == 4) {
+    for (uint32_t c = lane * 4; c < len; c += 128)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + c)),
+                   "l"(src + c)
+                   : "memory");
+  } else if (vec == 2) {
+    for (uint32_t c = lane * 2; c < len; c += 64)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst + c)),
+                   "l"(src + c)
+                   : "memory");
+  } else {
+    for (uint32_t c = lane; c < len; c += 32) cp_async4(dst + c, src + c, true);
+  }
+}
+// The widest such copy for rows of len floats at base.
+uint32_t row_vec(const float* base, uint32_t len) {
+  if (len % 4 == 0 && (uintptr_t)base % 16 == 0) return 4;
+  if (len % 2 == 0 && (uintptr_t)base % 8 == 0) return 2;
+  return 1;
+}
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
@@ -108,13 +140,14 @@ __device__ __forceinline__ void cp_async_wait() {
 
 // Shared-memory layout of k_h_block (offsets in bytes, each 16-aligned).
 struct BlockSmem {
-  size_t ys, zs, rs, ratio, bold, bnew, cid, cb, rid, rb, rk, seg, total;
+  size_t ys, zs, rs, ratio, bold, bnew, btot, cid, cb, rid, rb, rk, seg, total;
   uint32_t cp, yst, dp;  // padded cluster count (CPL x 32), Y's row stride
                          // (cp + 1: conflict-free transposed stores), Z's
 };
 
 __host__ __device__ inline BlockSmem block_smem(uint32_t d, uint32_t C, uint32_t B,
-                                                uint32_t chunk, uint32_t tile, int cpl) {
+                                                uint32_t chunk, uint32_t tile, int cpl,
+                                            bool split) {
   BlockSmem L;
   L.cp = (uint32_t)cpl * 32u;
   L.yst = L.cp + 1u;
@@ -136,6 +169,7 @@ __host__ __device__ inline BlockSmem block_smem(uint32_t d, uint32_t C, uint32_t
   L.ratio = take((size_t)B * C * 4);
   L.bold = take((size_t)B * C * 4);
   L.bnew = take((size_t)B * C * 4);
+  L.btot = split ? take((size_t)B * C * 4) : L.bold;  // the chunk's old sums
   L.cid = take((size_t)chunk * 4);
   L.cb = take((size_t)chunk * 4);
   L.seg = take((size_t)(B + 1) * 4);
@@ -192,17 +226,27 @@ __device__ __forceinline__ void sum_rows4(const float* a, const float* b, uint32
   *sb = (b0 + b1) + (b2 + b3);
 }
 
+// What one block launch has to wait for is short: the ratio needs E and O as
+// the block before left them; the cells' old sums, their products with Y and
+// the exponentials do not. So the kernel is launched as a programmatic
+// dependent and computes those before pdl_wait(). And a block has few chunks
+// (20 of 256 cells at 100k cells: 20 of 152 SMs), so a chunk is split over a
+// cluster of a.split CTAs, each with sub of its cells: their sums meet in
+// distributed shared memory, in rank order. 100k cells, 100 clusters, 50 PCs:
+// 77 us per block with a CTA per chunk, 35 us with eight (both alone, L2 cold;
+// about 25 us each in the pass, where they overlap).
 template <int CPL>
 __global__ void __launch_bounds__(kHThreads, 2) k_h_block(BlockArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const uint32_t d = a.d, C = a.C, B = a.B;
-  const BlockSmem L = block_smem(d, C, B, a.chunk, a.tile, CPL);
+  const BlockSmem L = block_smem(d, C, B, a.sub, a.tile, CPL, a.split > 1);
   float* ys = (float*)(smem + L.ys);
   float* zs = (float*)(smem + L.zs);
   float* rs = (float*)(smem + L.rs);
   float* ratio = (float*)(smem + L.ratio);
   float* bold = (float*)(smem + L.bold);
   float* bnew = (float*)(smem + L.bnew);
+  float* btot = (float*)(smem + L.btot);
   uint32_t* cid = (uint32_t*)(smem + L.cid);
   uint32_t* cb = (uint32_t*)(smem + L.cb);
   uint32_t* rid = (uint32_t*)(smem + L.rid);
@@ -214,8 +258,13 @@ __global__ void __launch_bounds__(kHThreads, 2) k_h_block(BlockArgs a) {
   __shared__ uint32_t running[kHMaxBatches];
   __shared__ int is_last;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const uint64_t p0 = a.start + (uint64_t)blockIdx.x * a.chunk;
-  const uint32_t ncell = (uint32_t)min_u64(a.chunk, a.start + a.len - p0);
+  cg::cluster_group cluster = cg::this_cluster();
+  const uint32_t split = a.split, rank = split > 1 ? cluster.block_rank() : 0u;
+  const uint32_t ci = blockIdx.x / split;  // the chunk
+  const uint64_t c_at = a.start + (uint64_t)ci * a.chunk;
+  const uint32_t c_len = (uint32_t)min_u64(a.chunk, a.start + a.len - c_at);
+  const uint64_t p0 = c_at + (uint64_t)rank * a.sub;
+  const uint32_t ncell = rank * a.sub < c_len ? min(a.sub, c_len - rank * a.sub) : 0u;
   const uint32_t cp = L.cp, yst = L.yst, dp = L.dp;
 
   // Y transposed ([dim][cluster], rows of yst) and zero-padded to cp
@@ -284,15 +333,13 @@ __global__ void __launch_bounds__(kHThreads, 2) k_h_block(BlockArgs a) {
   // per cell row, lanes along it
   auto stage_r = [&](uint32_t t0, uint32_t tn) {
     for (uint32_t i = wid; i < tn; i += kHWarps) {
-      const float* src = a.R + (uint64_t)cid[t0 + i] * C;
-      for (uint32_t c = lane; c < C; c += 32) cp_async4(rs + i * C + c, src + c, true);
+      copy_row(rs + i * C, a.R + (uint64_t)cid[t0 + i] * C, C, a.rvec, lane);
     }
   };
   auto stage_z = [&](uint32_t t0, uint32_t tn) {
     for (uint32_t i = wid; i < tn; i += kHWarps) {
-      const float* src = a.Z + (uint64_t)cid[t0 + i] * d;
-      for (uint32_t k = lane; k < dp; k += 32)
-        cp_async4(zs + i * dp + k, k < d ? src + k : src, k < d);
+      copy_row(zs + i * dp, a.Z + (uint64_t)cid[t0 + i] * d, d, a.zvec, lane);
+      if (d + lane < dp) zs[i * dp + d + lane] = 0.f;  // the padding, at most 3
     }
   };
   if (!a.init) stage_r(0, min(a.tile, ncell));
@@ -302,9 +349,9 @@ __global__ void __launch_bounds__(kHThreads, 2) k_h_block(BlockArgs a) {
   __syncthreads();
 
   const uint32_t j = tid;  // the thread's cluster in the per-cluster phases
-  float rold = 0.f;
+  const uint32_t BC = B * C;
   if (!a.init) {
-    // old contributions of the chunk's cells
+    // old contributions of the CTA's cells, then of the chunk's
     for (uint32_t t0 = 0; t0 < ncell; t0 += a.tile) {
       const uint32_t tn = min(a.tile, ncell - t0);
       if (t0 > 0) {
@@ -316,14 +363,64 @@ __global__ void __launch_bounds__(kHThreads, 2) k_h_block(BlockArgs a) {
       if (j < C) segment_sums(rs, seg, B, t0, tn, C, j, bold);
       __syncthreads();
     }
-    if (j < C) {
-      for (uint32_t b = 0; b < B; ++b) rold += bold[b * C + j];
-      // the block's ratio for this cluster (harmonize.pyx:585-598)
-      for (uint32_t b = 0; b < B; ++b) {
-        const float Eij = a.E[b * C + j] + -a.Pr[b] * rold;
-        const float Oij = a.O[b * C + j] - bold[b * C + j];
-        ratio[b * C + j] = a.ens * powf((Eij + 1.f) / (Oij + Eij + 1.f), a.theta[b]);
+    if (split > 1) cluster.sync();
+    for (uint32_t t = tid; t < BC; t += kHThreads) {
+      float v = bold[t];
+      if (split > 1) {
+        v = 0.f;
+        for (uint32_t r = 0; r < split; ++r) v += cluster.map_shared_rank(bold, r)[t];
       }
+      btot[t] = v;
+    }
+  }
+
+  // cells i0.. of tile rows against Y: dot[c][q] for cluster lane + 32 q
+  float dot[kHCellsPerWarp][CPL];
+  auto products = [&](uint32_t i0, uint32_t tn) {
+#pragma unroll
+    for (int c = 0; c < (int)kHCellsPerWarp; ++c)
+#pragma unroll
+      for (int q = 0; q < CPL; ++q) dot[c][q] = 0.f;
+    // rows past the tile re-read its last row: in bounds, results unused
+    const float* z0 = zs + (size_t)min(i0 + 0, tn - 1) * dp;
+    const float* z1 = zs + (size_t)min(i0 + 1, tn - 1) * dp;
+    const float* z2 = zs + (size_t)min(i0 + 2, tn - 1) * dp;
+    const float* z3 = zs + (size_t)min(i0 + 3, tn - 1) * dp;
+    for (uint32_t k = 0; k < dp; k += 4) {
+      const float4 v0 = *(const float4*)(z0 + k), v1 = *(const float4*)(z1 + k);
+      const float4 v2 = *(const float4*)(z2 + k), v3 = *(const float4*)(z3 + k);
+      const float za[4][4] = {{v0.x, v0.y, v0.z, v0.w}, {v1.x, v1.y, v1.z, v1.w},
+                              {v2.x, v2.y, v2.z, v2.w}, {v3.x, v3.y, v3.z, v3.w}};
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        if (k + kk >= d) break;
+        const float* yk = ys + (size_t)(k + kk) * yst + lane;
+#pragma unroll
+        for (int q = 0; q < CPL; ++q) {
+          const float y = yk[32 * q];
+#pragma unroll
+          for (int c = 0; c < (int)kHCellsPerWarp; ++c)
+            dot[c][q] = fmaf(za[c][kk], y, dot[c][q]);
+        }
+      }
+    }
+  };
+  // one tile with at most a group of cells per warp: its products come first
+  const bool ahead = ncell <= a.tile && ncell <= kHCellsPerWarp * kHWarps;
+  if (ahead && wid * kHCellsPerWarp < ncell) products(wid * kHCellsPerWarp, ncell);
+
+  pdl_wait();
+  pdl_trigger();
+  __syncthreads();  // btot is complete
+  if (!a.init) {
+    // the block's ratio for every batch and cluster (harmonize.pyx:585-598)
+    for (uint32_t t = tid; t < BC; t += kHThreads) {
+      const uint32_t b = t / C, jj = t % C;
+      float rold = 0.f;
+      for (uint32_t bb = 0; bb < B; ++bb) rold += btot[bb * C + jj];
+      const float Eij = __ldcg(a.E + t) + -a.Pr[b] * rold;
+      const float Oij = __ldcg(a.O + t) - btot[t];
+      ratio[t] = a.ens * powf((Eij + 1.f) / (Oij + Eij + 1.f), a.theta[b]);
     }
     __syncthreads();
   }
@@ -341,34 +438,7 @@ __global__ void __launch_bounds__(kHThreads, 2) k_h_block(BlockArgs a) {
     const uint32_t groups = (tn + kHCellsPerWarp - 1) / kHCellsPerWarp;
     for (uint32_t g = wid; g < groups; g += kHWarps) {
       const uint32_t i0 = g * kHCellsPerWarp;
-      float dot[kHCellsPerWarp][CPL];
-#pragma unroll
-      for (int c = 0; c < (int)kHCellsPerWarp; ++c)
-#pragma unroll
-        for (int q = 0; q < CPL; ++q) dot[c][q] = 0.f;
-      // rows past the tile re-read its last row: in bounds, results unused
-      const float* z0 = zs + (size_t)min(i0 + 0, tn - 1) * dp;
-      const float* z1 = zs + (size_t)min(i0 + 1, tn - 1) * dp;
-      const float* z2 = zs + (size_t)min(i0 + 2, tn - 1) * dp;
-      const float* z3 = zs + (size_t)min(i0 + 3, tn - 1) * dp;
-      for (uint32_t k = 0; k < dp; k += 4) {
-        const float4 v0 = *(const float4*)(z0 + k), v1 = *(const float4*)(z1 + k);
-        const float4 v2 = *(const float4*)(z2 + k), v3 = *(const float4*)(z3 + k);
-        const float za[4][4] = {{v0.x, v0.y, v0.z, v0.w}, {v1.x, v1.y, v1.z, v1.w},
-                                {v2.x, v2.y, v2.z, v2.w}, {v3.x, v3.y, v3.z, v3.w}};
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          if (k + kk >= d) break;
-          const float* yk = ys + (size_t)(k + kk) * yst + lane;
-#pragma unroll
-          for (int q = 0; q < CPL; ++q) {
-            const float y = yk[32 * q];
-#pragma unroll
-            for (int c = 0; c < (int)kHCellsPerWarp; ++c)
-              dot[c][q] = fmaf(za[c][kk], y, dot[c][q]);
-          }
-        }
-      }
+      if (!ahead) products(i0, tn);
 #pragma unroll
       for (int c = 0; c < (int)kHCellsPerWarp; ++c) {
         const uint32_t i = i0 + c;
@@ -405,15 +475,32 @@ __global__ void __launch_bounds__(kHThreads, 2) k_h_block(BlockArgs a) {
     if (j < C) segment_sums(rs, seg, B, t0, tn, C, j, bnew);
     __syncthreads();
   }
-  if (j < C) {
-    float rnew = 0.f;
-    for (uint32_t b = 0; b < B; ++b) rnew += bnew[b * C + j];
-    for (uint32_t b = 0; b < B; ++b) {
-      const uint64_t o = ((uint64_t)blockIdx.x * B + b) * C + j;
-      a.dE[o] = -a.Pr[b] * rold + a.Pr[b] * rnew;
-      a.dO[o] = -bold[b * C + j] + bnew[b * C + j];
+  // the chunk's changes of E and O, by its first CTA
+  if (split > 1) cluster.sync();
+  if (rank == 0) {
+    if (split > 1) {
+      for (uint32_t t = tid; t < BC; t += kHThreads) {
+        float v = 0.f;
+        for (uint32_t r = 0; r < split; ++r) v += cluster.map_shared_rank(bnew, r)[t];
+        ratio[t] = v;  // the ratios are used up
+      }
+      __syncthreads();
+    }
+    const float* total = split > 1 ? ratio : bnew;
+    if (j < C) {
+      float rold = 0.f, rnew = 0.f;
+      for (uint32_t b = 0; b < B; ++b) {
+        if (!a.init) rold += btot[b * C + j];
+        rnew += total[b * C + j];
+      }
+      for (uint32_t b = 0; b < B; ++b) {
+        const uint64_t o = ((uint64_t)ci * B + b) * C + j;
+        a.dE[o] = -a.Pr[b] * rold + a.Pr[b] * rnew;
+        a.dO[o] = a.init ? total[b * C + j] : -btot[b * C + j] + total[b * C + j];
+      }
     }
   }
+  if (split > 1) cluster.sync();  // the partial sums have been read
   if (a.obj) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -435,14 +522,15 @@ __global__ void __launch_bounds__(kHThreads, 2) k_h_block(BlockArgs a) {
       a.obj[2 * blockIdx.x + 1] = y;
     }
   }
+  if (rank != 0) return;
   // Fold every chunk's changes into E and O in two levels, with atomic
   // tickets after fences (no waiting): the last CTA of each group of
   // kHFoldGroup consecutive chunks sums the group's changes in chunk order;
   // the last group to finish adds the group sums to E and O in group order.
   __threadfence();
   __syncthreads();
-  const uint32_t BC = B * C, nch = gridDim.x;
-  const uint32_t gi = blockIdx.x / kHFoldGroup, ngroups = (nch + kHFoldGroup - 1) / kHFoldGroup;
+  const uint32_t nch = gridDim.x / split;
+  const uint32_t gi = ci / kHFoldGroup, ngroups = (nch + kHFoldGroup - 1) / kHFoldGroup;
   const uint32_t c0 = gi * kHFoldGroup, gsz = min(kHFoldGroup, nch - c0);
   if (tid == 0) is_last = atomicAdd(a.ticket + 1 + gi, 1u) == gsz - 1;
   __syncthreads();
@@ -552,38 +640,38 @@ k_h_rtm(const float* __restrict__ R, const float* __restrict__ M,
   }
 }
 
-// out[j][k] = sum over ranges c in [c0, c1) of part[c][j][k] (four
-// interleaved partial sums, combined in a fixed order); with normalise, each
-// row scaled by 1 / sqrt(sum of squares). One CTA per row, a thread per
-// dimension (d <= 128).
-__global__ void k_h_rtm_reduce(const float* __restrict__ part, uint32_t c0, uint32_t c1,
-                               uint32_t d, uint32_t C, int normalise, float* __restrict__ out) {
+// out[y][j][k] = sum over ranges c in [bound[y], bound[y + 1]) of part[c][j][k]
+// (kReduceRows interleaved partial sums, combined in a fixed order); with
+// normalise, each row scaled by 1 / sqrt(sum of squares). One CTA per row and
+// y, a thread per dimension (d <= 128) and partial sum.
+constexpr int kReduceRows = 4;
+__global__ void __launch_bounds__(128 * kReduceRows)
+k_h_rtm_reduce(const float* __restrict__ part, const uint32_t* __restrict__ bound, uint32_t d,
+               uint32_t C, int normalise, float* __restrict__ out) {
+  __shared__ float sums[kReduceRows][128];
   __shared__ float red[4];
   __shared__ float scale;
   const uint32_t j = blockIdx.x, k = threadIdx.x;
-  float v = 0.f;
+  const uint32_t c1 = bound[blockIdx.y + 1];
+  float t = 0.f;
   if (k < d) {
-    float p[4] = {0.f, 0.f, 0.f, 0.f};
-    uint32_t c = c0;
-    for (; c + 4 <= c1; c += 4)
-#pragma unroll
-      for (int u = 0; u < 4; ++u) p[u] += part[((uint64_t)(c + u) * C + j) * d + k];
-    for (int u = 0; c < c1; ++c, ++u) p[u] += part[((uint64_t)c * C + j) * d + k];
-    v = (p[0] + p[1]) + (p[2] + p[3]);
+#pragma unroll 8
+    for (uint32_t c = bound[blockIdx.y] + threadIdx.y; c < c1; c += kReduceRows)
+      t += part[((uint64_t)c * C + j) * d + k];
   }
+  sums[threadIdx.y][k] = t;
+  __syncthreads();
+  if (threadIdx.y != 0) return;
+  float v = (sums[0][k] + sums[1][k]) + (sums[2][k] + sums[3][k]);
   if (normalise) {
     const float sq = warp_sum(k < d ? v * v : 0.f);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sq;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      float t = 0.f;
-      for (uint32_t w = 0; w < (blockDim.x >> 5); ++w) t += red[w];
-      scale = 1.f / sqrtf(t);
-    }
-    __syncthreads();
+    if ((k & 31) == 0) red[k >> 5] = sq;
+    asm volatile("bar.sync 1, 128;" ::: "memory");  // the threads that are left
+    if (k == 0) scale = 1.f / sqrtf((red[0] + red[1]) + (red[2] + red[3]));
+    asm volatile("bar.sync 1, 128;" ::: "memory");
     v *= scale;
   }
-  if (k < d) out[(uint64_t)j * d + k] = v;
+  if (k < d) out[((uint64_t)blockIdx.y * C + j) * d + k] = v;
 }
 
 // Z = PCs - sum_k R[cell][k] W[k][batch][:] (harmonize.pyx:814-818), then,
@@ -687,11 +775,11 @@ k_h_normalize_rows(const float* __restrict__ in, float* __restrict__ out, uint64
 // Tile (cells staged at once) of the block kernel: the chunk split into the
 // fewest equal tiles (a multiple of 4 cells) whose layout fits the budget; 0
 // when even 4 cells do not fit.
-uint32_t block_tile(uint32_t d, uint32_t C, uint32_t B, uint32_t chunk, int cpl,
+uint32_t block_tile(uint32_t d, uint32_t C, uint32_t B, uint32_t chunk, int cpl, bool split,
                     size_t budget) {
   for (uint32_t nt = 1; nt <= chunk; ++nt) {
     const uint32_t tile = (uint32_t)round_up(ceil_div(chunk, nt), 4);
-    if (block_smem(d, C, B, chunk, tile, cpl).total <= budget) return tile;
+    if (block_smem(d, C, B, chunk, tile, cpl, split).total <= budget) return tile;
     if (tile == 4) break;
   }
   return 0;
@@ -699,10 +787,11 @@ uint32_t block_tile(uint32_t d, uint32_t C, uint32_t B, uint32_t chunk, int cpl,
 
 // Two CTAs per SM when a tile of at least 32 cells (or the whole chunk) fits
 // in half the shared memory, else one CTA per SM with the larger tile.
-uint32_t choose_tile(uint32_t d, uint32_t C, uint32_t B, uint32_t chunk, int cpl) {
-  const uint32_t two = block_tile(d, C, B, chunk, cpl, kHSmemBudget);
+uint32_t choose_tile(uint32_t d, uint32_t C, uint32_t B, uint32_t chunk, int cpl,
+                     bool split = false) {
+  const uint32_t two = block_tile(d, C, B, chunk, cpl, split, kHSmemBudget);
   if (two >= std::min<uint32_t>(chunk, 32)) return two;
-  return std::max(two, block_tile(d, C, B, chunk, cpl, kHSmemBudgetOne));
+  return std::max(two, block_tile(d, C, B, chunk, cpl, split, kHSmemBudgetOne));
 }
 
 int ranges_rtm(const float* R, const float* M, const uint32_t* cells, const uint64_t* starts,
@@ -714,12 +803,41 @@ int ranges_rtm(const float* R, const float* M, const uint32_t* cells, const uint
   return BGPU_OK;
 }
 
+// One block: a cluster of ba.split CTAs per chunk; `dependent`: may start
+// while the launch before runs (programmatic dependent launch).
+template <int CPL>
+int launch_block(const BlockArgs& ba, unsigned ctas, size_t smem, bool dependent,
+                 cudaStream_t s) {
+  cudaLaunchAttribute at[2];
+  unsigned n = 0;
+  if (ba.split > 1) {
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = ba.split;
+    at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (dependent) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = ctas;
+  cfg.blockDim = kHThreads;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = n;
+  BGPU_CUDA(cudaLaunchKernelEx(&cfg, k_h_block<CPL>, ba));
+  return BGPU_OK;
+}
+
 template <int CPL>
 int harmony_run(const float* PCs, float* Z, float* Y, float* R, const uint32_t* batch,
                 uint64_t n, uint32_t d, uint32_t C, uint32_t B, uint32_t max_iter,
                 uint32_t max_ci, float block_prop, float tol, int early, float ctol,
                 float theta, float tau, float alpha, float sigma, uint32_t chunk, uint64_t seed,
-                uint32_t tile, uint32_t* iters, cudaStream_t s) {
+                uint32_t* iters, cudaStream_t s) {
   const uint32_t BC = B * C;
   const uint32_t nchunks = (uint32_t)ceil_div(n, chunk);
   // the reference multiplies an unsigned long long by a float: float product
@@ -727,7 +845,19 @@ int harmony_run(const float* PCs, float* Z, float* Y, float* R, const uint32_t* 
   const uint32_t max_cpb = (uint32_t)ceil_div(block, chunk);
   const uint32_t nblocks = (uint32_t)ceil_div(n, block);
   const float tos = 2.f / sigma;
-  const size_t smem_blk = block_smem(d, C, B, chunk, tile, CPL).total;
+  // CTAs per chunk: as many (up to 8) as still give at most two per SM, and
+  // at least 32 cells each; the launch over all chunks (initialisation) has
+  // enough of them
+  uint32_t split = 1;
+  while (split < kHMaxSplit && max_cpb * split * 2 <= 2u * (uint32_t)num_sms() &&
+         chunk >= split * 2 * 32)
+    split *= 2;
+  if (split > 1 && !choose_tile(d, C, B, (uint32_t)ceil_div(chunk, split), CPL, true)) split = 1;
+  const uint32_t sub = (uint32_t)ceil_div(chunk, split);
+  const uint32_t tile = choose_tile(d, C, B, chunk, CPL);
+  const uint32_t sub_tile = choose_tile(d, C, B, sub, CPL, split > 1);
+  const size_t smem_all = block_smem(d, C, B, chunk, tile, CPL, false).total;
+  const size_t smem_blk = block_smem(d, C, B, sub, sub_tile, CPL, split > 1).total;
   // host-side batch bookkeeping, the random cell order, batch-sorted order
   std::vector<uint32_t> hb(n);
   BGPU_CUDA(cudaMemcpyAsync(hb.data(), batch, n * 4, cudaMemcpyDeviceToHost, s));
@@ -768,7 +898,9 @@ int harmony_run(const float* PCs, float* Z, float* Y, float* R, const uint32_t* 
     std::vector<uint64_t> pos(bstart.begin(), bstart.end() - 1);
     for (uint64_t i = 0; i < n; ++i) border[pos[hb[i]]++] = (uint32_t)i;
   }
-  const uint64_t rchunk = 2048;
+  // cells per range of the R^T reductions: two ranges per SM, 256 to 2048 cells
+  const uint64_t rchunk = std::min<uint64_t>(
+      2048, std::max<uint64_t>(256, round_up(ceil_div(n, 2ull * num_sms()), 32)));
   std::vector<uint32_t> brange0(B + 1, 0);
   for (uint32_t b = 0; b < B; ++b) {
     brange0[b] = (uint32_t)starts_b.size();
@@ -790,11 +922,16 @@ int harmony_run(const float* PCs, float* Z, float* Y, float* R, const uint32_t* 
   const uint32_t nr_nat = (uint32_t)starts_nat.size() - 1;
   const uint32_t nr_b = (uint32_t)starts_b.size() - 1;
   const uint32_t npart = std::max(nr_nat, nr_b);
-  const uint32_t nobj = std::max(nchunks, nblocks * max_cpb);
+  const uint32_t nobj = std::max(nchunks, nblocks * max_cpb * split);
   const uint32_t max_launch_chunks = std::max(nchunks, max_cpb);
   const uint32_t max_groups = (uint32_t)ceil_div(max_launch_chunks, kHFoldGroup);
 
-  float *E, *O, *Pr_d, *th_d, *dE, *dO, *gE, *gO, *part, *W;
+  // range bounds of the three reductions: one range (Y alone), all ranges, the
+  // batches' ranges
+  std::vector<uint32_t> bounds = {0, 1, 0, nr_nat};
+  bounds.insert(bounds.end(), brange0.begin(), brange0.end());
+  float *E, *O, *Pr_d, *th_d, *dE, *dO, *gE, *gO, *part, *W, *bsum;
+  uint32_t* bounds_d;
   double* obj;
   uint32_t *order_d, *border_d, *ticket;
   uint64_t *starts_nat_d, *starts_b_d, *cor_tiles_d;
@@ -818,6 +955,10 @@ int harmony_run(const float* PCs, float* Z, float* Y, float* R, const uint32_t* 
     BGPU_TRY(dalloc(&gO, (uint64_t)max_groups * BC * 4));
     BGPU_TRY(dalloc(&part, (uint64_t)npart * C * d * 4));
     BGPU_TRY(dalloc(&W, (uint64_t)C * (B + 1) * d * 4));
+    BGPU_TRY(dalloc(&bsum, (uint64_t)C * B * d * 4));
+    BGPU_TRY(dalloc(&bounds_d, bounds.size() * 4));
+    BGPU_CUDA(cudaMemcpyAsync(bounds_d, bounds.data(), bounds.size() * 4,
+                              cudaMemcpyHostToDevice, s));
     BGPU_TRY(dalloc(&obj, (uint64_t)nobj * 16));
     BGPU_TRY(dalloc(&order_d, n * 4));
     BGPU_TRY(dalloc(&border_d, n * 4));
@@ -877,6 +1018,10 @@ int harmony_run(const float* PCs, float* Z, float* Y, float* R, const uint32_t* 
     ba.B = B;
     ba.chunk = chunk;
     ba.tile = tile;
+    ba.split = 1;
+    ba.sub = chunk;
+    ba.rvec = row_vec(R, C);
+    ba.zvec = row_vec(Z, d);
     ba.tos = tos;
     ba.ens = std::exp(-tos);
     ba.Pr = Pr_d;
@@ -895,33 +1040,37 @@ int harmony_run(const float* PCs, float* Z, float* Y, float* R, const uint32_t* 
     ba.len = n;
     ba.obj = obj;
     ba.init = 1;
-    k_h_block<CPL><<<nchunks, kHThreads, smem_blk, s>>>(ba);
+    k_h_block<CPL><<<nchunks, kHThreads, smem_all, s>>>(ba);
     BGPU_CHECK_LAUNCH();
     float prev;
     BGPU_TRY(objective(&prev));
     // normalise Y's rows (harmonize.pyx:501)
     BGPU_CUDA(cudaMemcpyAsync(part, Y, (uint64_t)C * d * 4, cudaMemcpyDeviceToDevice, s));
-    k_h_rtm_reduce<<<C, 128, 0, s>>>(part, 0, 1, d, C, 1, Y);
+    k_h_rtm_reduce<<<C, dim3(128, kReduceRows), 0, s>>>(part, bounds_d, d, C, 1, Y);
     BGPU_CHECK_LAUNCH();
     float objective_v = prev;
     ba.order = order_d;
     ba.init = 0;
+    ba.split = split;
+    ba.sub = sub;
+    ba.tile = sub_tile;
     uint32_t it = 0;
     for (it = 1; it <= max_iter; ++it) {
       float past[3] = {0.f, 0.f, 0.f};
       for (uint32_t ci = 1; ci <= max_ci; ++ci) {
         // Y = normalise(R^T Z)
         BGPU_TRY(ranges_rtm(R, Z, nullptr, starts_nat_d, nr_nat, d, C, part, s));
-        k_h_rtm_reduce<<<C, 128, 0, s>>>(part, 0, nr_nat, d, C, 1, Y);
+        k_h_rtm_reduce<<<C, dim3(128, kReduceRows), 0, s>>>(part, bounds_d + 2, d, C, 1, Y);
         BGPU_CHECK_LAUNCH();
         const bool want = early || ci == max_ci;
         if (want) BGPU_CUDA(cudaMemsetAsync(obj, 0, (uint64_t)nobj * 16, s));
         for (uint32_t bi = 0; bi < nblocks; ++bi) {
           ba.start = (uint64_t)bi * block;
           ba.len = std::min<uint64_t>(block, n - ba.start);
-          ba.obj = want ? obj + 2ull * bi * max_cpb : nullptr;
-          k_h_block<CPL><<<(unsigned)ceil_div(ba.len, chunk), kHThreads, smem_blk, s>>>(ba);
-          BGPU_CHECK_LAUNCH();
+          ba.obj = want ? obj + 2ull * bi * max_cpb * split : nullptr;
+          // the first block of a pass waits for Y in the ordinary way
+          BGPU_TRY(launch_block<CPL>(ba, (unsigned)ceil_div(ba.len, chunk) * split, smem_blk,
+                                     bi > 0, s));
         }
         if (want) {
           BGPU_TRY(objective(&objective_v));
@@ -941,8 +1090,11 @@ int harmony_run(const float* PCs, float* Z, float* Y, float* R, const uint32_t* 
       }
       // correction: R-weighted per-batch PC sums per cluster
       BGPU_TRY(ranges_rtm(R, PCs, border_d, starts_b_d, nr_b, d, C, part, s));
-      hpart.resize((uint64_t)nr_b * C * d);
-      BGPU_CUDA(cudaMemcpyAsync(hpart.data(), part, hpart.size() * 4, cudaMemcpyDeviceToHost,
+      k_h_rtm_reduce<<<dim3(C, B), dim3(128, kReduceRows), 0, s>>>(part, bounds_d + 4, d, C, 0,
+                                                                  bsum);
+      BGPU_CHECK_LAUNCH();
+      hpart.resize((uint64_t)B * C * d);
+      BGPU_CUDA(cudaMemcpyAsync(hpart.data(), bsum, hpart.size() * 4, cudaMemcpyDeviceToHost,
                                 s));
       BGPU_CUDA(cudaStreamSynchronize(s));
       std::vector<float> Wh((uint64_t)C * (B + 1) * d, 0.f);
@@ -978,8 +1130,7 @@ int harmony_run(const float* PCs, float* Z, float* Y, float* R, const uint32_t* 
           for (uint32_t b = 0; b < B; ++b) {
             float bt = 0.f;
             if (!(hO[b * C + k] < 1e-5f * (float)Nb[b]))
-              for (uint32_t c = brange0[b]; c < brange0[b + 1]; ++c)
-                bt += hpart[((uint64_t)c * C + k) * d + jd];
+              bt = hpart[((uint64_t)b * C + k) * d + jd];
             rs[jd * (B + 1) + b] = bt;
             total += bt;
           }
@@ -1054,7 +1205,7 @@ extern "C" int bgpu_harmony(const float* PCs, float* Z, float* Y, float* R,
     return harmony_run<CPL>(PCs, Z, Y, R, batch_labels, n, d, C, B, max_iterations,
                             max_clustering_iterations, block_proportion, tolerance,
                             early_stopping, clustering_tolerance, theta, tau, alpha, sigma,
-                            chunk_size, seed, tile, iterations, s);
+                            chunk_size, seed, iterations, s);
   };
   if (C <= 32) return go(std::integral_constant<int, 1>{});
   if (C <= 64) return go(std::integral_constant<int, 2>{});

@@ -142,3 +142,25 @@ def test_harmony_shapes_match_oracle(cuda, n, d, C, B, chunk):
              ref_Z=Zo, ref_R_head=Ro[:500])
     Z, Y, R, it = _harmony(c)
     check_against(c, Z, R[:500], **TOL)
+
+
+@pytest.mark.parametrize("n,d,C,B,chunk,block", [
+    (3000, 13, 37, 3, 256, 0.05), (2500, 50, 100, 4, 100, 0.3), (1200, 30, 33, 1, 64, 1.0),
+    (4000, 7, 200, 6, 1000, 0.5), (900, 64, 20, 2, 31, 0.07)])
+def test_harmony_chunks_split_over_clusters(cuda, n, d, C, B, chunk, block):
+    """Chunks shared by one to eight CTAs, with a last chunk that leaves some
+    of them without a cell, one block per pass, row lengths of every
+    alignment, and more clusters than a warp's lanes: the oracle's embedding
+    and assignments."""
+    from synth import batched_pcs
+    from oracle import harmony as oh
+    X, b = batched_pcs(n, d, 12, B, seed=n)
+    rng = np.random.default_rng(1)
+    Z0 = oh.normalize_rows(X)
+    Y0 = np.ascontiguousarray(Z0[rng.choice(n, C, replace=False)])
+    kw = dict(seed=2, chunk_size=chunk, block_proportion=block, max_iterations=3)
+    Zo, Ro = oh.harmony(X, Z0.copy(), Y0, b, B, **kw)
+    c = dict(PCs=X, batch_labels=b, num_batches=B, harmony_kwargs=kw, Y_init=Y0, ref_Z=Zo,
+             ref_R_head=Ro)
+    Z, Y, R, it = _harmony(c)
+    check_against(c, Z, R, **TOL)
