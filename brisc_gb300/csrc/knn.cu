@@ -227,9 +227,123 @@ __global__ void k_km_gather(const float* __restrict__ X, const uint32_t* __restr
   C[t] = X[(uint64_t)idx[c] * d + j];
 }
 
-// One CTA per chunk, one thread per dimension: sums[chunk][label][dim] over
-// the chunk's cells in order (zeroed beforehand).
-__global__ void k_km_chunk_sums(const float* __restrict__ X, uint64_t n, uint32_t d,
+// sums[chunk][label][dim] over the chunk's cells in order. A CTA per chunk
+// sorts the cells by label, stably (per-warp counts of consecutive cells in
+// shared memory, their starts label by label, ranks among equal labels of 32
+// cells by warp matches), then a thread per (label, dimension) adds its
+// label's cells in order. The additions of one label are as sequential as
+// before, but those of different labels no longer wait for one another:
+// 300k cells, 2,191 clusters, 50 dimensions: 1.83 ms with a thread per
+// dimension walking the chunk (a chain of 4,096 loads and stores), 0.09 ms.
+constexpr int kSumThreads = 1024;
+constexpr uint32_t kSumMaxChunk = 16384;
+constexpr size_t kSumSmem = 200 * 1024;
+
+// Warps that count separately: as many (up to 32) as fit; 0: none does.
+uint32_t sum_warps(uint32_t chunk, uint32_t nc) {
+  if (chunk > kSumMaxChunk) return 0;
+  for (uint32_t w = kSumThreads / 32; w >= 1; w /= 2)
+    if ((size_t)w * nc * 4 + ((size_t)nc + 1) * 4 + (size_t)chunk * 4 <= kSumSmem) return w;
+  return 0;
+}
+
+__global__ void __launch_bounds__(kSumThreads)
+k_km_chunk_sums(const float* __restrict__ X, uint64_t n, uint32_t d,
+                const uint32_t* __restrict__ labels, uint32_t chunk, uint32_t nc,
+                uint32_t warps, float* __restrict__ sums) {
+  extern __shared__ uint32_t km[];
+  uint32_t* cnt = km;                  // [warps][nc]: counts, then next places
+  uint32_t* start = cnt + warps * nc;  // [nc + 1]
+  uint32_t* order = start + nc + 1;    // [chunk]: cells of the chunk by label
+  __shared__ uint32_t wsum[kSumThreads / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint64_t c0 = (uint64_t)blockIdx.x * chunk;
+  const uint32_t len = (uint32_t)min_u64(chunk, n - c0);
+  const uint32_t per = (len + warps - 1) / warps;
+  const uint32_t a = min(len, (uint32_t)wid * per), b = min(len, a + per);
+  const bool counts = (uint32_t)wid < warps;
+  for (uint32_t t = threadIdx.x; t < warps * nc; t += kSumThreads) cnt[t] = 0u;
+  __syncthreads();
+  uint32_t* my = cnt + (size_t)(counts ? wid : 0) * nc;
+  if (counts)
+    for (uint32_t i = a + lane; i < b; i += 32) atomicAdd(&my[labels[c0 + i]], 1u);
+  __syncthreads();
+  // start of every label: a run of labels per thread, a scan over the threads
+  const uint32_t run = (nc + kSumThreads - 1) / kSumThreads;
+  const uint32_t l0 = min(nc, threadIdx.x * run), l1 = min(nc, l0 + run);
+  uint32_t mine = 0;
+  for (uint32_t l = l0; l < l1; ++l)
+    for (uint32_t w = 0; w < warps; ++w) mine += cnt[w * nc + l];
+  uint32_t incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) wsum[wid] = incl;
+  __syncthreads();
+  uint32_t at = incl - mine;
+  for (int w = 0; w < wid; ++w) at += wsum[w];
+  for (uint32_t l = l0; l < l1; ++l) {
+    start[l] = at;
+    for (uint32_t w = 0; w < warps; ++w) {
+      const uint32_t t = cnt[w * nc + l];
+      cnt[w * nc + l] = at;
+      at += t;
+    }
+  }
+  if (threadIdx.x == 0) start[nc] = len;
+  __syncthreads();
+  if (counts)
+    for (uint32_t i0 = a; i0 < b; i0 += 32) {
+      const uint32_t i = i0 + lane;
+      const uint32_t lab = i < b ? labels[c0 + i] : 0xFFFFFFFFu;
+      const uint32_t peers = __match_any_sync(0xffffffffu, lab);
+      const int leader = __ffs(peers) - 1;
+      uint32_t slot = 0;
+      if (lane == leader && i < b) {
+        slot = my[lab];
+        my[lab] = slot + __popc(peers);
+      }
+      slot = __shfl_sync(0xffffffffu, slot, leader) + __popc(peers & ((1u << lane) - 1u));
+      if (i < b) order[slot] = i;
+      __syncwarp();
+    }
+  __syncthreads();
+  float* out = sums + (uint64_t)blockIdx.x * nc * d;
+  const float* x = X + c0 * d;
+  constexpr int U = 4;  // independent (label, dimension) sums per thread
+  for (uint32_t t0 = threadIdx.x; t0 < nc * d; t0 += kSumThreads * U) {
+    uint32_t s[U], e[U], j[U];
+    float acc[U];
+    uint32_t longest = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t t = t0 + u * kSumThreads, l = t / d;
+      j[u] = t % d;
+      s[u] = t < nc * d ? start[l] : 0u;
+      e[u] = t < nc * d ? start[l + 1] : 0u;
+      acc[u] = 0.f;
+      longest = max(longest, e[u] - s[u]);
+    }
+    for (uint32_t k = 0; k < longest; ++k) {
+      float v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        v[u] = s[u] + k < e[u] ? x[(uint64_t)order[s[u] + k] * d + j[u]] : 0.f;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (s[u] + k < e[u]) acc[u] = acc[u] + v[u];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (t0 + u * kSumThreads < nc * d) out[t0 + u * kSumThreads] = acc[u];
+  }
+}
+
+// The same for chunks or cluster counts past that: a thread per dimension
+// walks the chunk (sums zeroed beforehand).
+__global__ void k_km_chunk_walk(const float* __restrict__ X, uint64_t n, uint32_t d,
                                 const uint32_t* __restrict__ labels, uint32_t chunk,
                                 uint32_t nc, float* __restrict__ sums) {
   const uint64_t c0 = (uint64_t)blockIdx.x * chunk;
@@ -401,9 +515,16 @@ extern "C" int bgpu_kmeans(const float* X, uint32_t* cluster_labels, float* cent
     while (true) {
       BGPU_TRY(km_estep(x, d, Cc, cn, nc, mem + xb, cluster_labels, min_distances,
                         num_cells_per_cluster, err, s));
-      BGPU_CUDA(cudaMemsetAsync(sums, 0, sums_bytes, s));
-      k_km_chunk_sums<<<nchunks, std::min<uint32_t>(128, (d + 31) & ~31u), 0, s>>>(
-          X, n, d, cluster_labels, chunk_size, nc, sums);
+      if (const uint32_t warps = sum_warps(chunk_size, nc)) {
+        BGPU_CUDA(allow_max_smem(k_km_chunk_sums));
+        k_km_chunk_sums<<<nchunks, kSumThreads,
+                          ((size_t)warps * nc + nc + 1 + chunk_size) * 4, s>>>(
+            X, n, d, cluster_labels, chunk_size, nc, warps, sums);
+      } else {
+        BGPU_CUDA(cudaMemsetAsync(sums, 0, sums_bytes, s));
+        k_km_chunk_walk<<<nchunks, std::min<uint32_t>(128, (d + 31) & ~31u), 0, s>>>(
+            X, n, d, cluster_labels, chunk_size, nc, sums);
+      }
       BGPU_CHECK_LAUNCH();
       k_km_reduce<<<(unsigned)ceil_div(per, 256), 256, 0, s>>>(sums, nchunks, nc, d, Cn);
       BGPU_CHECK_LAUNCH();

@@ -234,3 +234,41 @@ def test_knn_self_bit_exact_with_ties(cuda, n, d, nc, k, cs):
     np.testing.assert_array_equal(o["distances"], want_d)
     np.testing.assert_array_equal(o["neighbors"] != 0xFFFFFFFF, have)
     np.testing.assert_array_equal(o["neighbors"][have], so[want_i[have]])
+
+
+@pytest.mark.parametrize("n,d,nc,chunk", [(5, 1, 2, 3), (700, 50, 700, 256), (9000, 33, 1, 4096),
+                                          (20000, 7, 300, 4096), (20000, 5, 40, 20000),
+                                          (3000, 20, 2500, 1000)])
+def test_kmeans_m_step_order(cuda, n, d, nc, chunk):
+    """Centroids after one iteration, bit for bit: each chunk's cells of a
+    cluster added in order, the chunks in order, times the float of 1 / count;
+    chunks that end inside the cells, one cluster, a cluster per cell, and a
+    chunk longer than the sorted path takes."""
+    from brisc_gb300 import knn
+    rng = np.random.default_rng(n)
+    X = rng.standard_normal((n, d)).astype(np.float32)
+    out = dict(cluster_labels=np.zeros(n, np.uint32), min_distances=np.zeros(n, np.float32),
+               cell_norms=np.zeros(0, np.float32), centroids=np.zeros((nc, d), np.float32),
+               centroids_new=np.zeros((nc, d), np.float32),
+               num_cells_per_cluster=np.zeros(nc, np.uint32))
+    assert knn.kmeans(X=X, chunk_size=chunk, num_kmeans_iterations=1, **out) == 1
+    C0 = out["centroids"]  # the initial centroids: cells
+    pd = _fma(np.float32(-2), _chain(X, C0), _norm_chain(C0)[None, :])
+    lab = np.argmin(pd, 1)
+    want = np.zeros((nc, d), np.float32)
+    for c0 in range(0, n, chunk):
+        part = np.zeros((nc, d), np.float32)
+        for i in range(c0, min(n, c0 + chunk)):
+            part[lab[i]] += X[i]
+        want += part
+    count = np.bincount(lab, minlength=nc)
+    assert count.min() > 0
+    want *= (1.0 / count).astype(np.float32)[:, None]
+    np.testing.assert_array_equal(out["centroids_new"], want)
+
+
+def _norm_chain(C):
+    cn = C[:, 0] * C[:, 0]
+    for j in range(1, C.shape[1]):
+        cn = _fma(C[:, j], C[:, j], cn)
+    return cn
