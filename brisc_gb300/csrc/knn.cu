@@ -266,7 +266,8 @@ k_km_chunk_sums(const float* __restrict__ X, uint64_t n, uint32_t d,
   __syncthreads();
   uint32_t* my = cnt + (size_t)(counts ? wid : 0) * nc;
   if (counts)
-    for (uint32_t i = a + lane; i < b; i += 32) atomicAdd(&my[labels[c0 + i]], 1u);
+    for (uint32_t i = a + lane; i < b; i += 32)
+      if (labels[c0 + i] < nc) atomicAdd(&my[labels[c0 + i]], 1u);
   __syncthreads();
   // start of every label: a run of labels per thread, a scan over the threads
   const uint32_t run = (nc + kSumThreads - 1) / kSumThreads;
@@ -292,21 +293,22 @@ k_km_chunk_sums(const float* __restrict__ X, uint64_t n, uint32_t d,
       at += t;
     }
   }
-  if (threadIdx.x == 0) start[nc] = len;
+  if (l1 == nc && l0 < nc) start[nc] = at;  // the thread of the last label
   __syncthreads();
   if (counts)
     for (uint32_t i0 = a; i0 < b; i0 += 32) {
       const uint32_t i = i0 + lane;
-      const uint32_t lab = i < b ? labels[c0 + i] : 0xFFFFFFFFu;
+      const uint32_t l = i < b ? labels[c0 + i] : 0xFFFFFFFFu;
+      const uint32_t lab = l < nc ? l : 0xFFFFFFFFu;
       const uint32_t peers = __match_any_sync(0xffffffffu, lab);
       const int leader = __ffs(peers) - 1;
       uint32_t slot = 0;
-      if (lane == leader && i < b) {
+      if (lane == leader && lab < nc) {
         slot = my[lab];
         my[lab] = slot + __popc(peers);
       }
       slot = __shfl_sync(0xffffffffu, slot, leader) + __popc(peers & ((1u << lane) - 1u));
-      if (i < b) order[slot] = i;
+      if (lab < nc) order[slot] = i;
       __syncwarp();
     }
   __syncthreads();
@@ -351,6 +353,7 @@ __global__ void k_km_chunk_walk(const float* __restrict__ X, uint64_t n, uint32_
   float* base = sums + (uint64_t)blockIdx.x * nc * d;
   for (uint32_t j = threadIdx.x; j < d; j += blockDim.x)
     for (uint64_t i = c0; i < c1; ++i) {
+      if (labels[i] >= nc) continue;
       float* p = base + (uint64_t)labels[i] * d + j;
       *p = *p + X[i * d + j];
     }
@@ -367,10 +370,12 @@ __global__ void k_km_reduce(const float* __restrict__ sums, uint32_t nchunks, ui
   Cn[t] = s;
 }
 
-__global__ void k_km_counts(const uint32_t* __restrict__ labels, uint64_t n,
+// A cell whose distances are all NaN has no label (0xFFFFFFFF) and counts
+// nowhere.
+__global__ void k_km_counts(const uint32_t* __restrict__ labels, uint64_t n, uint32_t nc,
                             uint32_t* __restrict__ counts) {
   const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i < n) atomicAdd(&counts[labels[i]], 1u);  // integer: order-free
+  if (i < n && labels[i] < nc) atomicAdd(&counts[labels[i]], 1u);  // integer: order-free
 }
 
 __global__ void k_km_normalize(float* __restrict__ Cn, const uint32_t* __restrict__ counts,
@@ -385,10 +390,14 @@ __global__ void k_km_normalize(float* __restrict__ Cn, const uint32_t* __restric
 // float sum (relocate_empty_clusters, kmeans.pyx:785-791).
 __global__ void k_km_assigned(const float* __restrict__ X, const uint32_t* __restrict__ lab,
                               const float* __restrict__ C, uint64_t n, uint32_t d,
-                              float* __restrict__ out) {
+                              uint32_t nc, float* __restrict__ out) {
   const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float* x = X + i * d;
+  if (lab[i] >= nc) {  // no label: its distances are NaN
+    out[i] = 0.f;
+    return;
+  }
   const float* c = C + (uint64_t)lab[i] * d;
   float diff = x[0] - c[0];
   float s = diff * diff;
@@ -402,16 +411,17 @@ __global__ void k_km_assigned(const float* __restrict__ X, const uint32_t* __res
 // E step: labels, min distances (= partial distances) and, when counts is
 // given, the cluster sizes. cmem: the centroids' operand.
 int km_estep(const KnnOperand& x, uint32_t d, const float* C, float* cn, uint32_t nc, void* cmem,
-             uint32_t* labels, float* mind, uint32_t* counts, int* err, cudaStream_t s) {
+             uint32_t* replay, uint32_t* labels, float* mind, uint32_t* counts, int* err,
+             cudaStream_t s) {
   const uint64_t n = x.n;
   k_knn_centroid_norms<<<(unsigned)ceil_div(nc, 256), 256, 0, s>>>(C, nc, d, cn);
   BGPU_CHECK_LAUNCH();
   KnnOperand c;
   BGPU_TRY(knn_prepare(&c, C, cn, nc, d, cmem, s));
-  BGPU_TRY(knn_tc_nearest(x, c, d, 1, nullptr, nullptr, labels, mind, err, s));
+  BGPU_TRY(knn_tc_nearest(x, c, d, 1, nullptr, replay, labels, mind, err, s));
   if (counts) {
     BGPU_CUDA(cudaMemsetAsync(counts, 0, (size_t)nc * 4, s));
-    k_km_counts<<<(unsigned)ceil_div(n, 256), 256, 0, s>>>(labels, n, counts);
+    k_km_counts<<<(unsigned)ceil_div(n, 256), 256, 0, s>>>(labels, n, nc, counts);
     BGPU_CHECK_LAUNCH();
   }
   return BGPU_OK;
@@ -476,13 +486,15 @@ extern "C" int bgpu_kmeans(const float* X, uint32_t* cluster_labels, float* cent
   uint32_t* didx = nullptr;
   const size_t xb = round_up(knn_operand_bytes(n, d), 256);
   const size_t cb = round_up(knn_operand_bytes(nc, d), 256);
-  unsigned char* mem = nullptr;  // operands of the cells and the centroids, error word
+  unsigned char* mem = nullptr;  // operands of the cells and the centroids, replays, error word
   float *cn = nullptr, *sums = nullptr, *norms = cell_norms, *own_norms = nullptr;
   BGPU_CUDA(scratch_alloc((void**)&didx, (size_t)nc * 4, s));
   BGPU_CUDA(scratch_alloc((void**)&cn, (size_t)nc * 4, s));
   BGPU_CUDA(scratch_alloc((void**)&sums, sums_bytes, s));
-  BGPU_CUDA(scratch_alloc((void**)&mem, xb + cb + 256, s));
-  int* err = (int*)(mem + xb + cb);
+  const size_t rb = round_up((n + 1) * 4, 256);
+  BGPU_CUDA(scratch_alloc((void**)&mem, xb + cb + rb + 256, s));
+  uint32_t* replay = (uint32_t*)(mem + xb + cb);
+  int* err = (int*)(mem + xb + cb + rb);
   if (!norms) {
     BGPU_CUDA(scratch_alloc((void**)&own_norms, n * 4, s));
     norms = own_norms;
@@ -513,7 +525,7 @@ extern "C" int bgpu_kmeans(const float* X, uint32_t* cluster_labels, float* cent
     uint32_t it = 0;
     std::vector<uint32_t> hcount(nc);
     while (true) {
-      BGPU_TRY(km_estep(x, d, Cc, cn, nc, mem + xb, cluster_labels, min_distances,
+      BGPU_TRY(km_estep(x, d, Cc, cn, nc, mem + xb, replay, cluster_labels, min_distances,
                         num_cells_per_cluster, err, s));
       if (const uint32_t warps = sum_warps(chunk_size, nc)) {
         BGPU_CUDA(allow_max_smem(k_km_chunk_sums));
@@ -538,7 +550,7 @@ extern "C" int bgpu_kmeans(const float* X, uint32_t* cluster_labels, float* cent
         float* dist = nullptr;
         BGPU_CUDA(scratch_alloc((void**)&dist, n * 4, s));
         k_km_assigned<<<(unsigned)ceil_div(n, 256), 256, 0, s>>>(X, cluster_labels, Cc,
-                                                                  n, d, dist);
+                                                                  n, d, nc, dist);
         std::vector<float> hd(n), hx, hcn(per);
         std::vector<uint32_t> hl(n);
         cudaMemcpyAsync(hd.data(), dist, n * 4, cudaMemcpyDeviceToHost, s);
@@ -586,7 +598,7 @@ extern "C" int bgpu_kmeans(const float* X, uint32_t* cluster_labels, float* cent
       old_total = total;
     }
     // the final E step (kmeans.pyx:1100-1153)
-    BGPU_TRY(km_estep(x, d, Cc, cn, nc, mem + xb, cluster_labels, min_distances,
+    BGPU_TRY(km_estep(x, d, Cc, cn, nc, mem + xb, replay, cluster_labels, min_distances,
                       num_cells_per_cluster, err, s));
     *iterations = it;
     return knn_status(err, s);

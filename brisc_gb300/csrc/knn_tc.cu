@@ -27,8 +27,6 @@
 // So each query also keeps the smallest value that its list turned away or
 // gave up, and where that equals the list's worst, the query is listed and
 // k_knn_replay computes it again, every candidate in the reference's order.
-// (The k-means E step keeps the reference's order itself: its cells have no
-// clusters yet, and lists of one entry tighten at once.)
 //
 // Error of s against the exact x.c - |c|^2/2, with X = the query's length and
 // G = the largest length or sqrt |norm| of the tile: the dropped low.low and
@@ -42,13 +40,14 @@
 // Why: the exhaustive FP32 loop is bound by the SIMT pipes (two candidates x
 // four queries per lane, six shared loads per eight multiply-adds: 7.7
 // TFLOP/s). Here the products cost tensor time, the filter two instructions
-// per pair of a 32-column TMEM load, and the exact work is proportional to
-// the list's replacements. 300k x 50 dims, 2,191 clusters, 64 searched, 20
-// neighbours: search 36.7 -> 15.1 ms, nearest clusters 20.9 -> 10.6 ms; the
-// E step against 2,191 centroids 6.07 -> 1.52 ms. What bounds it now is the
-// latency of the exact evaluations (a tile waits for its slowest warp).
+// per pair of a TMEM load, and the exact work is proportional to what passes.
+// 300k x 50 dims, 2,191 clusters, 64 searched, 20 neighbours: search 36.7 ->
+// 6.9 ms, nearest clusters 20.9 -> 2.5 ms, the E step against 2,191 centroids
+// 6.07 -> 0.57 ms. Lists of up to 64 entries take k_knn_two; longer ones
+// k_knn_tc, which keeps its lists while it goes (15.1, 10.6 and 1.52 ms; a
+// tile waits for the exact evaluations of its slowest warp).
 //
-// Shape: 512 threads, one CTA per SM, kQT queries (rows of the MMA), tiles of
+// Shape of k_knn_tc: 512 threads, one CTA per SM, kQT queries (rows of the MMA), tiles of
 // NT candidates. Warp w reads the TMEM lanes (queries) of quarter w % 4 and
 // the columns of quarter w / 4: a thread tests NT / 4 candidates of one query
 // into one mask word. The queries' queues and lists belong to warps (query q
@@ -82,8 +81,9 @@ constexpr uint32_t kNoRun = 0xFFFFFFFFu;
 struct KnnArgs {
   KnnOperand q, c;
   uint32_t d, kp, qt, size;
+  uint32_t stages;  // two passes: operand tiles in flight
   // the cells' clusters: the search, and nearest for cells sorted by cluster
-  // (nullptr: the tiles go in order and ties need no replay)
+  // (nullptr: lists of one entry only, the k-means E step)
   const uint64_t* coff;
   uint32_t nc, cs;
   const uint32_t* nearest;
@@ -243,7 +243,7 @@ __device__ __forceinline__ float row_dot(const float* __restrict__ x, const floa
                                          uint32_t d) {
   float acc = 0.f;
   if constexpr (VEC == 4) {
-#pragma unroll 4
+#pragma unroll 8
     for (uint32_t j = 0; j < d; j += 4) {
       const float4 a = *(const float4*)(x + j), b = *(const float4*)(c + j);
       acc = fmaf(a.x, b.x, acc);
@@ -252,7 +252,7 @@ __device__ __forceinline__ float row_dot(const float* __restrict__ x, const floa
       acc = fmaf(a.w, b.w, acc);
     }
   } else if constexpr (VEC == 2) {
-#pragma unroll 5
+#pragma unroll 13
     for (uint32_t j = 0; j < d; j += 2) {
       const float2 a = *(const float2*)(x + j), b = *(const float2*)(c + j);
       acc = fmaf(a.x, b.x, acc);
@@ -298,6 +298,46 @@ __device__ __forceinline__ void tmem_ld<32>(uint32_t taddr, float (&v)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// The same in two steps, for loads that overlap other work: the values may be
+// used behind tmem_loaded() only, which takes them as operands so that
+// nothing that reads them moves ahead of it.
+template <int N>
+__device__ __forceinline__ void tmem_load(uint32_t taddr, float (&v)[N]);
+template <int N>
+__device__ __forceinline__ void tmem_loaded(float (&v)[N]);
+template <>
+__device__ __forceinline__ void tmem_load<8>(uint32_t taddr, float (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]),
+                 "=f"(v[6]), "=f"(v[7])
+               : "r"(taddr)
+               : "memory");
+}
+template <>
+__device__ __forceinline__ void tmem_loaded<8>(float (&v)[8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]),
+                 "+f"(v[6]), "+f"(v[7])::"memory");
+}
+template <>
+__device__ __forceinline__ void tmem_load<16>(uint32_t taddr, float (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,"
+      "%12,%13,%14,%15}, [%16];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]),
+        "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]),
+        "=f"(v[14]), "=f"(v[15])
+      : "r"(taddr)
+      : "memory");
+}
+template <>
+__device__ __forceinline__ void tmem_loaded<16>(float (&v)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]),
+                 "+f"(v[6]), "+f"(v[7]), "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]),
+                 "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15])::"memory");
 }
 
 // Rows to a tensor-core operand. A block takes 4 groups (32 rows); group
@@ -504,7 +544,6 @@ __global__ void __launch_bounds__(kTcKnnThreads, 1) k_knn_tc(const KnnArgs a) {
   const uint32_t qi = (uint32_t)(wid & 3) * 32u + lane;  // the query this thread filters
   const uint32_t cq = (uint32_t)wid >> 2;                // and its column quarter
   const bool filters = qi < nq;
-  float trun = -INFINITY;  // lists of one entry: the best approximate value, less margins
 
   // Evaluates the first `cnt` queued candidates of query q and offers them.
   auto evaluate = [&](uint32_t q, uint32_t cnt) {
@@ -714,16 +753,11 @@ __global__ void __launch_bounds__(kTcKnnThreads, 1) k_knn_tc(const KnnArgs a) {
           }
           if (filters) {
             const float gm = meta_g[m], mg = kMargin * gm * (qlen[qi] + gm) + 1e-35f;
-            float lim = thr[qi] - mg;
+            const float lim = thr[qi] - mg;
             float top = v[0];  // most threads have nothing above the limit
 #pragma unroll
             for (int j = 1; j + 1 < CW; j += 2) top = max3_nan(top, v[j], v[j + 1]);
             top = max3_nan(top, v[CW - 1], top);
-            if (!SEARCH && R == 1 && a.size == 1) {
-              // one entry: the best approximate value so far bounds it too
-              trun = fmaxf(trun, top - 2.f * mg);
-              lim = fmaxf(lim, trun - mg);
-            }
             if (!(top <= lim)) {  // NaN passes
 #pragma unroll
               for (int j = 0; j < CW; ++j)
@@ -812,104 +846,958 @@ __global__ void __launch_bounds__(kTcKnnThreads, 1) k_knn_tc(const KnnArgs a) {
   }
 }
 
-// The queries in replay[1..replay[0]], a warp each: every candidate evaluated
-// and offered in the reference's order.
-constexpr int kReplayThreads = 128;
-template <int R, bool SEARCH, int VEC>
-__global__ void __launch_bounds__(kReplayThreads) k_knn_replay(const KnnArgs a) {
-  __shared__ float rd[kReplayThreads / 32][R * 32];
-  __shared__ uint32_t ri[kReplayThreads / 32][R * 32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const uint32_t count = a.replay[0], d = a.d;
-  for (uint32_t i = blockIdx.x * (kReplayThreads / 32) + wid; i < count;
-       i += gridDim.x * (kReplayThreads / 32)) {
-    const uint64_t q = a.replay[1 + i];
-    const float* x = a.q.rows + q * d;
-    const float nm = SEARCH ? a.q.norms[q] : 0.f;
-    for (uint32_t e = lane; e < R * 32; e += 32) {
-      rd[wid][e] = e < a.size ? FLT_MAX : -INFINITY;
-      ri[wid][e] = 0xFFFFFFFFu;
+// Lists of up to 64 entries in two passes over the candidates, without a list
+// that has to be kept up to date:
+//  1. each thread (one query, a quarter of every tile's columns) keeps the M
+//     largest lower bounds of s (s less the margin) over groups of GS columns:
+//     a group's largest. Groups are disjoint, so the size-th largest of a
+//     query's 4 M bounds has at least `size` candidates at or above it: tau.
+//     Neighbours lie close together in the cells' order, so the search takes
+//     every column by itself (groups of 8 left bounds so loose that 5 % of the
+//     queues of 2.7k cells overflowed); the nearest clusters, whose longer
+//     lists cost more per bound, take 4 at a time.
+//  2. the candidates whose s plus the margin reaches tau, a few more than
+//     `size`, are queued; at the end they are evaluated exactly and ranked by
+//     (distance, row).
+// The products are made twice (tensor time), but nothing in the loop waits for
+// an exact evaluation and no tile waits for its slowest query. Lists of one
+// entry (M == 1) need one pass: the largest lower bound so far, shared by the
+// query's four threads once per tile, is tight after a tile or two; what it
+// lets through is queued with its upper bound, and the final bound drops most
+// of it (E step 0.91 -> 0.57 ms).
+// One warp copies operands up to four tiles ahead, one issues the MMAs into
+// four accumulators, and the 16 filter warps follow at their own pace (barriers
+// per operand and accumulator). Cycles per tile of 128 x 128, of which the 12
+// MMAs take ~700: 4,700 with two buffers of each and one warp for both roles;
+// 3,100 while the copy warp looked up each tile's runs and norms in turn and
+// copied 8 rows at a time (1,250 cycles of issue); ~2,000 now, the filter's
+// instructions in the first pass, the MMAs in the second. A thread first takes
+// the largest of each slot's 8 values; almost always that ends it.
+// Queued candidates past the queue's room (margins too wide for the data), and
+// lists whose last distance is tied, are listed for k_knn_replay. Lists of
+// one entry need no tie rule: the first of equal distances is the lowest row.
+constexpr int kTwoThreads = kTcKnnThreads + 64;  // and the copy and MMA warps
+constexpr uint32_t kTwoAcc = 4;                  // accumulators in TMEM
+constexpr uint32_t kTwoMeta = 8;                 // tile descriptions in flight
+// queries evaluated together: lists of one entry have few rows each to wait for
+__host__ __device__ constexpr uint32_t eval_batch(bool one) { return one ? 128u : 64u; }
+constexpr uint32_t kRowChunk = 32;               // dimensions of a row staged at once
+
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src),
+               "n"(BYTES)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// Exact x.c, in order over the dimensions, for a pair per lane; x lies in
+// shared memory. The rows come by asynchronous copies of consecutive
+// dimensions, all of a chunk's in flight at once, through the warp's shared
+// `buf` (row stride kRowChunk + VEC: no bank conflicts). A lane that walks its
+// own row takes 32 sectors per load, reads each of them more than once, and
+// waits for L2 once per few loads: 132k cycles for the 9.7k pairs of 128
+// queries of the nearest clusters, 93k so.
+template <int VEC>
+__device__ __forceinline__ float staged_dot(const float* x, const float* __restrict__ rows,
+                                            uint32_t row, uint32_t d, float* buf, int lane) {
+  constexpr int LPR = kRowChunk / VEC;  // lanes per row, and copies per lane
+  constexpr int RPC = 32 / LPR;         // rows per copy
+  constexpr int S = kRowChunk + VEC;
+  const uint32_t at = (uint32_t)(lane % LPR) * VEC;
+  const int r0 = lane / LPR;
+  float acc = 0.f;
+  for (uint32_t j0 = 0; j0 < d; j0 += kRowChunk) {
+    __syncwarp();  // the chunk before has been read
+#pragma unroll
+    for (int i = 0; i < LPR; ++i) {
+      const uint32_t r = __shfl_sync(0xffffffffu, row, i * RPC + r0);
+      if (j0 + at < d)
+        cp_async<VEC * 4>(buf + (i * RPC + r0) * S + at, rows + (uint64_t)r * d + j0 + at);
     }
+    cp_async_wait();
     __syncwarp();
-    WarpList<R> best;
-    best.load(rd[wid], ri[wid], lane);
-    auto offer_rows = [&](uint64_t b, uint64_t e) {
-      for (uint64_t r0 = b; r0 < e; r0 += 32) {
-        const uint64_t row = r0 + lane;
-        const bool use = row < e && !(SEARCH && row == q);
-        float dist = INFINITY;
-        if (use) {
-          const float pd = fmaf(-2.f, row_dot<VEC>(x, a.c.rows + row * d, d), a.c.norms[row]);
-          dist = SEARCH ? nm + pd : pd;
+#pragma unroll
+    for (int k = 0; k < (int)kRowChunk; k += VEC) {
+      if (j0 + k < d) {
+        float c[VEC], v[VEC];
+        if constexpr (VEC == 4) {
+          *(float4*)c = *(const float4*)(buf + lane * S + k);
+          *(float4*)v = *(const float4*)(x + j0 + k);
+        } else if constexpr (VEC == 2) {
+          *(float2*)c = *(const float2*)(buf + lane * S + k);
+          *(float2*)v = *(const float2*)(x + j0 + k);
+        } else {
+          c[0] = buf[lane * S + k];
+          v[0] = x[j0 + k];
         }
-        best.offer(dist, (uint32_t)row, __ballot_sync(0xffffffffu, use), lane, 0.f);
-      }
-    };
-    if constexpr (SEARCH) {
-      uint32_t lab[8];  // the searched clusters, ascending: the least above the last
 #pragma unroll
-      for (int u = 0; u < 8; ++u)
-        lab[u] = lane + 32u * u < a.cs ? a.nearest[q * a.cs + lane + 32u * u] : 0xFFFFFFFFu;
-      uint32_t from = 0;
-      while (true) {
-        uint32_t m = 0xFFFFFFFFu;
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-          if (lab[u] >= from) m = min(m, lab[u]);
-        m = __reduce_min_sync(0xffffffffu, m);
-        if (m >= a.nc) break;
-        offer_rows(a.coff[m], a.coff[m + 1]);
-        from = m + 1;
+        for (int i = 0; i < VEC; ++i) acc = fmaf(v[i], c[i], acc);
       }
-    } else {
-      offer_rows(0, a.c.n);
     }
-    best.store(rd[wid], ri[wid], lane);
-    __syncwarp();
-    write_sorted(rd[wid], ri[wid], a.size, SEARCH ? a.id_map : nullptr, a.out_d + q * a.size,
-                 a.out_id + q * a.size, lane);
-    __syncwarp();
+  }
+  return acc;
+}
+
+struct TwoSmem {  // byte offsets
+  uint32_t a, b, x, rows, queue, upper, tau, qlen, qnorm, qcnt, qat, runs, qmask, bitmap, total;
+};
+
+__host__ __device__ inline TwoSmem two_smem(uint32_t d, uint32_t kp, uint32_t qt, uint32_t nt,
+                                            uint32_t cap, uint32_t stages, uint32_t vec,
+                                            bool one, bool search, uint32_t nc) {
+  TwoSmem L;
+  uint32_t o = 1024;
+  auto take = [&](uint32_t bytes) {
+    const uint32_t at = o;
+    o += (bytes + 127u) & ~127u;
+    return at;
+  };
+  L.a = take(qt / 8 * group_bytes(kp));
+  L.b = take(stages * (nt / 8) * group_bytes(kp));
+  // the MMA reads 128 rows of A: the bytes past the queries' are B's
+  if (o < L.a + 16 * group_bytes(kp)) o = L.a + 16 * group_bytes(kp);
+  // at the end these take the operands' place, for a batch of queries: the
+  // exact distances of what is queued, the queries, and rows on their way
+  const uint32_t batch = qt < eval_batch(one) ? qt : eval_batch(one), end = o;
+  o = L.a;
+  take(batch * cap * 4);
+  L.x = take(batch * d * 4);
+  L.rows = take(kTwoThreads * (kRowChunk + vec) * 4);
+  if (o < end) o = end;
+  L.queue = take(qt * cap * 4);  // pass 1: the bounds, 4 M <= cap per query
+  L.upper = take(one ? qt * cap * 4 : 16);
+  L.tau = take(qt * 4);
+  L.qlen = take(qt * 4);
+  L.qnorm = take(qt * 4);
+  L.qcnt = take(qt * 4);
+  L.qat = take((3 * qt + 1) * 4);
+  L.runs = take(search ? kUnionCap * 12 + 4 : 16);
+  L.qmask = take(search ? kUnionCap * 16 : 16);
+  L.bitmap = take(search ? (nc + 31) / 32 * 8 : 16);  // words and their ranks
+  L.total = o;
+  return L;
+}
+
+// A bound as a number that orders like it does; -inf is the smallest in use.
+__device__ __forceinline__ uint32_t order_key(float f) {
+  const uint32_t w = __float_as_uint(f);
+  return w & 0x80000000u ? ~w : w | 0x80000000u;
+}
+__device__ __forceinline__ float key_value(uint32_t key) {
+  return __uint_as_float(key & 0x80000000u ? key & 0x7FFFFFFFu : ~key);
+}
+
+template <int M, int GS, int CAP, bool SEARCH, int NT, int VEC>
+__global__ void __launch_bounds__(kTwoThreads, 1) k_knn_two(const KnnArgs a) {
+  constexpr int CW = NT / 4;          // candidates a thread tests per tile
+  constexpr int CS = CW / 8;          // of its slots
+  constexpr uint32_t SLOTS = NT / 8;  // 8-row groups per tile
+  static_assert(M == 1 || 4 * M <= CAP, "the bounds of pass 1 lie in the queue's place");
+  extern __shared__ __align__(1024) unsigned char smem[];
+  uint64_t* bfull = reinterpret_cast<uint64_t*>(smem);       // [4] operand of a tile landed
+  uint64_t* bfree = reinterpret_cast<uint64_t*>(smem) + 4;   // [4] operand used
+  uint64_t* mfull = reinterpret_cast<uint64_t*>(smem) + 8;   // [4] MMAs of a tile done
+  uint64_t* mfree = reinterpret_cast<uint64_t*>(smem) + 12;  // [4] accumulator read
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + 256);
+  // per slot of a tile: first row, run, rows of the run (bits), norm bound
+  __shared__ uint32_t meta_row[kTwoMeta][16], meta_run[kTwoMeta][16], meta_bits[kTwoMeta][16];
+  __shared__ __align__(16) float meta_g[kTwoMeta][16];
+  __shared__ uint32_t wsum[kTwoThreads / 32], s_union, s_slots;
+  __shared__ volatile int stop;
+  const uint32_t d = a.d, kp = a.kp, QT = a.qt;
+  const uint32_t NB = a.stages;
+  constexpr bool ONE = M == 1;
+  const TwoSmem L = two_smem(d, kp, QT, NT, CAP, NB, VEC, ONE, SEARCH, a.nc);
+  uint32_t* queue = reinterpret_cast<uint32_t*>(smem + L.queue);
+  float* upper = reinterpret_cast<float*>(smem + L.upper);  // ONE: upper bounds of the queued
+  float* tau = reinterpret_cast<float*>(smem + L.tau);
+  uint32_t* best_key = reinterpret_cast<uint32_t*>(tau);  // ONE: largest lower bound so far
+  float* qlen = reinterpret_cast<float*>(smem + L.qlen);
+  float* qnorm = reinterpret_cast<float*>(smem + L.qnorm);
+  uint32_t* qcnt = reinterpret_cast<uint32_t*>(smem + L.qcnt);
+  uint32_t* run_b = reinterpret_cast<uint32_t*>(smem + L.runs);  // run: rows [b, e)
+  uint32_t* run_e = run_b + (SEARCH ? kUnionCap : 1);
+  uint32_t* run_s = run_e + (SEARCH ? kUnionCap : 1);  // first slot; run_s[runs] = slots
+  uint32_t* qmask = reinterpret_cast<uint32_t*>(smem + L.qmask);  // [run][4]
+  uint32_t* bitmap = reinterpret_cast<uint32_t*>(smem + L.bitmap);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const bool copies = wid == kTcKnnWarps;        // the copy warp
+  const bool multiplies = wid == kTcKnnWarps + 1;  // the MMA warp
+  const bool service = copies || multiplies;
+  const uint64_t q0 = blockIdx.x * (uint64_t)QT;
+  const uint32_t nq = (uint32_t)min_u64(QT, a.q.n - q0);
+  const uint32_t gb = group_bytes(kp), kq = kp / 8;
+  const uint32_t base = smem_u32(smem);
+  const uint32_t readers = 4 * (QT / 32);  // warps that read an accumulator
+
+  if (wid == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 ::"r"(smem_u32(tslot)), "n"(kTwoAcc * NT)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (tid == 0) {
+    for (int i = 0; i < 4; ++i) {
+      mbar_init(bfull + i, 1);
+      mbar_init(bfree + i, 1);
+      mbar_init(mfull + i, 2);  // the commit, and the MMA lane for the description
+      mbar_init(mfree + i, readers);
+    }
+    fence_mbar_init();
+    stop = 0;
+  }
+  // the queries' operand, with ones against the candidates' norm columns
+  const uint64_t qgroups = (a.q.n + 7) / 8;
+  for (uint32_t t = tid; t < QT / 8 * (gb / 16); t += kTwoThreads) {
+    const uint32_t g = t / (gb / 16), o = t % (gb / 16);
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (q0 / 8 + g < qgroups)
+      v = *reinterpret_cast<const uint4*>(a.q.tiles + (q0 / 8 + g) * gb + o * 16u);
+    *reinterpret_cast<uint4*>(smem + L.a + g * gb + o * 16u) = v;
+  }
+  __syncthreads();
+  for (uint32_t t = tid; t < QT * kNormCols; t += kTwoThreads) {
+    const uint32_t r = t / kNormCols, j = d + t % kNormCols;
+    *reinterpret_cast<uint16_t*>(smem + L.a + (r >> 3) * gb + (j >> 3) * 128u + (r & 7u) * 16u +
+                                 (j & 7u) * 2u) = 0x3F80u;  // BF16 1.0
+  }
+  for (uint32_t q = tid; q < QT; q += kTwoThreads) {
+    const bool in = q < nq;
+    qlen[q] = in ? a.q.length[q0 + q] : 0.f;
+    qnorm[q] = SEARCH && in ? a.q.norms[q0 + q] : 0.f;
+    qcnt[q] = 0u;
+    if (ONE) best_key[q] = order_key(-INFINITY);
+  }
+  uint32_t nbits = 0;  // searched clusters of the CTA's queries
+  uint32_t own = 0;    // the cluster of the middle query
+  if (a.coff) {
+    const uint64_t mid_row = q0 + nq / 2;
+    uint32_t lo = 0, hi = a.nc;
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) / 2;
+      if (a.coff[mid] <= mid_row) lo = mid;
+      else hi = mid;
+    }
+    own = lo;
+  }
+  if constexpr (SEARCH) {
+    const uint32_t words = (a.nc + 31) / 32;
+    uint32_t* rank = bitmap + words;
+    for (uint32_t w = tid; w < words; w += kTwoThreads) bitmap[w] = 0u;
+    __syncthreads();
+    for (uint32_t t = tid; t < nq * a.cs; t += kTwoThreads) {
+      const uint32_t lab = a.nearest[q0 * a.cs + t];
+      if (lab < a.nc) atomicOr(&bitmap[lab >> 5], 1u << (lab & 31));  // order-free
+    }
+    __syncthreads();
+    // rank of each word: the searched clusters before it
+    const uint32_t per = (words + kTwoThreads - 1) / kTwoThreads;
+    const uint32_t w0 = min(words, tid * per), w1 = min(words, w0 + per);
+    uint32_t cnt = 0;
+    for (uint32_t w = w0; w < w1; ++w) cnt += __popc(bitmap[w]);
+    uint32_t incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) wsum[wid] = incl;
+    __syncthreads();
+    uint32_t pre = incl - cnt;
+    for (int w = 0; w < wid; ++w) pre += wsum[w];
+    for (uint32_t w = w0; w < w1; ++w) {
+      rank[w] = pre;
+      pre += __popc(bitmap[w]);
+    }
+    if (tid == kTwoThreads - 1) s_union = pre;
+    __syncthreads();
+    nbits = s_union;
+  }
+  fence_proxy_async_smem();  // A's generic writes -> tensor-core reads
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tslot;
+  const uint32_t idesc = idesc_bf16(128, NT);
+  const uint32_t qi = (uint32_t)(wid & 3) * 32u + lane;  // the query this thread filters
+  const uint32_t cq = (uint32_t)(wid >> 2) & 3u;         // and its column quarter
+  const bool filters = !service && qi < nq;
+  const bool reads = !service && (uint32_t)(wid & 3) * 32u < QT;
+  const uint32_t qrow = (uint32_t)(q0 + qi);  // the search leaves this row out
+  const float ql = filters ? qlen[qi] : 0.f;
+  const float aq = filters ? 1e-6f * fabsf(qnorm[qi]) + 1e-35f : 0.f;
+  float top[M];
+#pragma unroll
+  for (int i = 0; i < M; ++i) top[i] = -INFINITY;
+  float mytau = -INFINITY;
+
+  uint32_t gt = 0;              // tiles so far: accumulators and phases
+  uint32_t st = 0, phase = 0;   // the operand stage that comes next, its round (parity)
+  bool ok = true;
+  for (int pass = 0; pass < (ONE ? 1 : 2) && ok; ++pass) {
+    uint32_t ubase = 0;
+    do {
+      uint32_t nruns = 1;
+      if constexpr (SEARCH) {
+        // the next kUnionCap searched clusters in label order: their rows, and
+        // which queries search them
+        const uint32_t words = (a.nc + 31) / 32;
+        const uint32_t* rank = bitmap + words;
+        nruns = min(kUnionCap, nbits - ubase);
+        for (uint32_t t = tid; t < nruns * 4; t += kTwoThreads) qmask[t] = 0u;
+        __syncthreads();
+        for (uint32_t w = tid; w < words; w += kTwoThreads) {
+          uint32_t bits = bitmap[w], pos = rank[w];
+          while (bits) {
+            const uint32_t lab = w * 32 + __ffs(bits) - 1;
+            bits &= bits - 1u;
+            if (pos >= ubase && pos - ubase < nruns) {
+              run_b[pos - ubase] = (uint32_t)a.coff[lab];
+              run_e[pos - ubase] = (uint32_t)a.coff[lab + 1];
+            }
+            ++pos;
+          }
+        }
+        for (uint32_t t = tid; t < nq * a.cs; t += kTwoThreads) {
+          const uint32_t lab = a.nearest[q0 * a.cs + t], q = t / a.cs;
+          if (lab >= a.nc) continue;
+          const uint32_t pos =
+              rank[lab >> 5] + __popc(bitmap[lab >> 5] & ((1u << (lab & 31)) - 1u));
+          if (pos >= ubase && pos - ubase < nruns)
+            atomicOr(&qmask[(pos - ubase) * 4 + (q >> 5)], 1u << (q & 31));
+        }
+      } else if (tid == 0) {
+        run_b[0] = 0u;
+        run_e[0] = (uint32_t)a.c.n;
+      }
+      __syncthreads();
+      if (wid == 0) {  // first slot of every run
+        uint32_t total = 0;
+        for (uint32_t u0 = 0; u0 < nruns; u0 += 32) {
+          const uint32_t u = u0 + lane;
+          uint32_t g = 0;
+          if (u < nruns && run_e[u] > run_b[u]) g = (run_e[u] + 7) / 8 - run_b[u] / 8;
+          uint32_t incl = g;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+          }
+          if (u < nruns) run_s[u] = total + incl - g;
+          total += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) {
+          run_s[nruns] = total;
+          s_slots = total;
+        }
+      }
+      __syncthreads();
+      const uint32_t nslots = s_slots;
+      const uint32_t ntiles = (nslots + SLOTS - 1) / SLOTS;
+      // the tile that step t works on: from the own cluster's on, around
+      uint32_t t0 = 0;
+      if (a.coff && ntiles) {
+        uint32_t slot = own / 8;  // nearest: the own centroid's group
+        if constexpr (SEARCH) {
+          const uint32_t* rank = bitmap + (a.nc + 31) / 32;
+          const uint32_t pos =
+              rank[own >> 5] + __popc(bitmap[own >> 5] & ((1u << (own & 31)) - 1u));
+          slot = pos >= ubase && pos - ubase < nruns ? run_s[pos - ubase] : 0u;
+        }
+        t0 = min(slot / SLOTS, ntiles - 1);
+      }
+
+      if (copies) {
+        // ---- copies: tile t's description, then its operand into stage g % NB,
+        // whose MMAs (tile g - NB) have completed. The description is looked up
+        // one tile ahead: its chain of shared and global loads is as long as a
+        // tile's MMAs.
+        uint32_t group = 0, u = kNoRun, bits = 0, walk = 0;
+        float gm = 0.f;
+        auto look_up = [&](uint32_t t) {
+          const uint32_t slot = (t0 + t < ntiles ? t0 + t : t0 + t - ntiles) * SLOTS + lane;
+          group = 0, u = kNoRun, bits = 0;
+          gm = 0.f;
+          if ((uint32_t)lane < SLOTS && slot < nslots) {
+            if (t0 + t == ntiles) walk = 0;
+            if (t == 0) {
+              uint32_t hi = nruns;  // the last run that starts at or before slot
+              while (hi - walk > 1) {
+                const uint32_t mid = (walk + hi) / 2;
+                if (run_s[mid] <= slot) walk = mid;
+                else hi = mid;
+              }
+            } else {
+              while (run_s[walk + 1] <= slot) ++walk;  // run_s[nruns] = nslots
+            }
+            u = walk;
+            group = run_b[u] / 8 + (slot - run_s[u]);
+            gm = a.c.gmax[group];
+            const uint32_t r0 = group * 8, rb = max(run_b[u], r0) - r0;
+            const uint32_t re = min(run_e[u] - r0, 8u);
+            bits = ((1u << re) - 1u) & ~((1u << rb) - 1u);
+          }
+        };
+        if (ntiles) look_up(0);
+        for (uint32_t t = 0; t < ntiles; ++t) {
+          const uint32_t g = gt + t, m = g % kTwoMeta;
+          int fine = 1;
+          if (g >= NB && lane == 0) fine = tc_wait(bfree + st, phase ^ 1u, &stop, a.err);
+          fine = __shfl_sync(0xffffffffu, fine, 0);
+          if (!fine) break;
+          // description slot m: its last tile, g - 8, was read before tile g -
+          // NB's MMAs were issued (they follow the readers of tile g - NB - 4)
+          const unsigned used = __ballot_sync(0xffffffffu, u != kNoRun);
+          if ((uint32_t)lane < SLOTS) {
+            meta_row[m][lane] = group * 8;
+            meta_run[m][lane] = u;
+            meta_bits[m][lane] = bits;
+            meta_g[m][lane] = gm;
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive_expect_tx(bfull + st, __popc(used) * gb);
+          __syncwarp();
+          // one copy per stretch of successive groups: a copy's issue costs
+          // ~70 cycles, 16 of them more than the tile's MMAs
+          const uint32_t before = __shfl_up_sync(0xffffffffu, group, 1);
+          const bool starts = lane == 0 || group != before + 1;
+          const unsigned heads = __ballot_sync(0xffffffffu, starts) & used;
+          if ((heads >> lane) & 1u) {
+            const unsigned later = heads & ~((2u << lane) - 1u);
+            const uint32_t end = later ? __ffs(later) - 1u : __popc(used);
+            bulk_g2s(smem + L.b + (st * SLOTS + lane) * gb, a.c.tiles + (uint64_t)group * gb,
+                     (end - lane) * gb, bfull + st);
+          }
+          if (++st == NB) st = 0, phase ^= 1u;
+          if (t + 1 < ntiles) look_up(t + 1);
+        }
+      } else if (multiplies) {
+        // ---- MMAs: tile t into accumulator g % 4, which the readers of tile
+        // g - 4 have left
+        if (elect_lane()) {
+          const uint64_t ah0 = smem_desc(base + L.a, 128u, gb);
+          const uint64_t bh0 = smem_desc(base + L.b, 128u, gb);
+          const uint32_t low = kq * 128u >> 4;  // from the high parts to the low ones
+          for (uint32_t t = 0; t < ntiles; ++t) {
+            const uint32_t g = gt + t, b = g % kTwoAcc;
+            if (g >= kTwoAcc && !tc_wait(mfree + b, (g / kTwoAcc - 1u) & 1u, &stop, a.err)) break;
+            if (!tc_wait(bfull + st, phase, &stop, a.err)) break;
+            tc_fence_after();
+            const uint32_t acc = tmem + b * NT;
+            uint64_t ah = ah0, bh = bh0 + (st * SLOTS * gb >> 4);
+            for (uint32_t ks = 0; ks < kp / 16; ++ks) {
+              mma_bf16(acc, ah, bh + low, idesc, ks ? 1u : 0u);
+              mma_bf16(acc, ah + low, bh, idesc, 1u);
+              mma_bf16(acc, ah, bh, idesc, 1u);
+              ah += 16;  // 256 bytes
+              bh += 16;
+            }
+            mma_commit(bfree + st);
+            mma_commit(mfull + b);
+            mbar_arrive(mfull + b);  // passes the tile's description on
+            if (++st == NB) st = 0, phase ^= 1u;
+          }
+        }
+        __syncwarp();
+      } else if (reads) {
+        // ---- filter warps: half of the thread's columns are tested while the
+        // load of the next half (or of the next tile's first half) is in flight
+        constexpr int HW = CW / 2, HS = CS / 2;
+        const uint32_t lanes = tmem + cq * CW + ((uint32_t)(wid & 3) << 21);
+        auto ready = [&](uint32_t t) -> bool {
+          const uint32_t g = gt + t;
+          const int done = __shfl_sync(0xffffffffu,
+                                       lane == 0 ? (int)tc_wait(mfull + g % kTwoAcc,
+                                                                (g / kTwoAcc) & 1u, &stop, a.err)
+                                                 : 0,
+                                       0);
+          tc_fence_after();
+          return done != 0;
+        };
+        auto test = [&](float* v, uint32_t m, uint32_t slot0) {
+          float gs[HS], mx[HS];
+#pragma unroll
+          for (int i = 0; i < HS; ++i) {
+            const float* w = v + 8 * i;
+            gs[i] = meta_g[m][slot0 + i];
+            mx[i] = max3_nan(max3_nan(w[0], w[1], w[2]), max3_nan(w[3], w[4], w[5]),
+                             max3_nan(w[6], w[7], w[7]));
+          }
+#pragma unroll
+          for (int i = 0; i < HS; ++i) {
+            const float* w = v + 8 * i;
+            const float mg = kMargin * gs[i] * (ql + gs[i]) + aq;
+            const float lim = ONE ? mytau - mg : pass == 0 ? top[M - 1] + mg : mytau - mg;
+            if (mx[i] <= lim || !filters) continue;  // NaN goes on
+            const uint32_t slot = slot0 + i, u = meta_run[m][slot], row = meta_row[m][slot];
+            uint32_t left = u != kNoRun ? meta_bits[m][slot] : 0u;
+            if (SEARCH) {
+              if (u == kNoRun || !((qmask[u * 4 + (qi >> 5)] >> (qi & 31)) & 1u)) left = 0u;
+              if (qrow - row < 8u) left &= ~(1u << (qrow - row));
+            }
+            if (!left) continue;
+            if constexpr (ONE) {
+              float x = -INFINITY;  // NaN and what overflows are no bound
+#pragma unroll
+              for (int k = 0; k < 8; ++k)
+                if (((left >> k) & 1u) && w[k] < 1e37f) x = fmaxf(x, w[k]);
+              mytau = fmaxf(mytau, x - mg);
+#pragma unroll
+              for (int k = 0; k < 8; ++k)
+                if (((left >> k) & 1u) && !(w[k] <= mytau - mg)) {
+                  const uint32_t pos = atomicAdd(&qcnt[qi], 1u);
+                  if (pos < (uint32_t)CAP) {
+                    queue[qi * CAP + pos] = row + k;
+                    upper[qi * CAP + pos] = w[k] + mg;
+                  }
+                }
+            } else if (pass == 0) {
+#pragma unroll
+              for (int k = 0; k < 8; k += GS) {
+                float x = -INFINITY;  // NaN and what overflows are no bound
+#pragma unroll
+                for (int j = k; j < k + GS; ++j)
+                  if (((left >> j) & 1u) && w[j] < 1e37f) x = fmaxf(x, w[j]);
+                x -= mg;
+                if (x > top[M - 1]) {
+#pragma unroll
+                  for (int n = M - 1; n > 0; --n) top[n] = fmaxf(top[n], fminf(top[n - 1], x));
+                  top[0] = fmaxf(top[0], x);
+                }
+              }
+            } else {
+#pragma unroll
+              for (int k = 0; k < 8; ++k)
+                if (((left >> k) & 1u) && !(w[k] <= lim)) {
+                  const uint32_t pos = atomicAdd(&qcnt[qi], 1u);
+                  if (pos < (uint32_t)CAP) queue[qi * CAP + pos] = row + k;
+                }
+            }
+          }
+        };
+        float v0[HW], v1[HW];
+        bool go = ntiles > 0 && ready(0);
+        if (go) tmem_load<HW>(lanes + (gt % kTwoAcc) * NT, v0);
+        for (uint32_t t = 0; t < ntiles && go; ++t) {
+          const uint32_t g = gt + t, b = g % kTwoAcc, m = g % kTwoMeta;
+          tmem_loaded<HW>(v0);
+          tmem_load<HW>(lanes + b * NT + HW, v1);
+          float seen = mytau;
+          if constexpr (ONE) mytau = seen = filters ? key_value(best_key[qi]) : mytau;
+          test(v0, m, cq * CS);
+          tmem_loaded<HW>(v1);
+          tc_fence_before();
+          if (t + 1 < ntiles) {
+            go = ready(t + 1);
+            if (go) tmem_load<HW>(lanes + ((g + 1) % kTwoAcc) * NT, v0);
+          }
+          test(v1, m, cq * CS + HS);
+          if (ONE && mytau > seen) atomicMax(&best_key[qi], order_key(mytau));
+          __syncwarp();
+          if (lane == 0) mbar_arrive(mfree + b);  // values and description are read
+        }
+      }
+      gt += ntiles;
+      st = gt % NB;
+      phase = (gt / NB) & 1u;
+      ubase += nruns;
+      ok = !__syncthreads_or(stop);  // and the runs are no longer read
+    } while (SEARCH && ok && ubase < nbits);
+    if (!ONE && pass == 0 && ok) {
+      float* bound = reinterpret_cast<float*>(queue);  // [query][4 M]
+      if (filters)
+#pragma unroll
+        for (int i = 0; i < M; ++i) bound[qi * CAP + cq * M + i] = top[i];
+      __syncthreads();
+      if (!service) {
+        // tau: the size-th largest bound, the largest number with 23 leading
+        // bits that at least `size` bounds reach, bit by bit (keys: floats in
+        // the order of integers), four queries at a time: a bit's votes wait
+        // for the bit before
+        constexpr int E = (4 * M + 31) / 32, Q = 4;
+        for (uint32_t q1 = wid * Q; q1 < nq; q1 += kTcKnnWarps * Q) {
+          uint32_t key[Q][E], cut[Q];
+#pragma unroll
+          for (int i = 0; i < Q; ++i) {
+            const uint32_t q = min(q1 + i, nq - 1);
+            cut[i] = 0;
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+              const int n = e * 32 + lane;
+              key[i][e] = n < 4 * M ? order_key(bound[q * CAP + n]) : 0u;  // 0: no bound
+            }
+          }
+          for (uint32_t bit = 0x80000000u; bit >= 0x200u; bit >>= 1) {
+#pragma unroll
+            for (int i = 0; i < Q; ++i) {
+              uint32_t have = 0;
+#pragma unroll
+              for (int e = 0; e < E; ++e)
+                have += __popc(__ballot_sync(0xffffffffu, key[i][e] >= (cut[i] | bit)));
+              if (have >= a.size) cut[i] |= bit;
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < Q; ++i) {
+            // back to a float; fewer bounds than entries: no limit
+            float t = key_value(cut[i]);
+            if (cut[i] <= 0x007FFFFFu) t = -INFINITY;  // -inf's key and below
+            if (lane == i && q1 + i < nq) tau[q1 + i] = t;
+          }
+        }
+      }
+      __syncthreads();
+      if (filters) mytau = tau[qi];
+    }
+  }
+
+  if (ok) {
+    // The exact distances of what is queued, a thread per (query, entry) over
+    // the whole CTA (a warp per query instead waits for its few rows alone,
+    // eight times in turn), where the operands were; then the entries' ranks.
+    uint32_t* at = reinterpret_cast<uint32_t*>(smem + L.qat);  // first entry of each query
+    uint32_t* qbad = at + QT + 1;                              // entries that no list keeps
+    uint32_t* ranks = qbad + QT;                               // sum of the others' ranks
+    float* dists = reinterpret_cast<float*>(smem + L.a);       // [query of the batch][CAP]
+    float* xs = reinterpret_cast<float*>(smem + L.x);          // [query of the batch][d]
+    float* buf = reinterpret_cast<float*>(smem + L.rows) + wid * 32 * (kRowChunk + VEC);
+    float *last = tau, *next = qlen;  // distances of entries size - 1 and size
+    for (uint32_t q = tid; q < QT; q += kTwoThreads) {
+      if constexpr (ONE) {  // only what reaches the final bound
+        const uint32_t cnt = qcnt[q];
+        const float bound = key_value(best_key[q]);
+        uint32_t kept = 0;
+        if (cnt <= (uint32_t)CAP) {
+          for (uint32_t e = 0; e < cnt; ++e)
+            if (!(upper[q * CAP + e] < bound)) queue[q * CAP + kept++] = queue[q * CAP + e];
+          qcnt[q] = kept;
+        }
+      }
+      qbad[q] = ranks[q] = 0u;
+      last[q] = next[q] = INFINITY;
+    }
+    if (ONE) __syncthreads();
+    if (wid == 0) {
+      uint32_t total = 0;
+      for (uint32_t p0 = 0; p0 < QT; p0 += 32) {
+        const uint32_t q = p0 + lane;
+        const uint32_t c = q < nq && qcnt[q] <= (uint32_t)CAP ? qcnt[q] : 0u;
+        uint32_t incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += v;
+        }
+        if (q < QT) at[q] = total + incl - c;
+        total += __shfl_sync(0xffffffffu, incl, 31);
+      }
+      if (lane == 0) at[QT] = total;
+    }
+    constexpr uint32_t BATCH = eval_batch(ONE);
+    for (uint32_t qb = 0; qb < nq; qb += BATCH) {
+      const uint32_t qe = min(qb + BATCH, nq);
+      const float* src = a.q.rows + (q0 + qb) * d;
+      for (uint32_t t = tid * VEC; t < (qe - qb) * d; t += kTwoThreads * VEC) {
+        if constexpr (VEC == 4) *(float4*)(xs + t) = *(const float4*)(src + t);
+        else if constexpr (VEC == 2) *(float2*)(xs + t) = *(const float2*)(src + t);
+        else xs[t] = src[t];
+      }
+      __syncthreads();
+      const uint32_t first = at[qb], entries = at[qe];
+      auto owner = [&](uint32_t t) {  // the batch's last query that starts at or before t
+        uint32_t q = qb, hi = qe;
+        while (hi - q > 1) {
+          const uint32_t mid = (q + hi) / 2;
+          if (at[mid] <= t) q = mid;
+          else hi = mid;
+        }
+        return q;
+      };
+      for (uint32_t t0 = first + wid * 32u; t0 < entries; t0 += kTwoThreads) {
+        const uint32_t t = min(t0 + lane, entries - 1), q = owner(t), self = t - at[q];
+        const uint32_t row = queue[q * CAP + self];
+        const float cn = a.c.norms[row];
+        const float dot = staged_dot<VEC>(xs + (q - qb) * d, a.c.rows, row, d, buf, lane);
+        const float pd = fmaf(-2.f, dot, cn);  // |c|^2 - 2 x.c
+        const float ds = SEARCH ? qnorm[q] + pd : pd;
+        // what is not finite is never kept, as by the lists
+        dists[(q - qb) * CAP + self] = ds < FLT_MAX ? ds : INFINITY;
+      }
+      __syncthreads();
+      auto put = [&](uint32_t q, uint32_t rank, float de, uint32_t id) {
+        if (rank < a.size) {
+          a.out_d[(q0 + q) * a.size + rank] = de;
+          a.out_id[(q0 + q) * a.size + rank] = SEARCH ? a.id_map[id] : id;
+        }
+        if (rank == a.size - 1) last[q] = de;
+        if (rank == a.size) next[q] = de;
+      };
+      // rank: the closer entries, as if no two were equally close
+      for (uint32_t t = first + tid; t < entries; t += kTwoThreads) {
+        const uint32_t q = owner(t), cnt = at[q + 1] - at[q], self = t - at[q];
+        const float* dist = dists + (q - qb) * CAP;
+        const float de = dist[self];
+        if (!(de < FLT_MAX)) {
+          atomicAdd(&qbad[q], 1u);
+          continue;
+        }
+        uint32_t rank = 0, f = 0;
+        for (; f + 4 <= cnt; f += 4) {
+          const float4 v = *reinterpret_cast<const float4*>(dist + f);
+          rank += (v.x < de) + (v.y < de) + (v.z < de) + (v.w < de);
+        }
+        for (; f < cnt; ++f) rank += dist[f] < de;
+        atomicAdd(&ranks[q], rank);
+        put(q, rank, de, queue[q * CAP + self]);
+      }
+      __syncthreads();
+      // the ranks add up to 0 + 1 + .. unless some are equal: then by row too
+      for (uint32_t q = qb + wid; q < qe; q += kTwoThreads / 32) {
+        const uint32_t cnt = at[q + 1] - at[q], valid = cnt - qbad[q];
+        if (ranks[q] != valid * (valid - 1u) / 2u) {
+          const float* dist = dists + (q - qb) * CAP;
+          const uint32_t* ids = queue + q * CAP;
+          for (uint32_t e = lane; e < cnt; e += 32) {
+            const float de = dist[e];
+            uint32_t rank = 0;
+            for (uint32_t f = 0; f < cnt; ++f)
+              rank += dist[f] < de || (dist[f] == de && ids[f] < ids[e]);
+            if (de < FLT_MAX) put(q, rank, de, ids[e]);
+          }
+          __syncwarp();
+        }
+        const bool over = qcnt[q] > (uint32_t)CAP;
+        if (lane == 0 && (over || (a.size > 1 && valid > a.size && last[q] == next[q])))
+          a.replay[1 + atomicAdd(a.replay, 1u)] = (uint32_t)(q0 + q);
+        if (!over)
+          for (uint32_t e = valid + lane; e < a.size; e += 32) {  // empty entries
+            a.out_d[(q0 + q) * a.size + e] = FLT_MAX;
+            a.out_id[(q0 + q) * a.size + e] = 0xFFFFFFFFu;
+          }
+      }
+      __syncthreads();
+    }
+  } else if (tid == 0) {
+    // a wait ran out: the copies and MMAs in flight end (waits with a limit)
+    // before shared memory and TMEM go back
+    const long long until = clock64() + (1LL << 30);
+    for (int i = 0; i < 4; ++i)
+      for (uint32_t phase = 0; phase < 2; ++phase)
+        while (clock64() < until && !(mbar_test(bfull + i, phase) && mbar_test(mfull + i, phase)))
+          __nanosleep(64);
+  }
+  __syncthreads();
+  tc_fence_after();
+  if (wid == 0) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
+                 ::"r"(tmem), "n"(kTwoAcc * NT)
+                 : "memory");
   }
 }
 
+// The queries in replay[1..replay[0]], a CTA each: every candidate evaluated
+// (kReplayBatch at a time, a thread each) and offered by one warp in the
+// reference's order. The searched clusters' rows are one sequence: batches that
+// ended with each cluster of ~137 rows took 0.69 ms for 38 queries of 8.8k
+// candidates (three barriers and a latency per cluster), 0.35 ms so.
+constexpr int kReplayThreads = 256;
+constexpr uint32_t kReplayBatch = 1024;
+template <int R, bool SEARCH, int VEC>
+__global__ void __launch_bounds__(kReplayThreads) k_knn_replay(const KnnArgs a) {
+  __shared__ float rd[R * 32];
+  __shared__ uint32_t ri[R * 32];
+  __shared__ float dist[kReplayBatch];
+  __shared__ uint32_t ids[kReplayBatch];
+  // the searched clusters in label order: first row, rows before them
+  __shared__ uint32_t lab[SEARCH ? kReplayThreads : 1], begin[SEARCH ? kReplayThreads : 1];
+  __shared__ uint32_t before[SEARCH ? kReplayThreads + 1 : 1], wsum[kReplayThreads / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint32_t count = a.replay[0], d = a.d;
+  for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
+    const uint64_t q = a.replay[1 + i];
+    const float* x = a.q.rows + q * d;
+    const float nm = SEARCH ? a.q.norms[q] : 0.f;
+    for (uint32_t e = threadIdx.x; e < R * 32; e += kReplayThreads) {
+      rd[e] = e < a.size ? FLT_MAX : -INFINITY;
+      ri[e] = 0xFFFFFFFFu;
+    }
+    uint32_t total = (uint32_t)a.c.n;
+    if constexpr (SEARCH) {
+      const uint32_t u = threadIdx.x;
+      const uint32_t mine = u < a.cs ? a.nearest[q * a.cs + u] : 0xFFFFFFFFu;
+      lab[u] = mine;
+      __syncthreads();
+      uint32_t rank = 0;  // labels are distinct, except of clusters that do not exist
+      for (uint32_t v = 0; v < (uint32_t)kReplayThreads; ++v)
+        rank += lab[v] < mine || (lab[v] == mine && v < u);
+      __syncthreads();
+      lab[rank] = mine;
+      __syncthreads();
+      const uint32_t l = lab[u];
+      const bool has = l < a.nc && (u == 0 || lab[u - 1] != l);
+      const uint32_t first = has ? (uint32_t)a.coff[l] : 0u;
+      const uint32_t size = has ? (uint32_t)a.coff[l + 1] - first : 0u;
+      begin[u] = first;
+      uint32_t incl = size;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (lane == 31) wsum[wid] = incl;
+      __syncthreads();
+      for (int w = 0; w < wid; ++w) incl += wsum[w];
+      before[u] = incl - size;
+      if (u == kReplayThreads - 1) before[kReplayThreads] = incl;
+      __syncthreads();
+      total = before[kReplayThreads];
+    }
+    __syncthreads();
+    WarpList<R> best;  // warp 0's
+    if (wid == 0) best.load(rd, ri, lane);
+    for (uint64_t r0 = 0; r0 < total; r0 += kReplayBatch) {
+      const uint32_t len = (uint32_t)min_u64(kReplayBatch, total - r0);
+      for (uint32_t k = threadIdx.x; k < len; k += kReplayThreads) {
+        uint32_t row = (uint32_t)r0 + k;
+        if constexpr (SEARCH) {
+          uint32_t u = 0, hi = kReplayThreads;  // the last cluster that starts at or before it
+          while (hi - u > 1) {
+            const uint32_t mid = (u + hi) / 2;
+            if (before[mid] <= row) u = mid;
+            else hi = mid;
+          }
+          row = begin[u] + (row - before[u]);
+        }
+        const float pd =
+            fmaf(-2.f, row_dot<VEC>(x, a.c.rows + (uint64_t)row * d, d), a.c.norms[row]);
+        dist[k] = SEARCH ? nm + pd : pd;
+        ids[k] = row;
+      }
+      __syncthreads();
+      if (wid == 0)
+        for (uint32_t k = 0; k < len; k += 32) {
+          const bool in = k + lane < len;
+          const uint32_t row = in ? ids[k + lane] : 0u;
+          const bool use = in && !(SEARCH && row == q);
+          best.offer(use ? dist[k + lane] : INFINITY, row, __ballot_sync(0xffffffffu, use), lane,
+                     0.f);
+        }
+      __syncthreads();
+    }
+    if (wid == 0) {
+      best.store(rd, ri, lane);
+      __syncwarp();
+      write_sorted(rd, ri, a.size, SEARCH ? a.id_map : nullptr, a.out_d + q * a.size,
+                   a.out_id + q * a.size, lane);
+    }
+    __syncthreads();
+  }
+}
+
+template <int R, bool SEARCH, int VEC>
+int launch_replay(const KnnArgs& a, cudaStream_t s) {
+  k_knn_replay<R, SEARCH, VEC><<<num_sms() * 4, kReplayThreads, 0, s>>>(a);
+  BGPU_CHECK_LAUNCH();
+  return BGPU_OK;
+}
+
+// at least 120 KB of shared memory, so that one CTA (and one TMEM allocation)
+// runs per SM
 template <int R, bool SEARCH, int NT, int VEC>
-int launch_knn(const KnnArgs& a, cudaStream_t s) {
-  // at least 120 KB so that one CTA (and one TMEM allocation) runs per SM
+int launch_one(const KnnArgs& a, cudaStream_t s) {
   const size_t smem =
       std::max<size_t>(knn_smem(a.kp, a.qt, NT, R, SEARCH, a.nc).total, 120 * 1024);
   BGPU_CUDA((allow_max_smem(k_knn_tc<R, SEARCH, NT, VEC>)));
   k_knn_tc<R, SEARCH, NT, VEC>
       <<<(unsigned)ceil_div(a.q.n, a.qt), kTcKnnThreads, smem, s>>>(a);
   BGPU_CHECK_LAUNCH();
-  if (a.coff) {
-    k_knn_replay<R, SEARCH, VEC><<<num_sms() * 4, kReplayThreads, 0, s>>>(a);
-    BGPU_CHECK_LAUNCH();
-  }
-  return BGPU_OK;
+  return launch_replay<R, SEARCH, VEC>(a, s);
 }
 
-template <int R, bool SEARCH, int NT>
-int launch_vec(const KnnArgs& a, cudaStream_t s) {
+template <int M, int GS, int CAP, bool SEARCH, int NT, int VEC>
+int launch_two(const KnnArgs& a, cudaStream_t s) {
+  const size_t smem = std::max<size_t>(
+      two_smem(a.d, a.kp, a.qt, NT, CAP, a.stages, VEC, M == 1, SEARCH, a.nc).total, 120 * 1024);
+  BGPU_CUDA((allow_max_smem(k_knn_two<M, GS, CAP, SEARCH, NT, VEC>)));
+  k_knn_two<M, GS, CAP, SEARCH, NT, VEC>
+      <<<(unsigned)ceil_div(a.q.n, a.qt), kTwoThreads, smem, s>>>(a);
+  BGPU_CHECK_LAUNCH();
+  return launch_replay<CAP <= 96 ? 1 : 2, SEARCH, VEC>(a, s);
+}
+
+// Dynamic shared memory beside the kernels' static part.
+size_t knn_smem_limit() { return (size_t)device_smem_optin() - 4096; }
+
+// Floats per load of both matrices' rows.
+int row_vec(const KnnArgs& a) {
   const uintptr_t at = (uintptr_t)a.q.rows | (uintptr_t)a.c.rows;
-  if (a.d % 4 == 0 && at % 16 == 0) return launch_knn<R, SEARCH, NT, 4>(a, s);
-  if (a.d % 2 == 0 && at % 8 == 0) return launch_knn<R, SEARCH, NT, 2>(a, s);
-  return launch_knn<R, SEARCH, NT, 1>(a, s);
+  return a.d % 4 == 0 && at % 16 == 0 ? 4 : a.d % 2 == 0 && at % 8 == 0 ? 2 : 1;
 }
 
-// 128-candidate tiles where they fit with 128 queries' lists, else 64; then
-// the most queries per CTA (128, 64, 32) that fit and leave no SM idle.
+// 128-candidate tiles where they fit with 128 queries, else 64; then the most
+// queries per CTA (128, 64, 32) that fit and leave no SM idle. bytes(qt, nt):
+// the kernel's shared memory. Returns nt, 0 where nothing fits.
+template <typename F>
+uint32_t choose_shape(KnnArgs* a, F bytes) {
+  const size_t limit = knn_smem_limit();
+  const uint32_t nt = bytes(128, 128) <= limit ? 128u : 64u;
+  for (a->qt = 128; a->qt > 32; a->qt /= 2)
+    if (bytes(a->qt, nt) <= limit && ceil_div(a->q.n, a->qt) >= (uint64_t)num_sms()) break;
+  return bytes(a->qt, nt) <= limit ? nt : 0u;
+}
+
+template <int M, int GS, int CAP, bool SEARCH>
+int launch_two_shape(KnnArgs a, cudaStream_t s) {
+  const int vec = row_vec(a);
+  auto bytes = [&](uint32_t qt, uint32_t n, uint32_t stages) {
+    return (size_t)two_smem(a.d, a.kp, qt, n, CAP, stages, vec, M == 1, SEARCH, a.nc).total;
+  };
+  const uint32_t nt =
+      choose_shape(&a, [&](uint32_t qt, uint32_t n) { return bytes(qt, n, 2); });
+  BGPU_REQUIRE(nt, BGPU_ERR_UNSUPPORTED,
+               "nearest rows: the queues do not fit one CTA's shared memory");
+  for (a.stages = 4; a.stages > 2 && bytes(a.qt, nt, a.stages) > knn_smem_limit();) --a.stages;
+  if (nt == 128)
+    return vec == 4   ? launch_two<M, GS, CAP, SEARCH, 128, 4>(a, s)
+           : vec == 2 ? launch_two<M, GS, CAP, SEARCH, 128, 2>(a, s)
+                      : launch_two<M, GS, CAP, SEARCH, 128, 1>(a, s);
+  return vec == 4   ? launch_two<M, GS, CAP, SEARCH, 64, 4>(a, s)
+         : vec == 2 ? launch_two<M, GS, CAP, SEARCH, 64, 2>(a, s)
+                    : launch_two<M, GS, CAP, SEARCH, 64, 1>(a, s);
+}
+
 template <int R, bool SEARCH>
-int launch_shape(KnnArgs a, cudaStream_t s) {
-  const size_t limit = (size_t)device_smem_optin() - 2048;
-  const bool wide = knn_smem(a.kp, 128, 128, R, SEARCH, a.nc).total <= limit;
-  const uint32_t nt = wide ? 128u : 64u;
-  for (a.qt = 128; a.qt > 32; a.qt /= 2)
-    if (knn_smem(a.kp, a.qt, nt, R, SEARCH, a.nc).total <= limit &&
-        ceil_div(a.q.n, a.qt) >= (uint64_t)num_sms())
-      break;
-  BGPU_REQUIRE(knn_smem(a.kp, a.qt, nt, R, SEARCH, a.nc).total <= limit, BGPU_ERR_UNSUPPORTED,
+int launch_one_shape(KnnArgs a, cudaStream_t s) {
+  const uint32_t nt = choose_shape(&a, [&](uint32_t qt, uint32_t n) {
+    return (size_t)knn_smem(a.kp, qt, n, R, SEARCH, a.nc).total;
+  });
+  BGPU_REQUIRE(nt, BGPU_ERR_UNSUPPORTED,
                "nearest rows: the lists do not fit one CTA's shared memory");
-  return wide ? launch_vec<R, SEARCH, 128>(a, s) : launch_vec<R, SEARCH, 64>(a, s);
+  const int vec = row_vec(a);
+  if (nt == 128)
+    return vec == 4   ? launch_one<R, SEARCH, 128, 4>(a, s)
+           : vec == 2 ? launch_one<R, SEARCH, 128, 2>(a, s)
+                      : launch_one<R, SEARCH, 128, 1>(a, s);
+  return vec == 4   ? launch_one<R, SEARCH, 64, 4>(a, s)
+         : vec == 2 ? launch_one<R, SEARCH, 64, 2>(a, s)
+                    : launch_one<R, SEARCH, 64, 1>(a, s);
+}
+
+// Lists of up to 64 entries take the two passes (bounds per thread and queue
+// room by the size: the queue holds twice the entries and more); longer ones
+// would need bounds past a thread's registers and update their lists.
+template <bool SEARCH>
+int launch_lists(const KnnArgs& a, cudaStream_t s) {
+  constexpr int G = SEARCH ? 1 : 4;
+  if (a.size == 1) return launch_two_shape<1, 8, 64, SEARCH>(a, s);
+  if (a.size <= 24) return launch_two_shape<8, G, 96, SEARCH>(a, s);
+  if (a.size <= 40) return launch_two_shape<12, G, 128, SEARCH>(a, s);
+  if (a.size <= 64) return launch_two_shape<20, G, 160, SEARCH>(a, s);
+  if (a.size <= 128) return launch_one_shape<4, SEARCH>(a, s);
+  return launch_one_shape<8, SEARCH>(a, s);
 }
 
 }  // namespace
@@ -949,14 +1837,11 @@ int knn_tc_nearest(const KnnOperand& queries, const KnnOperand& cand, uint32_t d
   a.coff = coff;
   a.nc = (uint32_t)cand.n;
   a.replay = replay;
-  if (coff) BGPU_CUDA(cudaMemsetAsync(replay, 0, 4, s));
+  BGPU_CUDA(cudaMemsetAsync(replay, 0, 4, s));
   a.out_id = out_id;
   a.out_d = out_d;
   a.err = err;
-  if (count <= 32) return launch_shape<1, false>(a, s);
-  if (count <= 64) return launch_shape<2, false>(a, s);
-  if (count <= 128) return launch_shape<4, false>(a, s);
-  return launch_shape<8, false>(a, s);
+  return launch_lists<false>(a, s);
 }
 
 int knn_tc_search(const KnnOperand& cells, uint32_t d, const uint64_t* coff, uint32_t nc,
@@ -978,9 +1863,7 @@ int knn_tc_search(const KnnOperand& cells, uint32_t d, const uint64_t* coff, uin
   a.out_id = out_id;
   a.out_d = out_d;
   a.err = err;
-  if (k <= 32) return launch_shape<1, true>(a, s);
-  if (k <= 64) return launch_shape<2, true>(a, s);
-  return launch_shape<4, true>(a, s);
+  return launch_lists<true>(a, s);
 }
 
 }  // namespace bgpu

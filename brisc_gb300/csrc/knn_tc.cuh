@@ -29,8 +29,8 @@ int knn_prepare(KnnOperand* op, const float* rows, const float* norms, uint64_t 
 // For every query row, the `count` candidate rows with the smallest
 // |c|^2 - 2 x.c, sorted; ids are candidate rows. coff (may be nullptr): the
 // offsets of the queries' clusters where those are sorted by cluster and the
-// candidates are the clusters' centroids in order. replay: n + 1 words of
-// scratch, needed with coff. err: device error word.
+// candidates are the clusters' centroids in order; nullptr with count 1.
+// replay: n + 1 words of scratch. err: device error word.
 int knn_tc_nearest(const KnnOperand& queries, const KnnOperand& cand, uint32_t d, uint32_t count,
                    const uint64_t* coff, uint32_t* replay, uint32_t* out_id, float* out_d,
                    int* err, cudaStream_t s);
