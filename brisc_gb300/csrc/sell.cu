@@ -250,7 +250,11 @@ __device__ __forceinline__ void xt_sell_body(const XtView& X, const float* __res
     }
     __syncthreads();
     const uint32_t q1 = X.pgrp[p + 1];
-    for (uint32_t q = X.pgrp[p] + wid; q < q1; q += kSellWarps) {
+    // the groups come longest first: the warps take them forth and back
+    uint32_t turn = 0;
+    for (uint32_t qb = X.pgrp[p]; qb < q1; qb += kSellWarps, turn ^= 1u) {
+      const uint32_t q = qb + (turn ? kSellWarps - 1 - wid : wid);
+      if (q >= q1) continue;
       const uint32_t gene = X.gene[(uint64_t)q * 32 + lane];
       const uint2* src = X.data + X.grp[q] + lane;
       const uint32_t U = X.units[q];
