@@ -40,7 +40,16 @@
 // of two TMEM accumulators and commits them to that accumulator's mbarrier.
 // While they run, the next tile's loads are in flight and all 16 warps drain
 // the previous tile's accumulator (tcgen05.ld, 32 lanes x 8 columns per
-// load) and store C column-major (128-byte runs per column).
+// load) and store C column-major (128-byte runs per column). What bounds it is
+// the chain of a tile's phases (~10k cycles for 128 rows of 100 -> 75 columns:
+// a tile's loads are in flight for about half of it), so nothing in it waits
+// that need not: the pivot values are loaded together and take their sign when
+// they are added (each waited for its own load before), and the MMAs are issued
+// behind elect.sync from descriptors that only advance. 400k x 100 -> 75: 195 ->
+// 145 us, 1M: 422 -> 302 us per restart (floor 103). Loads of 32 rows of one
+// column instead of 8 rows of 4 (439), a warp of its own for the MMAs (459:
+// 544 threads leave 96 registers, too few for a tile) and the next tile's loads
+// ahead of the MMAs (331) were slower.
 //
 // Subspaces beyond one staging (K > 112: the 10M-cell solve's m = 200) run
 // in k_gemm_tc_pipe, which keeps B resident and streams A in K chunks of 16
@@ -210,7 +219,7 @@ k_gemm_tc(const float* __restrict__ A, uint64_t lda, uint64_t rows, uint32_t K,
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);  // two: one per accumulator
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + 64);
   __shared__ int stop;
-  __shared__ int spiv[kTcChunkN];  // pivot of each output column (0: none)
+  __shared__ uint32_t ssign[kTcChunkN];  // sign bit of each column's pivot
   __shared__ long long spoff[kTcChunkN];  // its source column's offset (-1: none)
   const TcLayout L(Kp, Np);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -231,7 +240,7 @@ k_gemm_tc(const float* __restrict__ A, uint64_t lda, uint64_t rows, uint32_t K,
   }
   for (uint32_t c = tid; c < kTcChunkN; c += kTcThreads) {
     const int pv = (piv && c < ncols) ? piv[c] : 0;
-    spiv[c] = pv;
+    ssign[c] = pv < 0 ? 0x80000000u : 0u;
     spoff[c] = pv == 0 ? -1ll : (long long)(pv > 0 ? pv - 1 : -pv - 1) * (long long)lda;
   }
   // B operand (N x K, K-major): row n of it is column n of Bm.
@@ -296,7 +305,7 @@ k_gemm_tc(const float* __restrict__ A, uint64_t lda, uint64_t rows, uint32_t K,
   // drains tile it - 1.
   const uint32_t q = wid & 3u, h = wid >> 2;
   const uint32_t quarter = Np / 4;  // columns per epilogue warp (<= 32)
-  float pa[32];                     // signed pivot values of this thread's row
+  float pa[32];                     // pivot values of this thread's row
   auto prefetch_pivots = [&](uint64_t row0) {
     const uint64_t gr = row0 + q * 32 + lane;
     const bool rok = gr < rows;
@@ -305,12 +314,7 @@ k_gemm_tc(const float* __restrict__ A, uint64_t lda, uint64_t rows, uint32_t K,
     for (int j = 0; j < 32; ++j) {
       const uint32_t c = h * quarter + j;  // < 128: spoff / spiv cover it
       const long long off = spoff[c];
-      float a = 0.f;
-      if ((uint32_t)j < quarter && off >= 0 && rok) {
-        a = ap[off];
-        if (spiv[c] < 0) a = -a;
-      }
-      pa[j] = a;
+      pa[j] = (uint32_t)j < quarter && off >= 0 && rok ? ap[off] : 0.f;
     }
   };
   // Epilogue: warp w reads TMEM lanes 32*(w%4).. (tile rows) and the columns
@@ -326,8 +330,9 @@ k_gemm_tc(const float* __restrict__ A, uint64_t lda, uint64_t rows, uint32_t K,
       tmem_ld8(acc + ((q * 32u) << 16) + c0, v);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        if (gr < rows && c0 + j < ncols) {
-          const float val = v[j] + pa[g8 * 8 + j];  // pivot column, FP32 add
+        if (gr < rows && c0 + j < ncols) {  // pivot column, FP32 add
+          const float val =
+              v[j] + __uint_as_float(__float_as_uint(pa[g8 * 8 + j]) ^ ssign[c0 + j]);
           *cp = accumulate ? *cp + val : val;  // K chunks add in order
         }
         cp += ldc;
@@ -367,30 +372,28 @@ k_gemm_tc(const float* __restrict__ A, uint64_t lda, uint64_t rows, uint32_t K,
       tc_fence_before();
       __syncthreads();
       const uint32_t acc = tmem + (it & 1u) * tmem_cols;
-      if (tid == 0) {
+      if (wid == 0 && elect_lane()) {
         tc_fence_after();
-        for (uint32_t ks = 0; ks < Kp / 16; ++ks) {
-          const uint32_t off = ks * 256u;  // two 16-byte K groups per K=16 step
-          uint64_t da[3], db[3];
+        uint64_t da[3], db[3];
 #pragma unroll
-          for (int part = 0; part < 3; ++part) {
-            da[part] = smem_desc(base + L.a[part] + off, 128u, sbo);
-            db[part] = smem_desc(base + L.b[part] + off, 128u, sbo);
-          }
+        for (int part = 0; part < 3; ++part) {
+          da[part] = smem_desc(base + L.a[part], 128u, sbo);
+          db[part] = smem_desc(base + L.b[part], 128u, sbo);
+        }
+        for (uint32_t ks = 0; ks < Kp / 16; ++ks) {
+          const uint32_t off = ks * 16u;  // two 16-byte K groups per K=16 step
           // the small cross products first: x1y3 + x2y2 + x3y1 + x1y2 + x2y1
-          mma_bf16(acc, da[0], db[2], idesc, ks > 0 ? 1u : 0u);
-          mma_bf16(acc, da[1], db[1], idesc, 1u);
-          mma_bf16(acc, da[2], db[0], idesc, 1u);
-          mma_bf16(acc, da[0], db[1], idesc, 1u);
-          mma_bf16(acc, da[1], db[0], idesc, 1u);
+          mma_bf16(acc, da[0] + off, db[2] + off, idesc, ks > 0 ? 1u : 0u);
+          mma_bf16(acc, da[1] + off, db[1] + off, idesc, 1u);
+          mma_bf16(acc, da[2] + off, db[0] + off, idesc, 1u);
+          mma_bf16(acc, da[0] + off, db[1] + off, idesc, 1u);
+          mma_bf16(acc, da[1] + off, db[0] + off, idesc, 1u);
         }
-        for (uint32_t ks = 0; ks < Kp / 16; ++ks) {  // then x1y1
-          const uint32_t off = ks * 256u;
-          mma_bf16(acc, smem_desc(base + L.a[0] + off, 128u, sbo),
-                   smem_desc(base + L.b[0] + off, 128u, sbo), idesc, 1u);
-        }
+        for (uint32_t ks = 0; ks < Kp / 16; ++ks)  // then x1y1
+          mma_bf16(acc, da[0] + ks * 16u, db[0] + ks * 16u, idesc, 1u);
         mma_commit(bars + (it & 1u));
       }
+      __syncwarp();
       pend = (int)(it & 1u);
       // the next tile's loads fly while these MMAs run
       if (tile + gridDim.x < ntiles) load_tile((tile + gridDim.x) * kTcRows);
