@@ -824,6 +824,69 @@ k_gemm_ts(const float* __restrict__ A, uint64_t lda, uint64_t rows, uint32_t K,
   }
 }
 
+// The same product for few rows (V's rotation, small U): 32 x 32 tiles, so that
+// 2000 rows reach 189 CTAs instead of 16, and 128 of K per step, so that a CTA
+// waits for memory once or twice instead of every 16 (2000 x 100 -> 75: 28.7 ->
+// 6.8 us, L2 cold). An element's sum runs over K in the same order.
+constexpr int SBM = 32, SBN = 32, SBK = 128;
+
+__global__ void __launch_bounds__(256)
+k_gemm_ts_small(const float* __restrict__ A, uint64_t lda, uint64_t rows, uint32_t K,
+                const float* __restrict__ Bp, uint64_t bsr, uint64_t bsc,
+                const float* __restrict__ cs, uint32_t ncols, float* __restrict__ C,
+                uint64_t ldc, int c_rowmajor) {
+  __shared__ __align__(16) float As[SBK][SBM];
+  __shared__ __align__(16) float Bs[SBK][SBN];
+  const int tid = threadIdx.x;
+  const int row = tid & 31, tx = tid >> 5;  // 4 columns per thread
+  const uint64_t r0 = (uint64_t)blockIdx.x * SBM;
+  const uint32_t c0 = blockIdx.y * SBN;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  for (uint32_t k0 = 0; k0 < K; k0 += SBK) {
+    const uint32_t kn = min(K - k0, (uint32_t)SBK);
+    float a[SBK / 8], b[SBK / 8];
+#pragma unroll
+    for (int t = 0; t < SBK / 8; ++t) {
+      const uint32_t kk = t * 8 + tx, c = c0 + row;
+      a[t] = kk < kn && r0 + row < rows ? A[(uint64_t)(k0 + kk) * lda + r0 + row] : 0.f;
+      // B: lanes along its contiguous direction
+      const uint32_t kb = bsr == 1 ? (uint32_t)(t % 4) * 32 + row : kk;
+      const uint32_t cb = bsr == 1 ? c0 + (uint32_t)(t / 4) * 8 + tx : c;
+      b[t] = 0.f;
+      if (kb < kn && cb < ncols) {
+        b[t] = Bp[(uint64_t)(k0 + kb) * bsr + (uint64_t)cb * bsc];
+        if (cs) b[t] *= cs[cb];
+      }
+    }
+    __syncthreads();  // the step before has been used
+#pragma unroll
+    for (int t = 0; t < SBK / 8; ++t) {
+      As[t * 8 + tx][row] = a[t];
+      if (bsr == 1) Bs[(t % 4) * 32 + row][(t / 4) * 8 + tx] = b[t];
+      else Bs[t * 8 + tx][row] = b[t];
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (uint32_t kk = 0; kk < kn; ++kk) {
+      const float x = As[kk][row];
+      const float4 y = *reinterpret_cast<const float4*>(&Bs[kk][tx * 4]);
+      acc[0] += x * y.x;
+      acc[1] += x * y.y;
+      acc[2] += x * y.z;
+      acc[3] += x * y.w;
+    }
+  }
+  const uint64_t r = r0 + row;
+  if (r >= rows) return;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t c = c0 + tx * 4 + j;
+    if (c >= ncols) continue;
+    if (c_rowmajor) C[r * ldc + c] = acc[j];
+    else C[r + (uint64_t)c * ldc] = acc[j];
+  }
+}
+
 __global__ void k_b_to_float(const double* __restrict__ B, uint64_t count,
                              float* __restrict__ Bf) {
   uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -998,6 +1061,14 @@ int launch_gemm_ts(const float* A, uint64_t lda, uint64_t rows, uint32_t K,
                    cudaStream_t s) {
   if (rows == 0 || ncols == 0) return BGPU_OK;
   dim3 grid((unsigned)ceil_div(rows, BM), (unsigned)ceil_div(ncols, BN));
+  // large tiles on fewer than a third of the SMs: small ones
+  if ((uint64_t)grid.x * grid.y * 3 < (uint64_t)num_sms()) {
+    grid = dim3((unsigned)ceil_div(rows, SBM), (unsigned)ceil_div(ncols, SBN));
+    k_gemm_ts_small<<<grid, 256, 0, s>>>(A, lda, rows, K, Bp, bsr, bsc, cs, ncols, C, ldc,
+                                         c_rowmajor ? 1 : 0);
+    BGPU_CHECK_LAUNCH();
+    return BGPU_OK;
+  }
   k_gemm_ts<<<grid, 256, 0, s>>>(A, lda, rows, K, Bp, bsr, bsc, cs, ncols, C,
                                  ldc, c_rowmajor ? 1 : 0);
   BGPU_CHECK_LAUNCH();

@@ -166,7 +166,7 @@ k_xv_sell_multi(const __grid_constant__ TaskList<XvTask> L) {
 // X^T.u (kMom = false) and the per-gene moments (kMom = true: u = 1, value
 // and squared value summed as float pairs per segment, then in FP64; the
 // moments of 28.5M entries at 300k x 2000: 303 us with FP64 sums per entry,
-// 77 us).
+// 75 us).
 template <bool kMom>
 struct XtAcc;
 template <>

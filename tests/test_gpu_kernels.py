@@ -254,6 +254,28 @@ def _rotate_both(cuda, A, Q, rows, K, ncols):
     return out, ref, scale
 
 
+@pytest.mark.parametrize("K,ncols", [(1, 1), (128, 33), (129, 32), (300, 100)])
+def test_few_rows_rotate_as_many_do(cuda, K, ncols):
+    """The FP32 GEMM's small tiles (few rows) give the bits of its large ones."""
+    import torch
+    rng = np.random.default_rng(K)
+    n = 20000
+    A = T(rng.standard_normal((K, n)).astype(np.float32).ravel(), cuda)
+    B = T(rng.standard_normal((K, K)).astype(np.float32).ravel(), cuda)
+
+    def rotate(rows):
+        C = torch.full((ncols, n), np.nan, dtype=torch.float32, device=cuda)
+        _lib.call("bgpu_rotate_basis", A.data_ptr(), n, rows, K, B.data_ptr(), K, ncols,
+                  C.data_ptr(), n, 1, None)
+        return C.cpu().numpy()
+
+    many = rotate(n)
+    for rows in (1, 31, 32, 33, 1000):
+        few = rotate(rows)
+        np.testing.assert_array_equal(few[:, :rows], many[:, :rows])
+        assert np.isnan(few[:, rows:]).all()
+
+
 @pytest.mark.parametrize("rows,K,ncols", [(20000, 100, 99), (20000, 100, 60),
                                           (8000, 200, 150), (5000, 64, 64)])
 def test_rotate_basis_ritz_rotation_unbiased(cuda, rows, K, ncols):
