@@ -387,15 +387,16 @@ __global__ void k_km_normalize(float* __restrict__ Cn, const uint32_t* __restric
 }
 
 // Squared distance of each cell to its assigned centroid, a dimension-ordered
-// float sum (relocate_empty_clusters, kmeans.pyx:785-791).
+// float sum (relocate_empty_clusters, kmeans.pyx:785-791); -1 for a cell without
+// a label, whose distances are all NaN.
 __global__ void k_km_assigned(const float* __restrict__ X, const uint32_t* __restrict__ lab,
                               const float* __restrict__ C, uint64_t n, uint32_t d,
                               uint32_t nc, float* __restrict__ out) {
   const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float* x = X + i * d;
-  if (lab[i] >= nc) {  // no label: its distances are NaN
-    out[i] = 0.f;
+  if (lab[i] >= nc) {
+    out[i] = -1.f;
     return;
   }
   const float* c = C + (uint64_t)lab[i] * d;
@@ -559,15 +560,21 @@ extern "C" int bgpu_kmeans(const float* X, uint32_t* cluster_labels, float* cent
         cudaFreeAsync(dist, s);
         BGPU_CUDA(cudaStreamSynchronize(s));
         // the num_empty largest distances, an earlier cell winning ties, in
-        // descending order
+        // descending order; cells without a label or a distance come last
+        // and are never taken
         const size_t ne = empty.size();
+        for (float& x : hd)
+          if (!(x >= 0.f)) x = -1.f;
         std::vector<uint64_t> order(n);
         for (uint64_t i = 0; i < n; ++i) order[i] = i;
         std::stable_sort(order.begin(), order.end(),
                          [&](uint64_t a, uint64_t b) { return hd[a] > hd[b]; });
-        BGPU_REQUIRE(hd[order[0]] != 0.f, BGPU_ERR_INVALID,
+        BGPU_REQUIRE(hd[order[0]] > 0.f, BGPU_ERR_INVALID,
                      "kmeans: num_clusters is greater than the number of cells with "
                      "distinct principal component loadings; decrease num_clusters");
+        BGPU_REQUIRE(hd[order[ne - 1]] >= 0.f, BGPU_ERR_INVALID,
+                     "kmeans: more empty clusters than cells whose distances are numbers; "
+                     "decrease num_clusters");
         std::vector<float> row(d);
         for (size_t e = 0; e < ne; ++e) {
           const uint64_t j = order[e];

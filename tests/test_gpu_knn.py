@@ -272,3 +272,46 @@ def _norm_chain(C):
     for j in range(1, C.shape[1]):
         cn = _fma(C[:, j], C[:, j], cn)
     return cn
+
+
+def _kmeans_of(X, nc, seed):
+    from brisc_gb300 import knn
+    n, d = X.shape
+    out = dict(cluster_labels=np.zeros(n, np.uint32), min_distances=np.zeros(n, np.float32),
+               cell_norms=np.zeros(0, np.float32), centroids=np.zeros((nc, d), np.float32),
+               centroids_new=np.zeros((nc, d), np.float32),
+               num_cells_per_cluster=np.zeros(nc, np.uint32))
+    assert knn.kmeans(X=X, chunk_size=n, num_kmeans_iterations=1, seed=seed, **out) == 1
+    return out
+
+
+def _nan_and_equal_cells(nan, equal, seed_of):
+    """`nan` cells of NaN first, then `equal` equal cells, then one far away, and a
+    seed whose random initial centroids leave that one out."""
+    from oracle import clib
+    n = nan + equal + 1
+    X = np.full((n, 3), np.nan, np.float32)
+    X[nan:] = 1.0
+    X[-1] = 50.0
+    seed = next(s for s in range(10_000) if n - 1 not in clib.kmeans_init(n, seed_of, s))
+    return X, seed
+
+
+def test_kmeans_relocation_never_takes_an_unlabelled_cell(cuda):
+    """61 empty clusters, one cell at a positive distance and 60 at zero: the
+    clusters take those 61, never one of the NaN cells in front of them, which
+    have no label."""
+    X, seed = _nan_and_equal_cells(3, 60, 62)
+    out = _kmeans_of(X, 62, seed)
+    assert (out["cluster_labels"][:3] == 0xFFFFFFFF).all()
+    assert (out["cluster_labels"][3:] < 62).all()
+    assert out["num_cells_per_cluster"].sum() == 61
+    assert np.isfinite(out["centroids_new"]).all()
+    np.testing.assert_array_equal(out["centroids_new"][out["cluster_labels"][-1]], X[-1])
+
+
+def test_kmeans_refuses_more_empty_clusters_than_labelled_cells(cuda):
+    """59 empty clusters, 34 cells with a label."""
+    X, seed = _nan_and_equal_cells(30, 33, 60)
+    with pytest.raises(ValueError, match="more empty clusters than cells"):
+        _kmeans_of(X, 60, seed)
