@@ -39,7 +39,6 @@ constexpr uint32_t kMaxDims = 128;
 constexpr uint32_t kMaxSearched = 256;
 constexpr uint32_t kMaxNeighbors = 128;
 constexpr uint32_t kMaxClusters = 32768;
-enum KnnErr : int { kKnnErrSizes = 2 };  // beside kDevErrTimeout of the waits
 
 __global__ void k_knn_centroid_norms(const float* __restrict__ C, uint32_t nc,
                                      uint32_t d, float* __restrict__ cn) {
@@ -53,8 +52,8 @@ __global__ void k_knn_centroid_norms(const float* __restrict__ C, uint32_t nc,
 
 // Cluster offsets (exclusive prefix sum of the sizes) and their total, by one
 // block: a run of clusters per thread, then a scan of the runs (2,191 clusters:
-// 57 us for one thread, 5 us). Sizes that do not sum to n set err and leave
-// every cluster empty.
+// 57 us for one thread, 5 us). Sizes that do not sum to n set err, behind which
+// the searches write nothing.
 constexpr int kOffThreads = 1024;
 __global__ void __launch_bounds__(kOffThreads)
 k_knn_offsets(const uint32_t* __restrict__ sizes, uint32_t nc, uint64_t n,

@@ -6,6 +6,11 @@
 
 namespace bgpu {
 
+// Error word of a call, beside kDevErrTimeout of the waits: the cluster sizes do
+// not sum to the number of cells. The kernels below write no result where it is
+// set, so a refused call leaves its outputs as they were.
+enum KnnErr : int { kKnnErrSizes = 2 };
+
 // A matrix of row vectors prepared as a tensor-core operand (knn_tc.cu): BF16
 // high and low parts in core-matrix order, 8 rows at a time, with the row's
 // norm in extra columns.

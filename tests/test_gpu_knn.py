@@ -315,3 +315,30 @@ def test_kmeans_refuses_more_empty_clusters_than_labelled_cells(cuda):
     X, seed = _nan_and_equal_cells(30, 33, 60)
     with pytest.raises(ValueError, match="more empty clusters than cells"):
         _kmeans_of(X, 60, seed)
+
+
+def _refused_call(cuda, n, d, nc, k, cs, offset):
+    """knn_self with a cluster one cell short; the outputs, filled with 7."""
+    import torch
+    from brisc_gb300 import knn
+    gen = torch.Generator(device=cuda).manual_seed(1)
+    X = torch.randn(n, d, generator=gen, device=cuda) + offset
+    sizes = torch.full((nc,), n // nc, dtype=torch.int32, device=cuda)
+    sizes[3] -= 1
+    out = dict(neighbors=torch.full((n, k), 7, dtype=torch.int32, device=cuda),
+               distances=torch.full((n, k), 7.0, device=cuda),
+               nearest_clusters=torch.full((n, cs), 7, dtype=torch.int32, device=cuda),
+               centroid_distances=torch.full((n, cs), 7.0, device=cuda))
+    with pytest.raises(ValueError, match="does not sum to the number of cells"):
+        knn.knn_self(X=X, sorted_order=torch.arange(n, dtype=torch.int32, device=cuda),
+                     centroids=X[:nc].contiguous(), num_cells_per_cluster=sizes,
+                     cell_norms=(X * X).sum(1), num_neighbors=k, num_clusters_searched=cs, **out)
+    return out
+
+
+@pytest.mark.parametrize("k,cs", [(5, 4), (70, 70)])
+def test_knn_self_refusal_leaves_the_outputs(cuda, k, cs):
+    """Cluster sizes that do not sum to the number of cells: refused, and
+    nothing is written (lists on both sides of 64 entries)."""
+    for name, t in _refused_call(cuda, 400, 6, 80, k, cs, 0.0).items():
+        assert (t == 7).all(), name
