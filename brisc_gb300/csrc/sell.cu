@@ -164,9 +164,9 @@ k_xv_sell_multi(const __grid_constant__ TaskList<XvTask> L) {
 
 // ---------------------------------------------------------------------------
 // X^T.u (kMom = false) and the per-gene moments (kMom = true: u = 1, value
-// and squared value summed as float pairs per segment, then in FP64; the
-// moments of 28.5M entries at 300k x 2000: 303 us with FP64 sums per entry,
-// 75 us).
+// and squared value summed in floats per segment (moments.cuh), then in FP64;
+// the moments of 28.5M entries at 300k x 2000: 303 us with FP64 sums per entry,
+// 74 us).
 template <bool kMom>
 struct XtAcc;
 template <>
@@ -175,7 +175,8 @@ struct XtAcc<false> {
   __device__ __forceinline__ void add(float v) { s += v; }
 };
 template <>
-struct XtAcc<true> : PairMoments {};
+struct XtAcc<true> : FloatMoments {};  // a segment has at most kXtMaxP terms
+static_assert(kXtMaxP <= kMomentTerms, "the moments of one segment are one run");
 
 __host__ __device__ inline uint32_t xt_esc_floats(uint32_t esc_max) {
   return (esc_max + 3u) & ~3u;
@@ -280,7 +281,7 @@ __device__ __forceinline__ void xt_sell_body(const XtView& X, const float* __res
       if (gene != kNoGene) {  // one segment per gene and panel: no collisions
         if constexpr (kMom) {
           double s = acc.sum(), q = acc.squares();
-          if (!acc.good()) {  // out of the pairs' range: the segment again, in FP64
+          if (!acc.good()) {  // out of the floats' range: the segment again, in FP64
             s = q = 0.0;
             for (uint32_t k = 0; k < U; ++k) {
               const uint2 a = ld_stream_u2(src + (uint64_t)k * 32);

@@ -181,8 +181,8 @@ k_rmat_partials(CscView X, const float* __restrict__ u,
   }
 }
 
-// Per (panel, gene): sum and sum of squares of the values, as float pairs per
-// lane (moments.cuh), the lanes added in FP64.
+// Per (panel, gene): sum and sum of squares of the values, per lane in runs of
+// up to kMomentTerms floats (moments.cuh), the runs and the lanes in FP64.
 template <int MODE, int G>
 __global__ void __launch_bounds__(256)
 k_gene_moments(CscView X, double2* __restrict__ partials, uint32_t colgroup) {
@@ -240,26 +240,32 @@ k_gene_moments(CscView X, double2* __restrict__ partials, uint32_t colgroup) {
         }
       }
     };
-    PairMoments m;
-    for (int64_t b = (e0 & ~3LL) + 4 * seg.lane; b < e1; b += 4 * G * kSegLoads) {
-      float vals[kSegLoads][4];
+    constexpr int64_t kStep = 4 * G * kSegLoads, kRun = kStep * (kMomentTerms / (4 * kSegLoads));
+    double s1 = 0.0, s2 = 0.0;
+    for (int64_t run = (e0 & ~3LL) + 4 * seg.lane; run < e1; run += kRun) {
+      const int64_t end = run + kRun < e1 ? run + kRun : e1;
+      FloatMoments m;
+      for (int64_t b = run; b < end; b += kStep) {
+        float vals[kSegLoads][4];
 #pragma unroll
-      for (int i = 0; i < kSegLoads; ++i) values(b + 4 * G * i, vals[i]);
+        for (int i = 0; i < kSegLoads; ++i) values(b + 4 * G * i, vals[i]);
 #pragma unroll
-      for (int i = 0; i < kSegLoads; ++i)
+        for (int i = 0; i < kSegLoads; ++i)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) m.add(vals[i][k]);
-    }
-    double s1 = m.sum(), s2 = m.squares();
-    if (!m.good()) {  // out of the pairs' range (or no entry): again, in FP64
-      s1 = s2 = 0.0;
-      for (int64_t b = (e0 & ~3LL) + 4 * seg.lane; b < e1; b += 4 * G) {
-        float vals[4];
-        values(b, vals);
+          for (int k = 0; k < 4; ++k) m.add(vals[i][k]);
+      }
+      if (m.good()) {
+        s1 += m.sum();
+        s2 += m.squares();
+      } else {  // out of the floats' range (or no entry): again, in FP64
+        for (int64_t b = run; b < end; b += 4 * G) {
+          float vals[4];
+          values(b, vals);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          s1 += (double)vals[k];
-          s2 += (double)vals[k] * (double)vals[k];
+          for (int k = 0; k < 4; ++k) {
+            s1 += (double)vals[k];
+            s2 += (double)vals[k] * (double)vals[k];
+          }
         }
       }
     }

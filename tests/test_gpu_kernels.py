@@ -361,6 +361,60 @@ def test_gene_stddev_of_any_scale(cuda, n, g, density, scale):
     np.testing.assert_allclose(sd.cpu().numpy(), want.astype(np.float32), rtol=1e-6)
 
 
+def _values_of_gene(M, j, n, g, cuda):
+    """The stored values of gene j as the kernels form them: X.e_j is the
+    product of each with 1, exactly."""
+    import torch
+    e = torch.zeros(g, device=cuda)
+    e[j] = 1.0
+    y = torch.empty(n, device=cuda)
+    M.matvec(e, torch.ones(g, device=cuda), y)
+    return y.cpu().numpy().astype(np.longdouble)
+
+
+@pytest.mark.parametrize("form,n,g,density,panel_rows", [
+    ("sell", 30000, 40, 0.1, 0), ("panels", 30000, 40, 0.1, 0), ("float", 30000, 40, 0.1, 0),
+    ("float", 100_000, 1500, 0.002, 16384)])
+def test_gene_stddev_of_a_mean_far_above_the_spread(cuda, form, n, g, density, panel_rows):
+    """Genes expressed in every cell at nearly one value (8.9 to 10, spread
+    0.001). n s2 - s1^2 loses
+    (mean / sd)^2 of the sums' precision; sums in FP64, of fewer than 64 rounded
+    additions each on the way of any entry, leave at most 64 2^-53 of that, and
+    the float result its own rounding. The others are ordinary genes (16384-row
+    panels with few entries elsewhere put 2048 terms of a dense gene on one
+    lane)."""
+    import torch
+    rng = np.random.default_rng(n)
+    X = sp.random(n, g, density, "coo", dtype=np.float32, random_state=rng,
+                  data_rvs=lambda k: rng.integers(1, 9, k))
+    dense = {3: 3.0, 17: 5.0, 39: 9.0}
+    other = ~np.isin(X.col, list(dense))
+    X = sp.csr_matrix(
+        (np.concatenate([X.data[other], np.repeat(np.float32(list(dense.values())), n)]),
+         (np.concatenate([X.row[other], np.tile(np.arange(n), 3)]),
+          np.concatenate([X.col[other], np.repeat(list(dense), n)]))), shape=(n, g))
+    X.sort_indices()
+    isf = (2500 * np.exp(1e-3 * rng.standard_normal(n))).astype(np.float32)
+    kw = dict(norm="logCP10k", inv_size_factors=isf, sell_panel_rows=512)
+    if form == "float":
+        rows = np.repeat(np.arange(n), np.diff(X.indptr))
+        X.data = np.log1p(X.data * isf[rows]).astype(np.float32)
+        kw = {}
+    M = DeviceMatrix(X.indptr.astype(np.int64), X.indices.astype(np.int64),
+                     X.data if form == "float" else X.data.astype(np.uint16), n, g,
+                     panel_rows=panel_rows, kernels=("panels",) if form == "panels" else (), **kw)
+    sd = torch.empty(g, dtype=torch.float32, device=cuda)
+    M.gene_stddev(sd)
+    sd = sd.cpu().numpy()
+    for j in list(dense) + [0, 20]:
+        v = _values_of_gene(M, j, n, g, cuda)
+        mean = v.mean()
+        want = np.sqrt(((v - mean) ** 2).sum() / (n - 1))
+        tol = 2.0**-24 + 64 * 2.0**-53 * (1 + (mean / want) ** 2)
+        assert abs(sd[j] - want) <= tol * want, (j, float(sd[j]), float(want), float(tol))
+    M.close()
+
+
 @pytest.mark.parametrize("itype", [np.int32, np.int64])
 @pytest.mark.parametrize("n,g", [(1, 1), (63, 31), (64, 33), (65, 6144), (40000, 37), (3000, 6145),
                                  (20000, 2000)])
