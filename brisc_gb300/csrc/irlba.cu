@@ -1182,11 +1182,15 @@ extern "C" void bgpu_solve_opts_default(bgpu_solve_opts* o) {
 
 static void choose_shapes(Matrix& m) {
   const double avg = m.n ? (double)m.nnz / (double)m.n : 0.0;
+  // Lanes per row of k_spmv, one to two 4-entry loads per lane; between 128 and
+  // 256 entries two to four, since 32 lanes leave a warp waiting on its row
+  // alone. 12M floats, us per call with the lanes of the rule and with half or
+  // twice as many: 53 entries per row 41.5 (8 lanes; 4: 45.2), 110: 39.6 (16; 8:
+  // 42.4), 159: 40.5 (16; 32: 43.8), 248: 39.2 (16; 32: 43.2). Past 256, 32 lanes
+  // keep the order of those rows' sums (348: 50.4; 16: 44.4; 494: 47.4; 16: 47.7).
   int G = 4;
-  // two to four 4-entry loads per lane, all in flight: with fewer, a warp
-  // waits on its row alone (50k x 2000 floats, 150 entries per row: 24.8 us
-  // with 32 lanes per row, 21.2 us with 16)
-  while (G < 32 && G * 16 < avg) G *= 2;
+  while (G < 16 && G * 8 < avg) G *= 2;
+  if (avg > 256.0) G = 32;
   m.spmv_group = G;
   m.spmv_blocks = num_sms() * 8;
   // genes per CTA of the panel products: fewer where the panels alone do not

@@ -361,6 +361,38 @@ def test_gene_stddev_of_any_scale(cuda, n, g, density, scale):
     np.testing.assert_allclose(sd.cpu().numpy(), want.astype(np.float32), rtol=1e-6)
 
 
+@pytest.mark.parametrize("per,lanes", [(30, 4), (32, 4), (33, 8), (64, 8), (65, 16), (100, 16),
+                                       (256, 16), (257, 32), (400, 32)])
+def test_float_matvec_lanes_per_row(cuda, per, lanes):
+    """X.v of float values, bit for bit: a row's lanes take its entries four at
+    a time (from 4-entry boundaries of the matrix), each a chain of fused
+    multiply-adds, and are added by a fixed tree; how many lanes depends on the
+    mean entries per row."""
+    import torch
+    n, g = 67, 900
+    rng = np.random.default_rng(per)
+    ix = np.concatenate([np.sort(rng.choice(g, per, replace=False)) for _ in range(n)])
+    ip = np.arange(n + 1) * per
+    x = rng.standard_normal(n * per).astype(np.float32)
+    v = rng.standard_normal(g).astype(np.float32)
+    M = DeviceMatrix(ip.astype(np.int64), ix.astype(np.int64), x, n, g)
+    y = torch.empty(n, device=cuda)
+    M.matvec(T(v, cuda), torch.ones(g, device=cuda), y)
+    M.close()
+    e = np.arange(n * per)
+    lane = (e // 4 - np.repeat(ip[:-1] // 4, per)) % lanes
+    acc = np.zeros((n, lanes), np.float32)
+    p = x.astype(np.longdouble) * v[ix]
+    for i in range(per):  # every row's i-th entry: exact products, one rounding
+        at = (np.arange(n), lane[ip[:-1] + i])
+        acc[at] = (acc[at] + p[ip[:-1] + i]).astype(np.float32)
+    o = lanes // 2
+    while o:
+        acc = acc + acc[:, np.arange(lanes) ^ o]
+        o //= 2
+    np.testing.assert_array_equal(y.cpu().numpy(), acc[:, 0])
+
+
 def _values_of_gene(M, j, n, g, cuda):
     """The stored values of gene j as the kernels form them: X.e_j is the
     product of each with 1, exactly."""
