@@ -67,13 +67,17 @@ int num_sms();                 // queried once per device
 // synchronisation, and every call ends in one, so each call mapped its
 // workspaces anew: 45 us per small call (the three products of a 50k x 2000
 // matrix: 121 us of kernels in 300 us, 168 us in all with the pool). This one keeps up to
-// kScratchKept bytes mapped; anything above goes back at the next
-// synchronisation, and all of it when an allocation fails. Resident matrices
-// stay in the default pool. A block freed on one stream is handed to another
-// only once that stream's work has passed it (never by a hidden wait), so
-// solves on several streams do not serialise.
+// kScratchKept bytes mapped for the life of the process; anything above goes
+// back at the next synchronisation, and all of it when one of the library's own
+// allocations (scratch or resident) fails. Other allocators of the process cannot
+// take it back: they have that much less. A block freed on one stream is handed
+// to another only once that stream's work has passed it (never by a hidden wait),
+// so solves on several streams do not serialise.
 constexpr uint64_t kScratchKept = 1ull << 30;
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
+// Stream-ordered memory that outlives the call (resident matrices), from the
+// device's default pool.
+cudaError_t resident_alloc(void** p, size_t bytes, cudaStream_t s);
 
 // Lets `fn` use up to the device's opt-in shared memory per block. The limit
 // is a per-function setting shared by every host thread: setting it to one

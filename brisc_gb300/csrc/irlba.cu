@@ -69,44 +69,67 @@ int device_smem_optin() {
   return cache[dev];
 }
 
-cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
+namespace {
+
+// The scratch pool of the current device, made at its first use.
+cudaError_t scratch_pool(cudaMemPool_t* out) {
   static std::mutex mu;
   static std::vector<cudaMemPool_t> pools;  // per device, for the process
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  cudaMemPool_t pool = nullptr;
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    if ((int)pools.size() <= dev) pools.resize(dev + 1, nullptr);
-    if (!pools[dev]) {
-      cudaMemPoolProps props{};
-      props.allocType = cudaMemAllocationTypePinned;
-      props.location.type = cudaMemLocationTypeDevice;
-      props.location.id = dev;
-      cudaMemPool_t made = nullptr;
-      e = cudaMemPoolCreate(&made, &props);
-      if (e != cudaSuccess) return e;
-      uint64_t kept = kScratchKept;
-      int off = 0;
-      e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &kept);
-      if (e == cudaSuccess)
-        e = cudaMemPoolSetAttribute(made, cudaMemPoolReuseAllowInternalDependencies, &off);
-      if (e != cudaSuccess) {
-        cudaMemPoolDestroy(made);
-        return e;
-      }
-      pools[dev] = made;
+  std::lock_guard<std::mutex> lk(mu);
+  if ((int)pools.size() <= dev) pools.resize(dev + 1, nullptr);
+  if (!pools[dev]) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t made = nullptr;
+    e = cudaMemPoolCreate(&made, &props);
+    if (e != cudaSuccess) return e;
+    uint64_t kept = kScratchKept;
+    int off = 0;
+    e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &kept);
+    if (e == cudaSuccess)
+      e = cudaMemPoolSetAttribute(made, cudaMemPoolReuseAllowInternalDependencies, &off);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(made);
+      return e;
     }
-    pool = pools[dev];
+    pools[dev] = made;
   }
-  e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+  *out = pools[dev];
+  return cudaSuccess;
+}
+
+// alloc(pool), and where memory is short once more after the pool has given back
+// what it keeps, which may be what is missing. A failure is returned, not left
+// behind for the next launch check.
+template <typename F>
+cudaError_t alloc_or_trim(cudaStream_t s, F alloc) {
+  cudaMemPool_t pool = nullptr;
+  cudaError_t e = scratch_pool(&pool);
+  if (e != cudaSuccess) return e;
+  e = alloc(pool);
   if (e != cudaErrorMemoryAllocation) return e;
-  // what the pool keeps may be what is missing: give it back and try again
   (void)cudaGetLastError();
   cudaStreamSynchronize(s);
   cudaMemPoolTrimTo(pool, 0);
-  return cudaMallocFromPoolAsync(p, bytes, pool, s);
+  e = alloc(pool);
+  if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError();
+  return e;
+}
+
+}  // namespace
+
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
+  return alloc_or_trim(
+      s, [&](cudaMemPool_t pool) { return cudaMallocFromPoolAsync(p, bytes, pool, s); });
+}
+
+cudaError_t resident_alloc(void** p, size_t bytes, cudaStream_t s) {
+  return alloc_or_trim(s, [&](cudaMemPool_t) { return cudaMallocAsync(p, bytes, s); });
 }
 
 // ---------------------------------------------------------------------------

@@ -48,7 +48,7 @@ struct DevBuf {
 template <typename T>
 int dev_alloc(T** out, size_t count, uint64_t* bytes_acc, cudaStream_t s) {
   size_t b = std::max<size_t>(count * sizeof(T), 16);
-  cudaError_t e = cudaMallocAsync((void**)out, b, s);
+  cudaError_t e = resident_alloc((void**)out, b, s);
   if (e != cudaSuccess) {
     *out = nullptr;
     set_error(std::string("cudaMalloc(") + std::to_string(b) +

@@ -653,7 +653,7 @@ int build_sell(Matrix* m, cudaStream_t s, bool* built) {
   } tmp{{}, s};
   int ntmp = 0;
   auto raw_alloc = [&](void** p, size_t b) -> int {
-    cudaError_t e = cudaMallocAsync(p, std::max<size_t>(b, 16), s);
+    cudaError_t e = resident_alloc(p, std::max<size_t>(b, 16), s);
     if (e != cudaSuccess) {
       *p = nullptr;
       set_error(std::string("cudaMalloc(") + std::to_string(b) + ") failed: " +

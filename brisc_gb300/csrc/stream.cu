@@ -700,7 +700,7 @@ int build_row_order(Matrix* m, cudaStream_t s, uint64_t* bytes_acc) {
   for (auto& c : cnt) { const uint64_t t = c; c = run; run += t; }
   std::vector<int32_t> order(m->n);
   for (uint64_t r = 0; r < m->n; ++r) order[cnt[key[r]]++] = (int32_t)r;
-  BGPU_CUDA(cudaMallocAsync((void**)&m->row_order, m->n * 4, s));
+  BGPU_CUDA(resident_alloc((void**)&m->row_order, m->n * 4, s));
   *bytes_acc += m->n * 4;
   BGPU_CUDA(cudaMemcpyAsync(m->row_order, order.data(), m->n * 4, cudaMemcpyHostToDevice, s));
   BGPU_CUDA(cudaStreamSynchronize(s));  // `order` is a host temporary
@@ -718,8 +718,8 @@ int build_stream_tiles(Matrix* m, const std::vector<int64_t>& panel_rowptr,
   if (!stream_supported(*m)) return BGPU_OK;
   const uint64_t nr = m->n * kCountTab;
   const uint64_t nc = (uint64_t)m->num_panels * kCountTab * m->P;
-  BGPU_CUDA(cudaMallocAsync((void**)&m->rtab_r, nr * 4, s));
-  BGPU_CUDA(cudaMallocAsync((void**)&m->rtab_c, nc * 4, s));
+  BGPU_CUDA(resident_alloc((void**)&m->rtab_r, nr * 4, s));
+  BGPU_CUDA(resident_alloc((void**)&m->rtab_c, nc * 4, s));
   *bytes_acc += (nr + nc) * 4;
   BGPU_CUDA(cudaMemsetAsync(m->rtab_c, 0, nc * 4, s));
   k_count_tables<<<(unsigned)ceil_div(nr, 256), 256, 0, s>>>(

@@ -273,7 +273,7 @@ bool compact16_supported(const Matrix& m) {
 int build_compact16(Matrix* m, cudaStream_t s, uint64_t* bytes_acc) {
   if (!compact16_supported(*m)) return BGPU_OK;
   const uint64_t n16 = round_up(m->nnz, 16) + 32;
-  BGPU_CUDA(cudaMallocAsync((void**)&m->csc16, n16 * 2, s));
+  BGPU_CUDA(resident_alloc((void**)&m->csc16, n16 * 2, s));
   *bytes_acc += n16 * 2;
   BGPU_CUDA(cudaMemsetAsync(m->csc16, 0, n16 * 2, s));
   if (m->nnz) {

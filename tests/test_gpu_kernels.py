@@ -499,3 +499,27 @@ def test_row_sums_of_large_values(cuda, vtype):
               0, None, isf.data_ptr(), None, rs.data_ptr(), None)
     want = [int(v[a:b].astype(np.int64).sum()) for a, b in zip(ip[:-1], ip[1:])]
     assert rs.cpu().tolist() == want
+
+
+def test_a_failed_matrix_takes_back_the_scratch_memory(cuda):
+    """What the workspace pool keeps goes back to the device when a matrix's
+    memory is refused (asked here for row offsets of half a terabyte, before any
+    entry is read), as when a workspace's is."""
+    import torch
+    n, g = 1_000_000, 2000
+    ip = torch.arange(n + 1, dtype=torch.int32, device=cuda)
+    ix = torch.zeros(n, dtype=torch.int32, device=cuda)
+    bp, bi, bx = torch.empty(g + 1, dtype=torch.int32, device=cuda), ix.clone(), ix.clone()
+    torch.cuda.synchronize()
+    _lib.call("bgpu_csr_tocsc", n, g, ip.data_ptr(), ix.data_ptr(), ix.data_ptr(),
+              _lib.INDEX_I32, bp.data_ptr(), bi.data_ptr(), bx.data_ptr(), None)
+    kept = torch.cuda.mem_get_info()[0]
+    d = _lib.MatrixDesc()
+    d.indptr, d.indices, d.values = ip.data_ptr(), ix.data_ptr(), bx.data_ptr()
+    d.index_type, d.value_type, d.on_device = _lib.INDEX_I32, _lib.VALUE_F32, 1
+    d.num_cells, d.num_genes, d.nnz, d.norm_method = 1 << 36, g, n, _lib.NORM_NONE
+    h = C.c_void_p()
+    with pytest.raises(_lib.BriscGPUError, match="failed"):
+        _lib.call("bgpu_matrix_create", C.byref(h), C.byref(d), None)
+    # most of the transpose's counters, 4 bytes per column and 64 rows
+    assert torch.cuda.mem_get_info()[0] - kept >= n // 64 * g * 2
