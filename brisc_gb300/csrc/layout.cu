@@ -1080,8 +1080,11 @@ __global__ void k_store_bp(const long long* __restrict__ cp, I* __restrict__ Bp,
 // 128 rows 551, with 64 rows 330 (200k x 2000, 19M entries). One warp per 256
 // rows with global counters, and one CTA to scan them, took 2.05 ms in all, this
 // 0.40 ms. More columns than fit take that path.
+// The counters are 4 bytes per column and sub-block: 1.25 GB for 10M x 2000.
+// Where the device has no room for them, sub-blocks of 128 rows or more take
+// their place (0.63 GB, what the other path takes).
 constexpr uint32_t kTrGenes = 6144;
-constexpr uint64_t kTrRows = 64;
+constexpr uint64_t kTrRows = 64, kTrMaxRows = 512;
 constexpr int kTrThreads = 256;
 constexpr int kTrWarps = kTrThreads / 32;
 constexpr int kTrLoads = 4;
@@ -1220,10 +1223,14 @@ int csr_tocsc_typed(uint64_t n, uint32_t g, const void* Ap, const void* Aj,
   long long* cp = (long long*)t_cp.p;
   if (g <= kTrGenes) {
     const size_t smem = (size_t)kTrWarps * g * 4;
-    const uint64_t rows_per = kTrRows;
+    uint64_t rows_per = kTrRows;
+    int got;
+    while ((got = t_cnt.alloc(ceil_div(n, rows_per) * g * 4, s)) != BGPU_OK &&
+           rows_per < kTrMaxRows)
+      rows_per *= 2;
+    BGPU_TRY(got);
     const uint32_t num_sub = (uint32_t)ceil_div(n, rows_per);
     DevBuf t_tot;
-    BGPU_TRY(t_cnt.alloc((size_t)num_sub * g * 4, s));
     BGPU_TRY(t_tot.alloc((size_t)g * 8, s));
     uint32_t* cnt = (uint32_t*)t_cnt.p;
     BGPU_CUDA((allow_max_smem(k_tr_scatter<I>)));
