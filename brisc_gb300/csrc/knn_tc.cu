@@ -1802,8 +1802,10 @@ int launch_lists(const KnnArgs& a, cudaStream_t s) {
   if (a.size <= 24) return launch_two_shape<8, G, 96, SEARCH>(a, s);
   if (a.size <= 40) return launch_two_shape<12, G, 128, SEARCH>(a, s);
   if (a.size <= 64) return launch_two_shape<20, G, 160, SEARCH>(a, s);
-  if (a.size <= 128) return launch_one_shape<4, SEARCH>(a, s);
-  return launch_one_shape<8, SEARCH>(a, s);
+  if constexpr (SEARCH)  // at most 128 neighbours
+    return launch_one_shape<4, SEARCH>(a, s);
+  else
+    return a.size <= 128 ? launch_one_shape<4, SEARCH>(a, s) : launch_one_shape<8, SEARCH>(a, s);
 }
 
 }  // namespace
