@@ -155,7 +155,7 @@ extern "C" int bgpu_knn_self(const float* X, const uint32_t* sorted_order,
   const size_t cb = round_up(knn_operand_bytes(nc, d), 256);
   const size_t nb = round_up((size_t)nc * 4, 256), ob = round_up(((size_t)nc + 1) * 8, 256);
   unsigned char* mem = nullptr;
-  const size_t rb = round_up((n + 1) * 4, 256);
+  const size_t rb = round_up(knn_replay_bytes(n), 256);
   BGPU_CUDA(scratch_alloc((void**)&mem, xb + cb + nb + ob + rb + 256, s));
   float* cn = (float*)(mem + xb + cb);
   uint64_t* coff = (uint64_t*)(mem + xb + cb + nb);
@@ -491,7 +491,7 @@ extern "C" int bgpu_kmeans(const float* X, uint32_t* cluster_labels, float* cent
   BGPU_CUDA(scratch_alloc((void**)&didx, (size_t)nc * 4, s));
   BGPU_CUDA(scratch_alloc((void**)&cn, (size_t)nc * 4, s));
   BGPU_CUDA(scratch_alloc((void**)&sums, sums_bytes, s));
-  const size_t rb = round_up((n + 1) * 4, 256);
+  const size_t rb = round_up(knn_replay_bytes(n), 256);
   BGPU_CUDA(scratch_alloc((void**)&mem, xb + cb + rb + 256, s));
   uint32_t* replay = (uint32_t*)(mem + xb + cb);
   int* err = (int*)(mem + xb + cb + rb);

@@ -26,7 +26,9 @@
 // hold them is too, unless the k-th and the (k+1)-th distance are equal.
 // So each query also keeps the smallest value that its list turned away or
 // gave up, and where that equals the list's worst, the query is listed and
-// k_knn_replay computes it again, every candidate in the reference's order.
+// computed again, every candidate in the reference's order: by k_knn_replay, or
+// by k_knn_all where many of 32 neighbouring queries are. So are queries on which
+// the filter decides nothing.
 //
 // Error of s against the exact x.c - |c|^2/2, with X = the query's length and
 // G = the largest length or sqrt |norm| of the tile: the dropped low.low and
@@ -44,8 +46,8 @@
 // 300k x 50 dims, 2,191 clusters, 64 searched, 20 neighbours: search 36.7 ->
 // 6.9 ms, nearest clusters 20.9 -> 2.5 ms, the E step against 2,191 centroids
 // 6.07 -> 0.57 ms. Lists of up to 64 entries take k_knn_two; longer ones
-// k_knn_tc, which keeps its lists while it goes (15.1, 10.6 and 1.52 ms; a
-// tile waits for the exact evaluations of its slowest warp).
+// k_knn_tc, which keeps its lists while it goes (the same lists 15.1 and 10.6 ms;
+// a tile waits for the exact evaluations of its slowest warp).
 //
 // Shape of k_knn_tc: 512 threads, one CTA per SM, kQT queries (rows of the MMA), tiles of
 // NT candidates. Warp w reads the TMEM lanes (queries) of quarter w % 4 and
@@ -77,6 +79,15 @@ constexpr uint32_t kUnionCap = 512;   // searched clusters taken at once
 constexpr uint32_t kNormCols = 3;
 constexpr float kMargin = 1.f / 8192.f;
 constexpr uint32_t kNoRun = 0xFFFFFFFFu;
+// Queries of a group of 32 from which on k_knn_all takes them: 300k x 50 dims, a
+// group costs 2.9 us of the GPU's time, a query by itself 0.33.
+constexpr int kGroupReplays = 8;
+// Exact evaluations per list entry past which k_knn_tc gives its queries up.
+// Ordinary data stay below 16. 300k x 50 dims, against the exhaustive search
+// alone: search of 100 neighbours, rows 10 spreads from the origin, 109 ms with
+// 16, 89 with 24 (112); 100 nearest clusters, 100 spreads, 95 with 16, 109 with 24
+// (97).
+constexpr uint32_t kSearchEvals = 24, kNearestEvals = 16;
 
 struct KnnArgs {
   KnnOperand q, c;
@@ -90,7 +101,10 @@ struct KnnArgs {
   const uint32_t* id_map;
   uint32_t* out_id;
   float* out_d;
-  uint32_t* replay;  // [0]: number of queries to replay, [1..]: the queries
+  uint32_t* counts;  // [0]: queries in replay, [1]: groups
+  uint32_t* replay;  // queries for k_knn_replay
+  uint32_t* groups;  // (group of 32 queries, mask of those) for k_knn_all, or nullptr
+  uint32_t* wide;    // with groups: per group, whether many of its margins were too wide
   int* err;
 };
 
@@ -196,6 +210,29 @@ struct WarpList {
     }
     worst_lane = __ffs(at) - 1;
   }
+  // Offers the candidates of the lanes in `mask`, all strictly closer than the
+  // worst, in ascending lane order.
+  __device__ __forceinline__ void keep(float cand, uint32_t cid, unsigned mask, int lane) {
+    while (mask) {  // its lowest lane is strictly closer than the worst
+      replace(cand, cid, __ffs(mask) - 1, lane);
+      mask &= mask - 1u;
+      mask &= __ballot_sync(0xffffffffu, cand < worst);
+    }
+  }
+  // The worst entry becomes lane src's candidate.
+  __device__ __forceinline__ void replace(float cand, uint32_t cid, int src, int lane) {
+    const float cd = __shfl_sync(0xffffffffu, cand, src);
+    const uint32_t ci = __shfl_sync(0xffffffffu, cid, src);
+    if (lane == worst_lane) {
+#pragma unroll
+      for (int s = 0; s < R; ++s)
+        if (s == worst_slot) {
+          d[s] = cd;
+          id[s] = ci;
+        }
+    }
+    find_worst();
+  }
   // Offers the candidates of the lanes in `mask` in ascending lane order;
   // returns the smaller of `next` and the values turned away or given up.
   __device__ __forceinline__ float offer(float cand, uint32_t cid, unsigned mask, int lane,
@@ -206,17 +243,7 @@ struct WarpList {
       const int src = __ffs(mask) - 1;
       away &= ~(1u << src);
       next = fminf(next, worst);
-      const float cd = __shfl_sync(0xffffffffu, cand, src);
-      const uint32_t ci = __shfl_sync(0xffffffffu, cid, src);
-      if (lane == worst_lane) {
-#pragma unroll
-        for (int s = 0; s < R; ++s)
-          if (s == worst_slot) {
-            d[s] = cd;
-            id[s] = ci;
-          }
-      }
-      find_worst();
+      replace(cand, cid, src, lane);
       mask &= mask - 1u;
       mask &= __ballot_sync(0xffffffffu, cand < worst);
     }
@@ -346,6 +373,146 @@ __device__ __forceinline__ void tmem_loaded<16>(float (&v)[16]) {
                  "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15])::"memory");
 }
 
+// The clusters that a CTA's queries search, in label order, as a bit per cluster
+// and, behind those words, the clusters before each word. uses(q): whether the
+// CTA's query q counts. Returns their number; wsum: a word per warp and one more.
+template <int THREADS, typename F>
+__device__ __forceinline__ uint32_t searched_clusters(const KnnArgs& a, uint64_t q0, uint32_t nq,
+                                                      uint32_t* bitmap, uint32_t* wsum, F uses) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const uint32_t words = (a.nc + 31) / 32;
+  uint32_t* rank = bitmap + words;
+  for (uint32_t w = tid; w < words; w += THREADS) bitmap[w] = 0u;
+  __syncthreads();
+  for (uint32_t t = tid; t < nq * a.cs; t += THREADS) {
+    const uint32_t lab = a.nearest[q0 * a.cs + t];
+    if (lab < a.nc && uses(t / a.cs)) atomicOr(&bitmap[lab >> 5], 1u << (lab & 31));  // order-free
+  }
+  __syncthreads();
+  const uint32_t per = (words + THREADS - 1) / THREADS;
+  const uint32_t w0 = min(words, tid * per), w1 = min(words, w0 + per);
+  uint32_t cnt = 0;
+  for (uint32_t w = w0; w < w1; ++w) cnt += __popc(bitmap[w]);
+  uint32_t incl = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) wsum[wid] = incl;
+  __syncthreads();
+  uint32_t pre = incl - cnt;
+  for (int w = 0; w < wid; ++w) pre += wsum[w];
+  for (uint32_t w = w0; w < w1; ++w) {
+    rank[w] = pre;
+    pre += __popc(bitmap[w]);
+  }
+  if (tid == THREADS - 1) wsum[THREADS / 32] = pre;
+  __syncthreads();
+  return wsum[THREADS / 32];
+}
+
+// The rank of a label among the searched clusters (of the next one, if it is
+// not one).
+__device__ __forceinline__ uint32_t cluster_rank(const uint32_t* bitmap, uint32_t nc,
+                                                 uint32_t lab) {
+  return bitmap[(nc + 31) / 32 + (lab >> 5)] +
+         __popc(bitmap[lab >> 5] & ((1u << (lab & 31)) - 1u));
+}
+
+// Searched clusters [ubase, ubase + nruns) of them: their rows [run_b, run_e),
+// and which of the CTA's queries search each (W words of bits). To be read
+// behind a barrier.
+template <int THREADS, int W, typename F>
+__device__ __forceinline__ void searched_runs(const KnnArgs& a, uint64_t q0, uint32_t nq,
+                                              const uint32_t* bitmap, uint32_t ubase,
+                                              uint32_t nruns, uint32_t* run_b, uint32_t* run_e,
+                                              uint32_t* qmask, F uses) {
+  if (nruns == 0) return;
+  const int tid = threadIdx.x;
+  const uint32_t words = (a.nc + 31) / 32;
+  for (uint32_t t = tid; t < nruns * W; t += THREADS) qmask[t] = 0u;
+  __syncthreads();
+  for (uint32_t w = tid; w < words; w += THREADS) {
+    uint32_t bits = bitmap[w], pos = bitmap[words + w];
+    while (bits) {
+      const uint32_t lab = w * 32 + __ffs(bits) - 1;
+      bits &= bits - 1u;
+      if (pos >= ubase && pos - ubase < nruns) {
+        run_b[pos - ubase] = (uint32_t)a.coff[lab];
+        run_e[pos - ubase] = (uint32_t)a.coff[lab + 1];
+      }
+      ++pos;
+    }
+  }
+  for (uint32_t t = tid; t < nq * a.cs; t += THREADS) {
+    const uint32_t lab = a.nearest[q0 * a.cs + t], q = t / a.cs;
+    if (lab >= a.nc || !uses(q)) continue;
+    const uint32_t pos = cluster_rank(bitmap, a.nc, lab);
+    if (pos >= ubase && pos - ubase < nruns)
+      atomicOr(&qmask[(pos - ubase) * W + (q >> 5)], 1u << (q & 31));
+  }
+}
+
+// One warp: run_s[u] = size(0) + .. + size(u - 1) for u in [0, nruns].
+template <typename F>
+__device__ __forceinline__ void run_starts(uint32_t* run_s, uint32_t nruns, F size) {
+  const int lane = threadIdx.x & 31;
+  uint32_t total = 0;
+  for (uint32_t u0 = 0; u0 < nruns; u0 += 32) {
+    const uint32_t u = u0 + lane, g = u < nruns ? size(u) : 0u;
+    uint32_t incl = g;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (u < nruns) run_s[u] = total + incl - g;
+    total += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  if (lane == 0) run_s[nruns] = total;
+}
+
+// The queries of a CTA (bits of bad, a word per 32) that are computed again:
+// groups of 32 with many go to k_knn_all, the others' queries to k_knn_replay.
+// over: queries whose margins are wider than the distances they are to tell
+// apart. Where that holds for a group's nearest clusters, it does for its cells:
+// their search does not try the filter (knows_wide).
+template <bool SEARCH>
+__device__ __forceinline__ void list_replays(const KnnArgs& a, uint64_t q0, const uint32_t* bad,
+                                             const uint32_t* over, uint32_t words) {
+  const uint32_t first = (uint32_t)q0 + 32 * threadIdx.x;
+  if (threadIdx.x >= words || first >= a.q.n) return;
+  uint32_t m = bad[threadIdx.x];
+  if (!SEARCH && a.groups)
+    a.wide[first / 32] = __popc(over[threadIdx.x]) >= kGroupReplays ? 1u : 0u;
+  if (a.groups && __popc(m) >= kGroupReplays) {
+    const uint32_t i = atomicAdd(a.counts + 1, 1u);
+    a.groups[2 * i] = first / 32;
+    a.groups[2 * i + 1] = m;
+  } else if (m) {
+    for (uint32_t i = atomicAdd(a.counts, (uint32_t)__popc(m)); m; m &= m - 1u)
+      a.replay[i++] = first + __ffs(m) - 1;
+  }
+}
+
+// Whether every group of the CTA's queries is known to be too wide for the
+// filter; they are listed for k_knn_all then.
+__device__ __forceinline__ bool knows_wide(const KnnArgs& a) {
+  if (!a.groups || refused(a)) return false;
+  const uint64_t q0 = blockIdx.x * (uint64_t)a.qt;
+  const uint32_t groups = (uint32_t)((min_u64(a.qt, a.q.n - q0) + 31) / 32);
+  bool all = true;
+  for (uint32_t g = 0; g < groups; ++g) all = all && a.wide[q0 / 32 + g] != 0u;
+  if (all && threadIdx.x < groups) {
+    const uint64_t first = q0 + 32 * threadIdx.x, left = a.q.n - first;
+    const uint32_t i = atomicAdd(a.counts + 1, 1u);
+    a.groups[2 * i] = (uint32_t)(first / 32);
+    a.groups[2 * i + 1] = left >= 32 ? 0xFFFFFFFFu : (1u << left) - 1u;
+  }
+  return all;
+}
+
 // Rows to a tensor-core operand. A block takes 4 groups (32 rows); group
 // storage: [part high, low][8-column group][row 0..7][8 BF16]. Columns d..d+2
 // of the high part hold -norm / 2 as three BF16 numbers; rows past n hold a
@@ -428,7 +595,7 @@ __global__ void __launch_bounds__(kTcKnnThreads, 1) k_knn_tc(const KnnArgs a) {
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + 64);
   __shared__ uint32_t meta_row[4][16], meta_run[4][16];  // per slot: first row, run
   __shared__ float meta_g[4];
-  __shared__ uint32_t wsum[kTcKnnWarps], s_union, s_slots;
+  __shared__ uint32_t wsum[kTcKnnWarps + 1], bad[4], over[4], evals, given;
   __shared__ volatile int stop;
   const uint32_t d = a.d, kp = a.kp, QT = a.qt;
   const KnnSmem L = knn_smem(kp, QT, NT, R, SEARCH, a.nc);
@@ -466,7 +633,9 @@ __global__ void __launch_bounds__(kTcKnnThreads, 1) k_knn_tc(const KnnArgs a) {
     }
     fence_mbar_init();
     stop = 0;
+    evals = 0;
   }
+  if (tid < 4) bad[tid] = over[tid] = 0u;
   // the queries' operand, with ones against the candidates' norm columns
   const uint64_t qgroups = (a.q.n + 7) / 8;
   for (uint32_t t = tid; t < QT / 8 * (gb / 16); t += kTcKnnThreads) {
@@ -508,38 +677,11 @@ __global__ void __launch_bounds__(kTcKnnThreads, 1) k_knn_tc(const KnnArgs a) {
     }
     own = lo;
   }
+  auto all = [](uint32_t) { return true; };
   if constexpr (SEARCH) {
-    const uint32_t words = (a.nc + 31) / 32;
-    uint32_t* rank = bitmap + words;
-    for (uint32_t w = tid; w < words; w += kTcKnnThreads) bitmap[w] = 0u;
-    __syncthreads();
-    for (uint32_t t = tid; t < nq * a.cs; t += kTcKnnThreads) {
-      const uint32_t lab = a.nearest[q0 * a.cs + t];
-      if (lab < a.nc) atomicOr(&bitmap[lab >> 5], 1u << (lab & 31));  // order-free
-    }
-    __syncthreads();
-    // rank of each word: the searched clusters before it
-    const uint32_t per = (words + kTcKnnThreads - 1) / kTcKnnThreads;
-    const uint32_t w0 = min(words, tid * per), w1 = min(words, w0 + per);
-    uint32_t cnt = 0;
-    for (uint32_t w = w0; w < w1; ++w) cnt += __popc(bitmap[w]);
-    uint32_t incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    if (lane == 31) wsum[wid] = incl;
-    __syncthreads();
-    uint32_t pre = incl - cnt;
-    for (int w = 0; w < wid; ++w) pre += wsum[w];
-    for (uint32_t w = w0; w < w1; ++w) {
-      rank[w] = pre;
-      pre += __popc(bitmap[w]);
-    }
-    if (tid == kTcKnnThreads - 1) s_union = pre;
-    __syncthreads();
-    nbits = s_union;
+    const bool wide = knows_wide(a);  // then there is nothing to do here
+    if (tid == 0) given = wide;
+    if (!wide) nbits = searched_clusters<kTcKnnThreads>(a, q0, nq, bitmap, wsum, all);
   }
   fence_proxy_async_smem();  // A's generic writes -> tensor-core reads
   tc_fence_before();
@@ -596,75 +738,37 @@ __global__ void __launch_bounds__(kTcKnnThreads, 1) k_knn_tc(const KnnArgs a) {
     __syncwarp();
   };
 
+  // Past this many exact evaluations the margins are too wide for the data: the
+  // CTA's queries go to the replay kernels, what is left of the tiles is not looked at.
+  const uint32_t most_evals = nq * a.size * (SEARCH ? kSearchEvals : kNearestEvals);
+  bool gave_up = false;  // known to this warp
   uint32_t gt = 0;  // tiles so far: buffers and phases
   uint32_t ubase = 0;
   bool ok = true;
   do {
     uint32_t nruns = 1, nslots;
     if constexpr (SEARCH) {
-      // the next kUnionCap searched clusters in label order: their rows, and
-      // which queries search them
-      const uint32_t words = (a.nc + 31) / 32;
-      const uint32_t* rank = bitmap + words;
+      // the next kUnionCap searched clusters in label order
       nruns = min(kUnionCap, nbits - ubase);
-      for (uint32_t t = tid; t < nruns * 4; t += kTcKnnThreads) qmask[t] = 0u;
-      __syncthreads();
-      for (uint32_t w = tid; w < words; w += kTcKnnThreads) {
-        uint32_t bits = bitmap[w], pos = rank[w];
-        while (bits) {
-          const uint32_t lab = w * 32 + __ffs(bits) - 1;
-          bits &= bits - 1u;
-          if (pos >= ubase && pos - ubase < nruns) {
-            run_b[pos - ubase] = (uint32_t)a.coff[lab];
-            run_e[pos - ubase] = (uint32_t)a.coff[lab + 1];
-          }
-          ++pos;
-        }
-      }
-      for (uint32_t t = tid; t < nq * a.cs; t += kTcKnnThreads) {
-        const uint32_t lab = a.nearest[q0 * a.cs + t], q = t / a.cs;
-        if (lab >= a.nc) continue;
-        const uint32_t pos =
-            rank[lab >> 5] + __popc(bitmap[lab >> 5] & ((1u << (lab & 31)) - 1u));
-        if (pos >= ubase && pos - ubase < nruns)
-          atomicOr(&qmask[(pos - ubase) * 4 + (q >> 5)], 1u << (q & 31));
-      }
+      searched_runs<kTcKnnThreads, 4>(a, q0, nq, bitmap, ubase, nruns, run_b, run_e, qmask, all);
     } else if (tid == 0) {
       run_b[0] = 0u;
       run_e[0] = (uint32_t)a.c.n;
     }
     __syncthreads();
-    if (wid == 0) {  // first slot of every run
-      uint32_t total = 0;
-      for (uint32_t u0 = 0; u0 < nruns; u0 += 32) {
-        const uint32_t u = u0 + lane;
-        uint32_t g = 0;
-        if (u < nruns && run_e[u] > run_b[u]) g = (run_e[u] + 7) / 8 - run_b[u] / 8;
-        uint32_t incl = g;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += v;
-        }
-        if (u < nruns) run_s[u] = total + incl - g;
-        total += __shfl_sync(0xffffffffu, incl, 31);
-      }
-      if (lane == 0) {
-        run_s[nruns] = total;
-        s_slots = total;
-      }
-    }
+    if (wid == 0)  // first slot of every run
+      run_starts(run_s, nruns, [&](uint32_t u) {
+        return run_e[u] > run_b[u] ? (run_e[u] + 7) / 8 - run_b[u] / 8 : 0u;
+      });
     __syncthreads();
-    nslots = s_slots;
+    nslots = run_s[nruns];
     const uint32_t ntiles = (nslots + SLOTS - 1) / SLOTS;
     // the tile that step t works on: from the own cluster's on, around
     uint32_t t0 = 0;
     if (a.coff && ntiles) {
       uint32_t slot = own / 8;  // nearest: the own centroid's group
       if constexpr (SEARCH) {
-        const uint32_t* rank = bitmap + (a.nc + 31) / 32;
-        const uint32_t pos =
-            rank[own >> 5] + __popc(bitmap[own >> 5] & ((1u << (own & 31)) - 1u));
+        const uint32_t pos = cluster_rank(bitmap, a.nc, own);
         slot = pos >= ubase && pos - ubase < nruns ? run_s[pos - ubase] : 0u;
       }
       t0 = min(slot / SLOTS, ntiles - 1);
@@ -783,6 +887,7 @@ __global__ void __launch_bounds__(kTcKnnThreads, 1) k_knn_tc(const KnnArgs a) {
       const uint32_t word =
           oq < nq ? masks[((g & 1u) * 4 + ((uint32_t)lane & 3u)) * 128 + oq] : 0u;
       uint32_t hit = __ballot_sync(0xffffffffu, word != 0u);
+      if (gave_up) continue;
       while (hit) {
         const int src = __ffs(hit) - 1;
         hit &= hit - 1u;
@@ -806,6 +911,9 @@ __global__ void __launch_bounds__(kTcKnnThreads, 1) k_knn_tc(const KnnArgs a) {
         __syncwarp();
         if (cnt >= 32u) {
           evaluate(q, 32u);
+          uint32_t made = 0;
+          if (lane == 0) made = atomicAdd(&evals, 32u);
+          gave_up = __shfl_sync(0xffffffffu, made, 0) >= most_evals;
           cnt -= 32u;
           const uint32_t rest = (uint32_t)lane < cnt ? queue[q * kQueue + 32 + lane] : 0u;
           __syncwarp();
@@ -820,9 +928,17 @@ __global__ void __launch_bounds__(kTcKnnThreads, 1) k_knn_tc(const KnnArgs a) {
     __syncthreads();  // the runs and tile descriptions are no longer read
   } while (SEARCH && ok && ubase < nbits);
 
-  if (ok && !refused(a)) {
+  if (ok && !(SEARCH && given) && !refused(a)) {
     // what is left in the queues, then the sorted lists
+    const bool again = evals > most_evals;
     for (uint32_t q = wid; q < nq; q += kTcKnnWarps) {
+      if (again) {
+        if (lane == 0) {
+          atomicOr(&bad[q >> 5], 1u << (q & 31));
+          atomicOr(&over[q >> 5], 1u << (q & 31));
+        }
+        continue;
+      }
       const uint32_t cnt = qcnt[q];
       if (cnt) evaluate(q, cnt);
       write_sorted(ld + q * R * 32, li + q * R * 32, a.size, SEARCH ? a.id_map : nullptr,
@@ -830,7 +946,7 @@ __global__ void __launch_bounds__(kTcKnnThreads, 1) k_knn_tc(const KnnArgs a) {
       if (a.coff && lane == 0) {
         float w = ld[q * R * 32];
         for (uint32_t e = 1; e < a.size; ++e) w = fmaxf(w, ld[q * R * 32 + e]);
-        if (qnext[q] == w) a.replay[1 + atomicAdd(a.replay, 1u)] = (uint32_t)(q0 + q);
+        if (qnext[q] == w) atomicOr(&bad[q >> 5], 1u << (q & 31));
       }
     }
   } else if (!ok && tid == 0) {
@@ -844,6 +960,7 @@ __global__ void __launch_bounds__(kTcKnnThreads, 1) k_knn_tc(const KnnArgs a) {
     }
   }
   __syncthreads();
+  list_replays<SEARCH>(a, q0, bad, over, QT / 32);
   tc_fence_after();
   if (wid == 0) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
@@ -879,8 +996,8 @@ __global__ void __launch_bounds__(kTcKnnThreads, 1) k_knn_tc(const KnnArgs a) {
 // copied 8 rows at a time (1,250 cycles of issue); ~2,000 now, the filter's
 // instructions in the first pass, the MMAs in the second. A thread first takes
 // the largest of each slot's 8 values; almost always that ends it.
-// Queued candidates past the queue's room (margins too wide for the data), and
-// lists whose last distance is tied, are listed for k_knn_replay. Lists of
+// Queries with more queued candidates than the queue's room (margins too wide for
+// the data), and lists whose last distance is tied, are computed again. Lists of
 // one entry need no tie rule: the first of equal distances is the lowest row.
 constexpr int kTwoThreads = kTcKnnThreads + 64;  // and the copy and MMA warps
 constexpr uint32_t kTwoAcc = 4;                  // accumulators in TMEM
@@ -1011,7 +1128,7 @@ __global__ void __launch_bounds__(kTwoThreads, 1) k_knn_two(const KnnArgs a) {
   // per slot of a tile: first row, run, rows of the run (bits), norm bound
   __shared__ uint32_t meta_row[kTwoMeta][16], meta_run[kTwoMeta][16], meta_bits[kTwoMeta][16];
   __shared__ __align__(16) float meta_g[kTwoMeta][16];
-  __shared__ uint32_t wsum[kTwoThreads / 32], s_union, s_slots;
+  __shared__ uint32_t wsum[kTwoThreads / 32 + 1], bad[4], over[4], given;
   __shared__ volatile int stop;
   const uint32_t d = a.d, kp = a.kp, QT = a.qt;
   const uint32_t NB = a.stages;
@@ -1055,6 +1172,7 @@ __global__ void __launch_bounds__(kTwoThreads, 1) k_knn_two(const KnnArgs a) {
     fence_mbar_init();
     stop = 0;
   }
+  if (tid < 4) bad[tid] = over[tid] = 0u;
   // the queries' operand, with ones against the candidates' norm columns
   const uint64_t qgroups = (a.q.n + 7) / 8;
   for (uint32_t t = tid; t < QT / 8 * (gb / 16); t += kTwoThreads) {
@@ -1089,38 +1207,11 @@ __global__ void __launch_bounds__(kTwoThreads, 1) k_knn_two(const KnnArgs a) {
     }
     own = lo;
   }
+  auto all = [](uint32_t) { return true; };
   if constexpr (SEARCH) {
-    const uint32_t words = (a.nc + 31) / 32;
-    uint32_t* rank = bitmap + words;
-    for (uint32_t w = tid; w < words; w += kTwoThreads) bitmap[w] = 0u;
-    __syncthreads();
-    for (uint32_t t = tid; t < nq * a.cs; t += kTwoThreads) {
-      const uint32_t lab = a.nearest[q0 * a.cs + t];
-      if (lab < a.nc) atomicOr(&bitmap[lab >> 5], 1u << (lab & 31));  // order-free
-    }
-    __syncthreads();
-    // rank of each word: the searched clusters before it
-    const uint32_t per = (words + kTwoThreads - 1) / kTwoThreads;
-    const uint32_t w0 = min(words, tid * per), w1 = min(words, w0 + per);
-    uint32_t cnt = 0;
-    for (uint32_t w = w0; w < w1; ++w) cnt += __popc(bitmap[w]);
-    uint32_t incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    if (lane == 31) wsum[wid] = incl;
-    __syncthreads();
-    uint32_t pre = incl - cnt;
-    for (int w = 0; w < wid; ++w) pre += wsum[w];
-    for (uint32_t w = w0; w < w1; ++w) {
-      rank[w] = pre;
-      pre += __popc(bitmap[w]);
-    }
-    if (tid == kTwoThreads - 1) s_union = pre;
-    __syncthreads();
-    nbits = s_union;
+    const bool wide = knows_wide(a);  // then there is nothing to do here
+    if (tid == 0) given = wide;
+    if (!wide) nbits = searched_clusters<kTwoThreads>(a, q0, nq, bitmap, wsum, all);
   }
   fence_proxy_async_smem();  // A's generic writes -> tensor-core reads
   tc_fence_before();
@@ -1139,6 +1230,7 @@ __global__ void __launch_bounds__(kTwoThreads, 1) k_knn_two(const KnnArgs a) {
 #pragma unroll
   for (int i = 0; i < M; ++i) top[i] = -INFINITY;
   float mytau = -INFINITY;
+  bool open = filters;  // pass 2: until the query's queue overflows
 
   uint32_t gt = 0;              // tiles so far: accumulators and phases
   uint32_t st = 0, phase = 0;   // the operand stage that comes next, its round (parity)
@@ -1148,69 +1240,27 @@ __global__ void __launch_bounds__(kTwoThreads, 1) k_knn_two(const KnnArgs a) {
     do {
       uint32_t nruns = 1;
       if constexpr (SEARCH) {
-        // the next kUnionCap searched clusters in label order: their rows, and
-        // which queries search them
-        const uint32_t words = (a.nc + 31) / 32;
-        const uint32_t* rank = bitmap + words;
+        // the next kUnionCap searched clusters in label order
         nruns = min(kUnionCap, nbits - ubase);
-        for (uint32_t t = tid; t < nruns * 4; t += kTwoThreads) qmask[t] = 0u;
-        __syncthreads();
-        for (uint32_t w = tid; w < words; w += kTwoThreads) {
-          uint32_t bits = bitmap[w], pos = rank[w];
-          while (bits) {
-            const uint32_t lab = w * 32 + __ffs(bits) - 1;
-            bits &= bits - 1u;
-            if (pos >= ubase && pos - ubase < nruns) {
-              run_b[pos - ubase] = (uint32_t)a.coff[lab];
-              run_e[pos - ubase] = (uint32_t)a.coff[lab + 1];
-            }
-            ++pos;
-          }
-        }
-        for (uint32_t t = tid; t < nq * a.cs; t += kTwoThreads) {
-          const uint32_t lab = a.nearest[q0 * a.cs + t], q = t / a.cs;
-          if (lab >= a.nc) continue;
-          const uint32_t pos =
-              rank[lab >> 5] + __popc(bitmap[lab >> 5] & ((1u << (lab & 31)) - 1u));
-          if (pos >= ubase && pos - ubase < nruns)
-            atomicOr(&qmask[(pos - ubase) * 4 + (q >> 5)], 1u << (q & 31));
-        }
+        searched_runs<kTwoThreads, 4>(a, q0, nq, bitmap, ubase, nruns, run_b, run_e, qmask, all);
       } else if (tid == 0) {
         run_b[0] = 0u;
         run_e[0] = (uint32_t)a.c.n;
       }
       __syncthreads();
-      if (wid == 0) {  // first slot of every run
-        uint32_t total = 0;
-        for (uint32_t u0 = 0; u0 < nruns; u0 += 32) {
-          const uint32_t u = u0 + lane;
-          uint32_t g = 0;
-          if (u < nruns && run_e[u] > run_b[u]) g = (run_e[u] + 7) / 8 - run_b[u] / 8;
-          uint32_t incl = g;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-          }
-          if (u < nruns) run_s[u] = total + incl - g;
-          total += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (lane == 0) {
-          run_s[nruns] = total;
-          s_slots = total;
-        }
-      }
+      if (wid == 0)  // first slot of every run
+        run_starts(run_s, nruns, [&](uint32_t u) {
+          return run_e[u] > run_b[u] ? (run_e[u] + 7) / 8 - run_b[u] / 8 : 0u;
+        });
       __syncthreads();
-      const uint32_t nslots = s_slots;
+      const uint32_t nslots = run_s[nruns];
       const uint32_t ntiles = (nslots + SLOTS - 1) / SLOTS;
       // the tile that step t works on: from the own cluster's on, around
       uint32_t t0 = 0;
       if (a.coff && ntiles) {
         uint32_t slot = own / 8;  // nearest: the own centroid's group
         if constexpr (SEARCH) {
-          const uint32_t* rank = bitmap + (a.nc + 31) / 32;
-          const uint32_t pos =
-              rank[own >> 5] + __popc(bitmap[own >> 5] & ((1u << (own & 31)) - 1u));
+          const uint32_t pos = cluster_rank(bitmap, a.nc, own);
           slot = pos >= ubase && pos - ubase < nruns ? run_s[pos - ubase] : 0u;
         }
         t0 = min(slot / SLOTS, ntiles - 1);
@@ -1337,7 +1387,7 @@ __global__ void __launch_bounds__(kTwoThreads, 1) k_knn_two(const KnnArgs a) {
             const float* w = v + 8 * i;
             const float mg = kMargin * gs[i] * (ql + gs[i]) + aq;
             const float lim = ONE ? mytau - mg : pass == 0 ? top[M - 1] + mg : mytau - mg;
-            if (mx[i] <= lim || !filters) continue;  // NaN goes on
+            if (mx[i] <= lim || !open) continue;  // NaN goes on
             const uint32_t slot = slot0 + i, u = meta_run[m][slot], row = meta_row[m][slot];
             uint32_t left = u != kNoRun ? meta_bits[m][slot] : 0u;
             if (SEARCH) {
@@ -1380,6 +1430,7 @@ __global__ void __launch_bounds__(kTwoThreads, 1) k_knn_two(const KnnArgs a) {
                 if (((left >> k) & 1u) && !(w[k] <= lim)) {
                   const uint32_t pos = atomicAdd(&qcnt[qi], 1u);
                   if (pos < (uint32_t)CAP) queue[qi * CAP + pos] = row + k;
+                  else open = false;
                 }
             }
           }
@@ -1452,6 +1503,15 @@ __global__ void __launch_bounds__(kTwoThreads, 1) k_knn_two(const KnnArgs a) {
             float t = key_value(cut[i]);
             if (cut[i] <= 0x007FFFFFu) t = -INFINITY;  // -inf's key and below
             if (lane == i && q1 + i < nq) tau[q1 + i] = t;
+            if constexpr (!SEARCH) {  // the list's own range is within the margins
+              uint32_t most = key[i][0];
+#pragma unroll
+              for (int e = 1; e < E; ++e) most = max(most, key[i][e]);
+              const float range = key_value(__reduce_max_sync(0xffffffffu, most)) - t;
+              const float len = qlen[min(q1 + i, nq - 1)];
+              if (lane == i && q1 + i < nq && range <= 4.f * kMargin * len * len)
+                atomicOr(&over[(q1 + i) >> 5], 1u << ((q1 + i) & 31));
+            }
           }
         }
       }
@@ -1460,7 +1520,7 @@ __global__ void __launch_bounds__(kTwoThreads, 1) k_knn_two(const KnnArgs a) {
     }
   }
 
-  if (ok && !refused(a)) {
+  if (ok && !(SEARCH && given) && !refused(a)) {
     // The exact distances of what is queued, a thread per (query, entry) over
     // the whole CTA (a warp per query instead waits for its few rows alone,
     // eight times in turn), where the operands were; then the entries' ranks.
@@ -1575,10 +1635,10 @@ __global__ void __launch_bounds__(kTwoThreads, 1) k_knn_two(const KnnArgs a) {
           }
           __syncwarp();
         }
-        const bool over = qcnt[q] > (uint32_t)CAP;
-        if (lane == 0 && (over || (a.size > 1 && valid > a.size && last[q] == next[q])))
-          a.replay[1 + atomicAdd(a.replay, 1u)] = (uint32_t)(q0 + q);
-        if (!over)
+        const bool full = qcnt[q] > (uint32_t)CAP;
+        if (lane == 0 && (full || (a.size > 1 && valid > a.size && last[q] == next[q])))
+          atomicOr(&bad[q >> 5], 1u << (q & 31));
+        if (!full)
           for (uint32_t e = valid + lane; e < a.size; e += 32) {  // empty entries
             a.out_d[(q0 + q) * a.size + e] = FLT_MAX;
             a.out_id[(q0 + q) * a.size + e] = 0xFFFFFFFFu;
@@ -1596,6 +1656,7 @@ __global__ void __launch_bounds__(kTwoThreads, 1) k_knn_two(const KnnArgs a) {
           __nanosleep(64);
   }
   __syncthreads();
+  list_replays<SEARCH>(a, q0, bad, over, QT / 32);
   tc_fence_after();
   if (wid == 0) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
@@ -1604,7 +1665,7 @@ __global__ void __launch_bounds__(kTwoThreads, 1) k_knn_two(const KnnArgs a) {
   }
 }
 
-// The queries in replay[1..replay[0]], a CTA each: every candidate evaluated
+// The queries in replay, a CTA each: every candidate evaluated
 // (kReplayBatch at a time, a thread each) and offered by one warp in the
 // reference's order. The searched clusters' rows are one sequence: batches that
 // ended with each cluster of ~137 rows took 0.69 ms for 38 queries of 8.8k
@@ -1621,9 +1682,9 @@ __global__ void __launch_bounds__(kReplayThreads) k_knn_replay(const KnnArgs a) 
   __shared__ uint32_t lab[SEARCH ? kReplayThreads : 1], begin[SEARCH ? kReplayThreads : 1];
   __shared__ uint32_t before[SEARCH ? kReplayThreads + 1 : 1], wsum[kReplayThreads / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const uint32_t count = a.replay[0], d = a.d;
+  const uint32_t count = a.counts[0], d = a.d;
   for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
-    const uint64_t q = a.replay[1 + i];
+    const uint64_t q = a.replay[i];
     const float* x = a.q.rows + q * d;
     const float nm = SEARCH ? a.q.norms[q] : 0.f;
     for (uint32_t e = threadIdx.x; e < R * 32; e += kReplayThreads) {
@@ -1688,8 +1749,8 @@ __global__ void __launch_bounds__(kReplayThreads) k_knn_replay(const KnnArgs a) 
           const bool in = k + lane < len;
           const uint32_t row = in ? ids[k + lane] : 0u;
           const bool use = in && !(SEARCH && row == q);
-          best.offer(use ? dist[k + lane] : INFINITY, row, __ballot_sync(0xffffffffu, use), lane,
-                     0.f);
+          const float cand = use ? dist[k + lane] : INFINITY;
+          best.keep(cand, row, __ballot_sync(0xffffffffu, cand < best.worst), lane);
         }
       __syncthreads();
     }
@@ -1703,9 +1764,231 @@ __global__ void __launch_bounds__(kReplayThreads) k_knn_replay(const KnnArgs a) 
   }
 }
 
+// Row stride (floats) of rows staged whole: a multiple of 4 whose float4 count
+// is odd, so that lanes reading float4s of successive rows meet no bank twice.
+__host__ __device__ inline uint32_t row_stride(uint32_t d) {
+  const uint32_t s = (d + 3u) & ~3u;
+  return (s >> 2) & 1u ? s : s + 4u;
+}
+
+// The groups of 32 queries in groups, a CTA each: the exhaustive search, for
+// data on which the filter decides nothing (margins wider than the distances'
+// spread, as PCs far from their origin have, or ties at most lists' ends, as
+// repeated cells have). All rows of the group's searched clusters as one
+// sequence, 128 staged at a time; a warp takes four of the queries and four rows
+// per lane, an FP32 chain each, and offers what is closer than a list's worst in
+// the reference's order. Shared loads: 20 wavefronts per 16 warp multiply-adds
+// of four dimensions, against 12 per 8 for two rows per lane. 300k x 50 dims, 2,191
+// clusters, 64 searched, 20 neighbours, every list: search 27 ms, nearest clusters
+// 10.5 ms (two rows per lane, lists in registers: 36.7 and 20.9; a CTA per query:
+// 124 both). Three CTAs per SM: with 256 clusters at a time for lists of up to 128
+// (100 neighbours 48.6 ms, with two CTAs 70); four leave 64 registers, slower for
+// lists past 32 (50 neighbours 33 and 42 ms).
+constexpr int kAllThreads = 256;
+constexpr uint32_t kAllQueries = 32, kAllRows = 128;
+constexpr uint32_t kAllRuns = 256;  // searched clusters taken at once
+constexpr int kAllPerWarp = (int)kAllQueries / (kAllThreads / 32), kAllPerLane = (int)kAllRows / 32;
+
+struct AllSmem {  // byte offsets
+  uint32_t tile, x, norm, row, mask, list, runs, qmask, bitmap, total;
+};
+
+__host__ __device__ inline AllSmem all_smem(uint32_t d, uint32_t R, bool search, uint32_t nc) {
+  AllSmem L;
+  uint32_t o = 0;
+  auto take = [&](uint32_t bytes) {
+    const uint32_t at = o;
+    o += (bytes + 15u) & ~15u;
+    return at;
+  };
+  L.tile = take(kAllRows * row_stride(d) * 4);
+  L.x = take(kAllQueries * row_stride(d) * 4);
+  L.norm = take(kAllRows * 4);
+  L.row = take(kAllRows * 4);
+  L.mask = take(kAllRows * 4);  // the group's queries that search the row's cluster
+  L.list = take(kAllQueries * R * 32 * 8);
+  L.runs = take(search ? kAllRuns * 12 + 4 : 16);
+  L.qmask = take(search ? kAllRuns * 4 : 16);
+  L.bitmap = take(search ? (nc + 31) / 32 * 8 : 16);  // words and their ranks
+  L.total = o;
+  return L;
+}
+
+template <int R, bool SEARCH>
+__global__ void __launch_bounds__(kAllThreads, R <= 4 ? 3 : 2)
+k_knn_all(const KnnArgs a, int vec) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  __shared__ uint32_t wsum[kAllThreads / 32 + 1];
+  const uint32_t d = a.d, st = row_stride(d);
+  const AllSmem L = all_smem(d, R, SEARCH, a.nc);
+  float* tile = reinterpret_cast<float*>(smem + L.tile);
+  float* xs = reinterpret_cast<float*>(smem + L.x);
+  float* norm = reinterpret_cast<float*>(smem + L.norm);
+  uint32_t* rows = reinterpret_cast<uint32_t*>(smem + L.row);
+  uint32_t* mask = reinterpret_cast<uint32_t*>(smem + L.mask);
+  float* ld = reinterpret_cast<float*>(smem + L.list);
+  uint32_t* li = reinterpret_cast<uint32_t*>(ld + kAllQueries * R * 32);
+  uint32_t* run_b = reinterpret_cast<uint32_t*>(smem + L.runs);  // run: rows [b, e)
+  uint32_t* run_e = run_b + (SEARCH ? kAllRuns : 1);
+  uint32_t* run_s = run_e + (SEARCH ? kAllRuns : 1);  // rows before the run
+  uint32_t* qmask = reinterpret_cast<uint32_t*>(smem + L.qmask);
+  uint32_t* bitmap = reinterpret_cast<uint32_t*>(smem + L.bitmap);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  // a query's columns past d are zero, so what the rows hold there adds nothing
+  // once it is a number
+  for (uint32_t t = tid; t < kAllRows * (st - d); t += kAllThreads)
+    tile[t / (st - d) * st + d + t % (st - d)] = 0.f;
+  const uint32_t count = a.counts[1];
+  for (uint32_t gi = blockIdx.x; gi < count; gi += gridDim.x) {
+    const uint64_t q0 = (uint64_t)a.groups[2 * gi] * kAllQueries;
+    const uint32_t live = a.groups[2 * gi + 1];
+    const uint32_t nq = (uint32_t)min_u64(kAllQueries, a.q.n - q0);
+    auto uses = [&](uint32_t q) { return ((live >> q) & 1u) != 0u; };
+    __syncthreads();  // the group before is done
+    for (uint32_t t = tid; t < kAllQueries * st; t += kAllThreads) {
+      const uint32_t q = t / st, j = t % st;
+      xs[t] = q < nq && j < d ? a.q.rows[(q0 + q) * d + j] : 0.f;
+    }
+    for (uint32_t t = tid; t < kAllQueries * R * 32; t += kAllThreads) {
+      ld[t] = t % (R * 32) < a.size ? FLT_MAX : -INFINITY;
+      li[t] = 0xFFFFFFFFu;
+    }
+    float worst[kAllPerWarp], qn[kAllPerWarp];
+#pragma unroll
+    for (int i = 0; i < kAllPerWarp; ++i) {
+      const uint32_t q = wid * kAllPerWarp + i;
+      worst[i] = uses(q) ? FLT_MAX : -INFINITY;  // nothing is closer than -inf
+      qn[i] = SEARCH && q < nq ? a.q.norms[q0 + q] : 0.f;
+    }
+    const uint32_t mine = live & (((1u << kAllPerWarp) - 1u) << (wid * kAllPerWarp));
+    uint32_t nbits = 0, ubase = 0;
+    if constexpr (SEARCH) nbits = searched_clusters<kAllThreads>(a, q0, nq, bitmap, wsum, uses);
+    do {
+      uint32_t nruns = 1, total = (uint32_t)a.c.n;
+      if constexpr (SEARCH) {
+        nruns = min(kAllRuns, nbits - ubase);
+        searched_runs<kAllThreads, 1>(a, q0, nq, bitmap, ubase, nruns, run_b, run_e, qmask, uses);
+        __syncthreads();
+        if (wid == 0) run_starts(run_s, nruns, [&](uint32_t u) { return run_e[u] - run_b[u]; });
+        __syncthreads();
+        total = run_s[nruns];
+      }
+      for (uint32_t r0 = 0; r0 < total; r0 += kAllRows) {
+        __syncthreads();  // the tile before has been read
+        if (tid < (int)kAllRows) {
+          const uint32_t at = r0 + tid;
+          uint32_t row = 0, who = 0;
+          if (at < total) {
+            row = at;
+            who = live;
+            if constexpr (SEARCH) {
+              uint32_t u = 0, hi = nruns;  // the last run that starts at or before it
+              while (hi - u > 1) {
+                const uint32_t mid = (u + hi) / 2;
+                if (run_s[mid] <= at) u = mid;
+                else hi = mid;
+              }
+              row = run_b[u] + (at - run_s[u]);
+              who = qmask[u];
+            }
+          }
+          rows[tid] = row;
+          mask[tid] = who;
+          norm[tid] = who ? a.c.norms[row] : 0.f;
+        }
+        __syncthreads();
+        for (uint32_t r = wid; r < kAllRows; r += kAllThreads / 32) {
+          if (mask[r] == 0u) continue;  // past the last row
+          const float* src = a.c.rows + (uint64_t)rows[r] * d;
+          float* dst = tile + r * st;
+          if (vec == 4)
+            for (uint32_t j = lane * 4; j < d; j += 128) cp_async<16>(dst + j, src + j);
+          else if (vec == 2)
+            for (uint32_t j = lane * 2; j < d; j += 64) cp_async<8>(dst + j, src + j);
+          else
+            for (uint32_t j = lane; j < d; j += 32) cp_async<4>(dst + j, src + j);
+        }
+        cp_async_wait();
+        __syncthreads();
+        uint32_t who = 0;
+#pragma unroll
+        for (int c = 0; c < kAllPerLane; ++c) who |= mask[32 * c + lane];
+        if (!__any_sync(0xffffffffu, (who & mine) != 0u)) continue;
+        float acc[kAllPerWarp][kAllPerLane];
+#pragma unroll
+        for (int i = 0; i < kAllPerWarp; ++i)
+#pragma unroll
+          for (int c = 0; c < kAllPerLane; ++c) acc[i][c] = 0.f;
+        const float* xp = xs + (size_t)wid * kAllPerWarp * st;
+        const float* cp = tile + (size_t)lane * st;
+        for (uint32_t j = 0; j < d; j += 4) {
+          float4 cv[kAllPerLane];
+#pragma unroll
+          for (int c = 0; c < kAllPerLane; ++c)
+            cv[c] = *reinterpret_cast<const float4*>(cp + 32 * c * st + j);
+#pragma unroll
+          for (int i = 0; i < kAllPerWarp; ++i) {
+            const float4 x = *reinterpret_cast<const float4*>(xp + i * st + j);
+#pragma unroll
+            for (int c = 0; c < kAllPerLane; ++c) {
+              acc[i][c] = fmaf(x.x, cv[c].x, acc[i][c]);
+              acc[i][c] = fmaf(x.y, cv[c].y, acc[i][c]);
+              acc[i][c] = fmaf(x.z, cv[c].z, acc[i][c]);
+              acc[i][c] = fmaf(x.w, cv[c].w, acc[i][c]);
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < kAllPerWarp; ++i) {
+          const uint32_t q = wid * kAllPerWarp + i;
+          WarpList<R> best;
+          bool loaded = false;
+#pragma unroll
+          for (int c = 0; c < kAllPerLane; ++c) {
+            const uint32_t r = 32 * c + lane, row = rows[r];
+            const float pd = fmaf(-2.f, acc[i][c], norm[r]);  // |c|^2 - 2 x.c
+            const float cand = SEARCH ? qn[i] + pd : pd;
+            const bool use = ((mask[r] >> q) & 1u) && !(SEARCH && row == q0 + q);
+            const unsigned closer = __ballot_sync(0xffffffffu, use && cand < worst[i]);
+            if (!closer) continue;
+            if (!loaded) best.load(ld + q * R * 32, li + q * R * 32, lane);
+            loaded = true;
+            // lanes that may not be offered never get closer than the worst
+            best.keep(use ? cand : INFINITY, row, closer, lane);
+            worst[i] = best.worst;
+          }
+          if (loaded) best.store(ld + q * R * 32, li + q * R * 32, lane);
+        }
+      }
+      ubase += nruns;
+    } while (SEARCH && ubase < nbits);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < kAllPerWarp; ++i) {
+      const uint32_t q = wid * kAllPerWarp + i;
+      if (uses(q))
+        write_sorted(ld + q * R * 32, li + q * R * 32, a.size, SEARCH ? a.id_map : nullptr,
+                     a.out_d + (q0 + q) * a.size, a.out_id + (q0 + q) * a.size, lane);
+    }
+  }
+}
+
+// Floats per load of both matrices' rows.
+int row_vec(const KnnArgs& a) {
+  const uintptr_t at = (uintptr_t)a.q.rows | (uintptr_t)a.c.rows;
+  return a.d % 4 == 0 && at % 16 == 0 ? 4 : a.d % 2 == 0 && at % 8 == 0 ? 2 : 1;
+}
+
 template <int R, bool SEARCH, int VEC>
 int launch_replay(const KnnArgs& a, cudaStream_t s) {
   k_knn_replay<R, SEARCH, VEC><<<num_sms() * 4, kReplayThreads, 0, s>>>(a);
+  BGPU_CHECK_LAUNCH();
+  if (!a.groups) return BGPU_OK;
+  const size_t smem = all_smem(a.d, R, SEARCH, a.nc).total;
+  BGPU_CUDA((allow_max_smem(k_knn_all<R, SEARCH>)));
+  const uint64_t want = ceil_div(a.q.n, kAllQueries);
+  k_knn_all<R, SEARCH><<<(unsigned)std::min<uint64_t>(want, (uint64_t)num_sms() * 3),
+                         kAllThreads, smem, s>>>(a, VEC);
   BGPU_CHECK_LAUNCH();
   return BGPU_OK;
 }
@@ -1736,12 +2019,6 @@ int launch_two(const KnnArgs& a, cudaStream_t s) {
 
 // Dynamic shared memory beside the kernels' static part.
 size_t knn_smem_limit() { return (size_t)device_smem_optin() - 4096; }
-
-// Floats per load of both matrices' rows.
-int row_vec(const KnnArgs& a) {
-  const uintptr_t at = (uintptr_t)a.q.rows | (uintptr_t)a.c.rows;
-  return a.d % 4 == 0 && at % 16 == 0 ? 4 : a.d % 2 == 0 && at % 8 == 0 ? 2 : 1;
-}
 
 // 128-candidate tiles where they fit with 128 queries, else 64; then the most
 // queries per CTA (128, 64, 32) that fit and leave no SM idle. bytes(qt, nt):
@@ -1808,6 +2085,19 @@ int launch_lists(const KnnArgs& a, cudaStream_t s) {
     return a.size <= 128 ? launch_one_shape<4, SEARCH>(a, s) : launch_one_shape<8, SEARCH>(a, s);
 }
 
+// The lists of what is computed again. Groups from one per SM on: where every list
+// is computed again they pay from 1,800 cells (2,700 cells: 0.50 ms against 0.65,
+// 4,500: 0.69 against 1.31), but k_knn_all's two launches cost every call ~8 us.
+int set_replay(KnnArgs* a, uint32_t* mem, cudaStream_t s) {
+  a->counts = mem;
+  a->replay = mem + 2;
+  const uint64_t groups = ceil_div(a->q.n, kAllQueries);
+  a->groups = groups >= (uint64_t)num_sms() ? mem + 2 + a->q.n : nullptr;
+  a->wide = mem + 2 + a->q.n + 2 * groups;
+  BGPU_CUDA(cudaMemsetAsync(mem, 0, 8, s));
+  return BGPU_OK;
+}
+
 }  // namespace
 
 uint32_t knn_kp(uint32_t d) { return (d + kNormCols + 15u) & ~15u; }
@@ -1833,6 +2123,8 @@ int knn_prepare(KnnOperand* op, const float* rows, const float* norms, uint64_t 
   return BGPU_OK;
 }
 
+size_t knn_replay_bytes(uint64_t n) { return (2 + n + 3 * ceil_div(n, kAllQueries)) * 4; }
+
 int knn_tc_nearest(const KnnOperand& queries, const KnnOperand& cand, uint32_t d, uint32_t count,
                    const uint64_t* coff, uint32_t* replay, uint32_t* out_id, float* out_d,
                    int* err, cudaStream_t s) {
@@ -1844,8 +2136,7 @@ int knn_tc_nearest(const KnnOperand& queries, const KnnOperand& cand, uint32_t d
   a.size = count;
   a.coff = coff;
   a.nc = (uint32_t)cand.n;
-  a.replay = replay;
-  BGPU_CUDA(cudaMemsetAsync(replay, 0, 4, s));
+  BGPU_TRY(set_replay(&a, replay, s));
   a.out_id = out_id;
   a.out_d = out_d;
   a.err = err;
@@ -1856,9 +2147,8 @@ int knn_tc_search(const KnnOperand& cells, uint32_t d, const uint64_t* coff, uin
                   const uint32_t* nearest, uint32_t cs, uint32_t k, const uint32_t* id_map,
                   uint32_t* replay, uint32_t* out_id, float* out_d, int* err, cudaStream_t s) {
   KnnArgs a{};
-  BGPU_CUDA(cudaMemsetAsync(replay, 0, 4, s));
-  a.replay = replay;
   a.q = cells;
+  BGPU_TRY(set_replay(&a, replay, s));
   a.c = cells;
   a.d = d;
   a.kp = knn_kp(d);

@@ -26,6 +26,7 @@ struct KnnOperand {
 
 uint32_t knn_kp(uint32_t d);                       // padded columns of an operand
 size_t knn_operand_bytes(uint64_t n, uint32_t d);  // device bytes of one
+size_t knn_replay_bytes(uint64_t n);               // scratch of a search by n queries
 // Lays `op` out in `mem` (knn_operand_bytes) and fills it. norms may be
 // nullptr for an operand used for queries only (zeros take their place).
 int knn_prepare(KnnOperand* op, const float* rows, const float* norms, uint64_t n, uint32_t d,
@@ -35,7 +36,7 @@ int knn_prepare(KnnOperand* op, const float* rows, const float* norms, uint64_t 
 // |c|^2 - 2 x.c, sorted; ids are candidate rows. coff (may be nullptr): the
 // offsets of the queries' clusters where those are sorted by cluster and the
 // candidates are the clusters' centroids in order; nullptr with count 1.
-// replay: n + 1 words of scratch. err: device error word.
+// replay: knn_replay_bytes(queries) of scratch. err: device error word.
 int knn_tc_nearest(const KnnOperand& queries, const KnnOperand& cand, uint32_t d, uint32_t count,
                    const uint64_t* coff, uint32_t* replay, uint32_t* out_id, float* out_d,
                    int* err, cudaStream_t s);

@@ -342,3 +342,75 @@ def test_knn_self_refusal_leaves_the_outputs(cuda, k, cs):
     nothing is written (lists on both sides of 64 entries)."""
     for name, t in _refused_call(cuda, 400, 6, 80, k, cs, 0.0).items():
         assert (t == 7).all(), name
+
+
+
+def _norms_of(X):
+    return np.einsum("ij,ij->i", X, X).astype(np.float32)
+
+
+@pytest.mark.parametrize("queries,d,nc,k,cs,kind", [
+    (64, 4, 60, 20, 3, "repeat"), (64, 3, 60, 64, 5, "offset"), (64, 2, 700, 5, 256, "offset"),
+    (64, 6, 90, 65, 66, "offset"), (128, 5, 150, 33, 40, "repeat"), (128, 4, 90, 1, 2, "repeat"),
+    (128, 2, 150, 128, 130, "repeat"), (128, 7, 200, 24, 64, "plain"), (128, 50, 300, 40, 9, "plain"),
+    (128, 8, 90, 100, 70, "plain")])
+def test_knn_self_bit_exact_at_full_tiles(cuda, queries, d, nc, k, cs, kind):
+    """The exhaustive loop's bits where a CTA takes 64 or 128 queries (that many
+    per SM, and a ragged last CTA), for every class of list lengths; with rows
+    that repeat (most lists end in a tie) and rows far from the origin (margins
+    wider than the spread), which whole groups of queries compute again. First,
+    last and random rows are compared."""
+    import torch
+    n = queries * torch.cuda.get_device_properties(cuda).multi_processor_count + 37
+    rng = np.random.default_rng(n + d)
+    X = rng.standard_normal((n, d)).astype(np.float32)
+    if kind == "repeat":
+        at = rng.integers(0, n, 6 * n // 10)
+        X[at] = X[rng.integers(0, 40, len(at))]
+    if kind == "offset":
+        X += np.float32(300)
+    C = X[rng.choice(n, nc, replace=False)] + np.float32(0.1)
+    counts = np.bincount(np.sort(rng.integers(0, nc, n)), minlength=nc).astype(np.uint32)
+    norms = _norms_of(X)
+    so = rng.permutation(n).astype(np.uint32)
+    o = _run(dict(X=X, sorted_order=so, centroids=C, num_cells_per_cluster=counts,
+                  cell_norms=norms, num_neighbors=k, num_clusters_searched=cs))
+    rows = np.unique(np.concatenate([np.arange(12), np.arange(n - 40, n),
+                                     rng.choice(n, 40, replace=False)]))
+    pd = _fma(np.float32(-2), _chain(X[rows], C), _norm_chain(C)[None, :])
+    near, cdist = _lists(pd, [range(nc)] * len(rows), cs)
+    np.testing.assert_array_equal(o["nearest_clusters"][rows], near)
+    np.testing.assert_array_equal(o["centroid_distances"][rows], cdist)
+    start = np.concatenate([[0], np.cumsum(counts)]).astype(int)
+    for i, row in enumerate(rows):
+        ids = np.concatenate([np.arange(start[u], start[u + 1]) for u in np.sort(near[i])])
+        ids = ids[ids != row]
+        dist = norms[row] + _fma(np.float32(-2), _chain(X[row:row + 1], X[ids]), norms[ids])
+        at, want = _lists(dist, [range(len(ids))], k)
+        have = at[0] != 0xFFFFFFFF
+        np.testing.assert_array_equal(o["distances"][row], want[0])
+        np.testing.assert_array_equal(o["neighbors"][row][have], so[ids[at[0][have]]])
+        assert (o["neighbors"][row][~have] == 0xFFFFFFFF).all()
+
+
+def test_kmeans_e_step_far_from_the_origin(cuda):
+    """Labels and distances of cells whose margins are wider than the centroids'
+    spread, bit for bit the first nearest centroid's."""
+    import torch
+    n = 64 * torch.cuda.get_device_properties(cuda).multi_processor_count + 5
+    rng = np.random.default_rng(3)
+    X = (rng.standard_normal((n, 6)) + 400).astype(np.float32)
+    out = _kmeans_of(X, 300, 1)
+    rows = np.unique(np.concatenate([np.arange(40), np.arange(n - 40, n),
+                                     rng.choice(n, 100, replace=False)]))
+    C = out["centroids_new"]
+    pd = _fma(np.float32(-2), _chain(X[rows], C), _norm_chain(C)[None, :])
+    np.testing.assert_array_equal(out["cluster_labels"][rows], pd.argmin(1))
+    np.testing.assert_array_equal(out["min_distances"][rows], pd.min(1))
+
+
+@pytest.mark.parametrize("k,cs", [(5, 20), (70, 66)])
+def test_knn_self_refusal_of_wide_margins(cuda, k, cs):
+    """The same where every list would be computed again."""
+    for name, t in _refused_call(cuda, 16000, 6, 400, k, cs, 300.0).items():
+        assert (t == 7).all(), name
