@@ -312,7 +312,7 @@ k_gemm_tc(const float* __restrict__ A, uint64_t lda, uint64_t rows, uint32_t K,
     const float* ap = Apiv + gr;
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
-      const uint32_t c = h * quarter + j;  // < 128: spoff / spiv cover it
+      const uint32_t c = h * quarter + j;  // < 128: spoff / ssign cover it
       const long long off = spoff[c];
       pa[j] = (uint32_t)j < quarter && off >= 0 && rok ? ap[off] : 0.f;
     }

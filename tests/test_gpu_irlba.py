@@ -342,3 +342,27 @@ def test_small_and_large_paths_of_the_u_pass_agree(cuda, n):
     np.testing.assert_array_equal(single.PCs, fused.result.PCs)
     np.testing.assert_array_equal(single.singular_values, fused.result.singular_values)
     assert single.info["second_passes"] == fused.result.info["second_passes"]
+
+
+@pytest.mark.parametrize("n", [2700, 32768, 32769, 40000])
+def test_split_second_pass_agrees_with_whole_blocks(cuda, n):
+    """Cells of 15 distinct kinds: the basis fills the kinds' span and most steps
+    need their second Gram-Schmidt pass. Its update, split over four CTAs per
+    block behind the gate, with its column sums folded in up to 32 blocks and
+    reduced by a launch past that, gives the bits of the whole-block kernels
+    that a batch launches."""
+    import torch
+    from brisc_gb300.batch import SharedMatrix, pca_subsets
+    c = nb_counts(n, 300, seed=5, density=0.08, workers=1)
+    rows = np.random.default_rng(0).integers(0, 15, c.num_cells)
+    S = SharedMatrix(c.indptr, c.indices, c.data, c.num_cells, 300, inv_size_factors=c.isf)
+    fused = pca_subsets(S, [rows], num_PCs=6, subspace_size=30, max_iterations=3,
+                        mode="fused")[0].result
+    M = S.subset(rows)
+    single = M.solve(6, 30, max_iterations=3)
+    M.close()
+    torch.cuda.synchronize()
+    assert single.info["second_passes"] > 0
+    assert single.info["second_passes"] == fused.info["second_passes"]
+    np.testing.assert_array_equal(single.PCs, fused.PCs)
+    np.testing.assert_array_equal(single.singular_values, fused.singular_values)
