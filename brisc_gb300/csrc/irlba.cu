@@ -15,6 +15,7 @@
 #include <chrono>
 #include <cstdio>
 #include <cstdlib>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -69,7 +70,22 @@ int device_smem_optin() {
   return cache[dev];
 }
 
+bool& early_launches() {
+  static thread_local bool on = true;
+  return on;
+}
+
 namespace {
+
+// The solves of this process that are running on each device.
+constexpr int kMaxDevices = 64;
+std::atomic<int> running[kMaxDevices];
+struct RunningSolve {
+  std::atomic<int>& n;
+  explicit RunningSolve(int device) : n(running[device % kMaxDevices]) { ++n; }
+  ~RunningSolve() { --n; }
+  bool alone() const { return n == 1; }
+};
 
 // The scratch pool of the current device, made at its first use.
 cudaError_t scratch_pool(cudaMemPool_t* out) {
@@ -641,6 +657,7 @@ int irlba_solve(const Matrix& X, const bgpu_solve_opts& o, float* pcs,
   const uint32_t m = S.m, k = S.k, g = S.g;
   BGPU_TRY(S.begin(o.seed));
 
+  const RunningSolve self(X.device);
   uint32_t kc = 0, restarts = 0, steps = 0;
   RestartStatus last{};
   bool converged = false;
@@ -651,6 +668,7 @@ int irlba_solve(const Matrix& X, const bgpu_solve_opts& o, float* pcs,
         set_error("solve cancelled");
         return BGPU_ERR_CANCELLED;
       }
+      const EarlyLaunches early(self.alone());
       BGPU_TRY(S.step(j, s));
       ++steps;
     }
