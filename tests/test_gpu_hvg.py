@@ -224,3 +224,34 @@ def test_hvg_csr_gene_slices(cuda, n, g):
                 *oh.clipped_sum_csr(d, ix, ip, nc, g, c, clip))
         for a, w, name in zip(got, want, ("mean", "var", "nnz", "bsum", "bsq")):
             assert np.array_equal(a, w, equal_nan=True), name
+
+
+LARGE_COUNTS = [
+    (np.uint16, [60000, 65535, 65533]),           # every few additions wrap a word
+    (np.float32, [16, 17, 300, 2.75, 0.5, 5000]), (np.float64, [40, 7e4, 1e6, 3]),
+    (np.int64, [20, 65535, 65536, 2**33, 1]), (np.int32, [1] * 19 + [500]),  # below the line
+    (np.uint32, [1] * 12 + [500])]                # above it
+
+
+@pytest.mark.parametrize("n,g,dtype,values", [
+    (n, g, t, v) for n, g in ((1, 3), (9000, 3), (2500, 700)) for t, v in LARGE_COUNTS] +
+    [(900, 38000, *LARGE_COUNTS[1]), (3000, 150000, *LARGE_COUNTS[0])])
+def test_hvg_csr_of_large_counts(cuda, n, g, dtype, values):
+    """Counts that are mostly or partly above the 32-bit accumulators' limit, few
+    and many per gene, whole and by cell list (150,000 genes: the words are taken
+    out within a chunk): bit-identical to the oracle's integers."""
+    rng = np.random.default_rng(n + g)
+    lens = rng.integers(1, min(g, 60) + 1, n)
+    ip = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    ix = np.concatenate([rng.choice(min(g, 400), m, replace=False) for m in lens]).astype(np.int64)
+    ix = ix * (g // min(g, 400))
+    d = rng.choice(np.array(values, np.float64), ix.size).astype(dtype)
+    clip = rng.choice(np.float32([0.5, 15, 299, 64000, 1e9]), g)
+    for c in (np.zeros(0, np.int64), np.concatenate([np.arange(n), np.arange(n)[::-3]])):
+        c = c.astype(np.int64)
+        nc = len(c) if len(c) else n
+        got = _run("csr", d, ix, ip, c, None, nc, g, clip, False)
+        want = (*oh.gene_mean_and_variance_csr(d, ix, ip, c, nc, g),
+                *oh.clipped_sum_csr(d, ix, ip, nc, g, c, clip))
+        for a, w, name in zip(got, want, ("mean", "var", "nnz", "bsum", "bsq")):
+            assert np.array_equal(a, w, equal_nan=True), name
