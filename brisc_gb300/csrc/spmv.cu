@@ -85,7 +85,7 @@ k_spmv(CsrView X, const float* __restrict__ v, const float* __restrict__ sd,
 // segments per warp. A whole warp per segment leaves most lanes without an
 // entry where segments are short (1024 rows x 8 %: 80 entries) and pays its
 // shuffles per segment: 50k x 2000 float values, 7.8M entries: X^T.u 47 us,
-// moments 212 us with 32 lanes and one load at a time, 39 us and 50 us with 8 lanes and
+// moments 212 us with 32 lanes and one load at a time, 39 us and 61 us with 8 lanes and
 // kSegLoads loads in flight.
 constexpr int kSegLoads = 3;
 template <int G>
@@ -371,8 +371,11 @@ int launch_matvec(const Matrix& m, const float* v, const float* sd, float* y,
   return BGPU_OK;
 }
 
-// Segments of more than 128 entries on average keep a whole warp's lanes at
-// work; below that 8 lanes per segment (see Segments).
+// X^T.u: segments of more than 128 entries on average keep a whole warp's lanes
+// at work; below that 8 lanes per segment (see Segments). 6 to 12M floats, us per
+// call with 8 and 32 lanes: 43 entries per segment 78, 118; 81: 78, 91; 106: 79, 79;
+// 128: 69, 68; 162: 75, 66; 221: 79, 68. The moments take 8 lanes at every length
+// (128: 81, 127; 162: 86, 122; 221: 75, 108), whose chains of additions are long.
 static bool wide_segments(const Matrix& m) {
   return (double)m.nnz > 128.0 * (double)m.num_panels * (double)m.g;
 }
@@ -390,13 +393,13 @@ static int launch_partials_typed(const Matrix& m, const float* u, const float* u
   return BGPU_OK;
 }
 
-template <int MODE, int G>
+template <int MODE>
 static int launch_moments_typed(const Matrix& m, double* partials, cudaStream_t s) {
   const uint32_t cg = m.rmat_colgroup;
   const dim3 grid(m.num_panels, (unsigned)ceil_div(m.g, cg));
   const size_t smem = (size_t)m.P * 2 * sizeof(float);
-  if (smem > 48 * 1024) BGPU_CUDA((allow_max_smem(k_gene_moments<MODE, G>)));
-  k_gene_moments<MODE, G><<<grid, 256, smem, s>>>(csc_view(m), (double2*)partials, cg);
+  if (smem > 48 * 1024) BGPU_CUDA((allow_max_smem(k_gene_moments<MODE, 8>)));
+  k_gene_moments<MODE, 8><<<grid, 256, smem, s>>>(csc_view(m), (double2*)partials, cg);
   BGPU_CHECK_LAUNCH();
   return BGPU_OK;
 }
@@ -421,13 +424,8 @@ int launch_gene_stddev(const Matrix& m, double* partials, float* sd,
     BGPU_CHECK_LAUNCH();
     return BGPU_OK;
   }
-  const bool wide = wide_segments(m);
-  if (m.mode == kCounts)
-    BGPU_TRY((wide ? launch_moments_typed<kCounts, 32>(m, partials, s)
-                   : launch_moments_typed<kCounts, 8>(m, partials, s)));
-  else
-    BGPU_TRY((wide ? launch_moments_typed<kFloat, 32>(m, partials, s)
-                   : launch_moments_typed<kFloat, 8>(m, partials, s)));
+  BGPU_TRY(m.mode == kCounts ? launch_moments_typed<kCounts>(m, partials, s)
+                             : launch_moments_typed<kFloat>(m, partials, s));
   k_gene_sd<<<(unsigned)ceil_div(m.g, 32), 32 * kSdWarps, 0, s>>>(
       (const double2*)partials, m.num_panels, m.g, m.n, sd);
   BGPU_CHECK_LAUNCH();
