@@ -6,20 +6,20 @@
 // moments need two of them and a conversion per stored entry, 300 us of
 // k_xt_sell at 300k x 2000 (28.5M entries) against 35 us for the FP32 product
 // over the same entries. So a short run of entries is summed in FP32 additions
-// (23 per entry) and converted to FP64 once.
+// (18 per entry) and converted to FP64 once.
 // The variance is n s2 - s1^2: a gene whose mean is r times its spread loses
 // r^2 of the sums' precision, so these have to be as good as FP64 sums of the
 // run. The values, the squares and the squares' remainders each have a float
-// for the sum and one for what its rounding lost. Over runs of kMomentTerms or
+// for the sum and one for what its rounding lost (the remainders of four squares
+// are added first: rounding those costs 2^-48 of a square). Over runs of kMomentTerms or
 // fewer values within a factor of four of one another (squares: of 16) the lost
 // parts add up without another rounding (they are multiples of the smallest
 // term's ulp, below 2^24 of it), so a run's sums are exact but for the
-// remainders' last bits, 2^-70 of it: that is nearly every value of a gene with
-// r >> 1. Values further apart leave 2^-42, in genes whose spread is of their
+// remainders' last bits: that is nearly every value of a gene with r >> 1. Values further apart leave 2^-42, in genes whose spread is of their
 // mean's size.
 // Measured over 1024 runs of 256 values with mean 10 and sd 0.001: error of the
 // sd 6e-8, with FP64 sums 9e-8; with the remainders added to the squares' lost
-// part (17 additions) 1.2e-6.
+// part 1.2e-6.
 #pragma once
 
 namespace bgpu {
@@ -36,11 +36,17 @@ struct FloatMoments {
     a[0] = t;
     a[1] = __fadd_rn(a[1], e);
   }
-  __device__ __forceinline__ void add(float v) {
-    two_sum(s, v);
-    const float p = __fmul_rn(v, v);
-    two_sum(q, p);
-    two_sum(r, __fmaf_rn(v, v, -p));
+  __device__ __forceinline__ void add(float v0, float v1, float v2, float v3) {
+    const float v[4] = {v0, v1, v2, v3};
+    float e[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      two_sum(s, v[i]);
+      const float p = __fmul_rn(v[i], v[i]);
+      two_sum(q, p);
+      e[i] = __fmaf_rn(v[i], v[i], -p);
+    }
+    two_sum(r, __fadd_rn(__fadd_rn(e[0], e[1]), __fadd_rn(e[2], e[3])));
   }
   // Whether the floats hold the sums: squares within the range where a
   // product's remainder is exact. Otherwise (tiny, huge or non-finite values,

@@ -172,7 +172,12 @@ struct XtAcc;
 template <>
 struct XtAcc<false> {
   float s = 0.f;
-  __device__ __forceinline__ void add(float v) { s += v; }
+  __device__ __forceinline__ void add(float v0, float v1, float v2, float v3) {
+    s += v0;
+    s += v1;
+    s += v2;
+    s += v3;
+  }
 };
 template <>
 struct XtAcc<true> : FloatMoments {};  // a segment has at most kXtMaxP terms
@@ -272,10 +277,9 @@ __device__ __forceinline__ void xt_sell_body(const XtView& X, const float* __res
         const uint2 b3 = k + 7 < U ? ld_stream_u2(nx + 96) : z2;
         const uint32_t wd[8] = {a0.x, a0.y, a1.x, a1.y, a2.x, a2.y, a3.x, a3.y};
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          acc.add(smem_at(smem, wd[i] & 0xffffu));
-          acc.add(smem_at(smem, wd[i] >> 16));
-        }
+        for (int i = 0; i < 8; i += 2)
+          acc.add(smem_at(smem, wd[i] & 0xffffu), smem_at(smem, wd[i] >> 16),
+                  smem_at(smem, wd[i + 1] & 0xffffu), smem_at(smem, wd[i + 1] >> 16));
         a0 = b0; a1 = b1; a2 = b2; a3 = b3;
       }
       if (gene != kNoGene) {  // one segment per gene and panel: no collisions

@@ -85,7 +85,7 @@ k_spmv(CsrView X, const float* __restrict__ v, const float* __restrict__ sd,
 // segments per warp. A whole warp per segment leaves most lanes without an
 // entry where segments are short (1024 rows x 8 %: 80 entries) and pays its
 // shuffles per segment: 50k x 2000 float values, 7.8M entries: X^T.u 47 us,
-// moments 212 us with 32 lanes and one load at a time, 39 us and 61 us with 8 lanes and
+// moments 212 us with 32 lanes and one load at a time, 39 us and 52 us with 8 lanes and
 // kSegLoads loads in flight.
 constexpr int kSegLoads = 3;
 template <int G>
@@ -182,9 +182,11 @@ k_rmat_partials(CscView X, const float* __restrict__ u,
 }
 
 // Per (panel, gene): sum and sum of squares of the values, per lane in runs of
-// up to kMomentTerms floats (moments.cuh), the runs and the lanes in FP64.
+// up to kMomentTerms floats (moments.cuh), the runs and the lanes in FP64. Six
+// blocks per SM: 40 registers, of which a few spill, against 57 and four (50k x
+// 2000, 7.8M entries: 59 -> 52 us).
 template <int MODE, int G>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 6)
 k_gene_moments(CscView X, double2* __restrict__ partials, uint32_t colgroup) {
   extern __shared__ float sm[];
   const uint32_t P = 1u << X.pshift;
@@ -251,8 +253,7 @@ k_gene_moments(CscView X, double2* __restrict__ partials, uint32_t colgroup) {
         for (int i = 0; i < kSegLoads; ++i) values(b + 4 * G * i, vals[i]);
 #pragma unroll
         for (int i = 0; i < kSegLoads; ++i)
-#pragma unroll
-          for (int k = 0; k < 4; ++k) m.add(vals[i][k]);
+          m.add(vals[i][0], vals[i][1], vals[i][2], vals[i][3]);
       }
       if (m.good()) {
         s1 += m.sum();
@@ -375,7 +376,7 @@ int launch_matvec(const Matrix& m, const float* v, const float* sd, float* y,
 // at work; below that 8 lanes per segment (see Segments). 6 to 12M floats, us per
 // call with 8 and 32 lanes: 43 entries per segment 78, 118; 81: 78, 91; 106: 79, 79;
 // 128: 69, 68; 162: 75, 66; 221: 79, 68. The moments take 8 lanes at every length
-// (128: 81, 127; 162: 86, 122; 221: 75, 108), whose chains of additions are long.
+// (128: 81, 127; 162: 86, 122; 221: 75, 108): their chains of additions are long.
 static bool wide_segments(const Matrix& m) {
   return (double)m.nnz > 128.0 * (double)m.num_panels * (double)m.g;
 }
