@@ -85,8 +85,8 @@ k_spmv(CsrView X, const float* __restrict__ v, const float* __restrict__ sd,
 // segments per warp. A whole warp per segment leaves most lanes without an
 // entry where segments are short (1024 rows x 8 %: 80 entries) and pays its
 // shuffles per segment: 50k x 2000 float values, 7.8M entries: X^T.u 47 us,
-// moments 212 us with 32 lanes and one load at a time, 39 us and 52 us with 8 lanes and
-// kSegLoads loads in flight.
+// moments 212 us with 32 lanes and one load at a time, 39 us and 37 us with 8 lanes
+// and kSegLoads loads in flight.
 constexpr int kSegLoads = 3;
 template <int G>
 struct Segments {
@@ -181,12 +181,14 @@ k_rmat_partials(CscView X, const float* __restrict__ u,
   }
 }
 
-// Per (panel, gene): sum and sum of squares of the values, per lane in runs of
-// up to kMomentTerms floats (moments.cuh), the runs and the lanes in FP64. Six
-// blocks per SM: 40 registers, of which a few spill, against 57 and four (50k x
-// 2000, 7.8M entries: 59 -> 52 us).
+// Per (panel, gene): sum and sum of squares of the values, in runs of up to
+// kMomentTerms entries as floats (moments.cuh), the lanes' together, and the runs
+// in FP64: that unit is what short segments wait for (the lanes' sums in FP64, and
+// every lane's: segments of 10 entries, 6M of them, 411 us a call against 230; 7.8M
+// entries of 80: 40 and 37 us). 62 registers, four blocks per SM: held to 40 it
+// spills (53 us).
 template <int MODE, int G>
-__global__ void __launch_bounds__(256, 6)
+__global__ void __launch_bounds__(256, 4)
 k_gene_moments(CscView X, double2* __restrict__ partials, uint32_t colgroup) {
   extern __shared__ float sm[];
   const uint32_t P = 1u << X.pshift;
@@ -203,77 +205,79 @@ k_gene_moments(CscView X, double2* __restrict__ partials, uint32_t colgroup) {
   }
   __syncthreads();
   const Segments<G> seg;
+  const unsigned group = 0xFFFFFFFFu >> (32 - G) << (threadIdx.x & 31 & ~(G - 1));
   const int64_t pbase = X.rowptr[r0];
   const int32_t* cp = X.colptr + (uint64_t)p * (X.g + 1);
   const uint32_t c0 = blockIdx.y * colgroup;
   const uint32_t c1 = min(X.g, c0 + colgroup);
   uint32_t c = c0 + seg.first;
-  int64_t n0 = c < c1 ? cp[c] : 0, n1 = c < c1 ? cp[c + 1] : 0;
+  int32_t n0 = c < c1 ? cp[c] : 0, n1 = c < c1 ? cp[c + 1] : 0;
   for (uint32_t cb = c0; cb < c1; cb += seg.step, c += seg.step) {
-    const int64_t e0 = pbase + n0, e1 = pbase + n1;
+    // the segment from the 4-entry boundary at or before it, in 32 bits
+    const int64_t e0 = pbase + n0, at = e0 & ~3LL;
+    const uint32_t skip = (uint32_t)(e0 - at), len = (uint32_t)(n1 - n0), span = skip + len;
     const uint32_t cn = c + seg.step;
     n0 = cn < c1 ? cp[cn] : 0;
     n1 = cn < c1 ? cp[cn + 1] : 0;
-    auto values = [&](int64_t b, float (&vals)[4]) {
-      if (b >= e1) {
-        vals[0] = vals[1] = vals[2] = vals[3] = 0.f;
-        return;
-      }
+    auto values = [&](uint32_t b, float (&vals)[4]) {  // b < span
       if constexpr (MODE == kCounts) {
-        const uint4 q = ld_stream_u4(X.packed + b);
+        const uint4 q = ld_stream_u4(X.packed + at + b);
         const uint32_t qq[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const uint32_t lr = (qq[k] >> 16) & (P - 1);  // bit 31 may flag a segment head
-          const int64_t e = b + k;
-          vals[k] = (e >= e0 && e < e1)
+          vals[k] = b + k - skip < len
                         ? (X.post ? norm_count(qq[k] & 0xffffu, fs[lr]) * qs[lr]
                                   : norm_count(qq[k] & 0xffffu, fs[lr]))
                         : 0.f;
         }
       } else {
-        const uint4 qv = ld_stream_u4(X.val + b);
+        const uint4 qv = ld_stream_u4(X.val + at + b);
         const float vv[4] = {__uint_as_float(qv.x), __uint_as_float(qv.y),
                              __uint_as_float(qv.z), __uint_as_float(qv.w)};
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int64_t e = b + k;
-          vals[k] = (e >= e0 && e < e1) ? vv[k] : 0.f;
-        }
+        for (int k = 0; k < 4; ++k) vals[k] = b + k - skip < len ? vv[k] : 0.f;
       }
     };
-    constexpr int64_t kStep = 4 * G * kSegLoads, kRun = kStep * (kMomentTerms / (4 * kSegLoads));
+    constexpr uint32_t kStep = 4 * G * kSegLoads, kRun = kMomentTerms / kStep * kStep;
     double s1 = 0.0, s2 = 0.0;
-    for (int64_t run = (e0 & ~3LL) + 4 * seg.lane; run < e1; run += kRun) {
-      const int64_t end = run + kRun < e1 ? run + kRun : e1;
+    for (uint32_t run = 0; run < span && len != 0u; run += kRun) {
+      const uint32_t end = min(span, run + kRun);
       FloatMoments m;
-      for (int64_t b = run; b < end; b += kStep) {
+      for (uint32_t b = run + 4 * seg.lane; b < end; b += kStep) {
         float vals[kSegLoads][4];
 #pragma unroll
-        for (int i = 0; i < kSegLoads; ++i) values(b + 4 * G * i, vals[i]);
+        for (int i = 0; i < kSegLoads; ++i)
+          if (b + 4 * G * i < span) values(b + 4 * G * i, vals[i]);
 #pragma unroll
         for (int i = 0; i < kSegLoads; ++i)
-          m.add(vals[i][0], vals[i][1], vals[i][2], vals[i][3]);
+          if (b + 4 * G * i < span) m.add(vals[i][0], vals[i][1], vals[i][2], vals[i][3]);
       }
+      m.merge<G>(group);
       if (m.good()) {
-        s1 += m.sum();
-        s2 += m.squares();
-      } else {  // out of the floats' range (or no entry): again, in FP64
-        for (int64_t b = run; b < end; b += 4 * G) {
-          float vals[4];
-          values(b, vals);
+        if (seg.lane == 0) {  // the others' have no reader
+          s1 += m.sum();
+          s2 += m.squares();
+        }
+        continue;
+      }
+      double t1 = 0.0, t2 = 0.0;  // out of the floats' range: again, in FP64
+      for (uint32_t b = run + 4 * seg.lane; b < end; b += 4 * G) {
+        float vals[4];
+        values(b, vals);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            s1 += (double)vals[k];
-            s2 += (double)vals[k] * (double)vals[k];
-          }
+        for (int k = 0; k < 4; ++k) {
+          t1 += (double)vals[k];
+          t2 += (double)vals[k] * (double)vals[k];
         }
       }
-    }
 #pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) {
-      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+      for (int o = G / 2; o > 0; o >>= 1) {
+        t1 += __shfl_xor_sync(group, t1, o);
+        t2 += __shfl_xor_sync(group, t2, o);
+      }
+      s1 += t1;
+      s2 += t2;
     }
     if (seg.lane == 0 && c < c1) partials[(uint64_t)p * X.g + c] = make_double2(s1, s2);
   }
@@ -375,8 +379,10 @@ int launch_matvec(const Matrix& m, const float* v, const float* sd, float* y,
 // X^T.u: segments of more than 128 entries on average keep a whole warp's lanes
 // at work; below that 8 lanes per segment (see Segments). 6 to 12M floats, us per
 // call with 8 and 32 lanes: 43 entries per segment 78, 118; 81: 78, 91; 106: 79, 79;
-// 128: 69, 68; 162: 75, 66; 221: 79, 68. The moments take 8 lanes at every length
-// (128: 81, 127; 162: 86, 122; 221: 75, 108): their chains of additions are long.
+// 128: 69, 68; 162: 75, 66; 221: 79, 68. The moments take 8 lanes at every length:
+// their chains of additions are long, and more lanes have more sums to join (128:
+// 81, 127; 162: 86, 122; 221: 75, 108 when each lane's ended in FP64; now 68, 65 and
+// 63 with 8).
 static bool wide_segments(const Matrix& m) {
   return (double)m.nnz > 128.0 * (double)m.num_panels * (double)m.g;
 }
