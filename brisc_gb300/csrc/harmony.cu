@@ -233,7 +233,7 @@ __device__ __forceinline__ void sum_rows4(const float* a, const float* b, uint32
 // (20 of 256 cells at 100k cells: 20 of 152 SMs), so a chunk is split over a
 // cluster of a.split CTAs, each with sub of its cells: their sums meet in
 // distributed shared memory, in rank order. 100k cells, 100 clusters, 50 PCs:
-// 77 us per block with a CTA per chunk, 35 us with eight (both alone, L2 cold;
+// 77 us per block with a CTA per chunk, 36 us with eight (both alone, L2 cold;
 // about 25 us each in the pass, where they overlap).
 template <int CPL>
 __global__ void __launch_bounds__(kHThreads, 2) k_h_block(BlockArgs a) {
